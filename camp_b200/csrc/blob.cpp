@@ -287,10 +287,44 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     return g.unit_target.size() <= 65535 && g.pair_a.size() <= 65535 && dummy <= 65535 &&
            o->rec.size() / 2 / kLanes <= 65535;
   };
-  G gfb, gfw, gbw;
-  if (!pack(t.fb, &gfb, t.n_lu) || !pack(t.fwd, &gfw, n) || !pack(t.bwd, &gbw, n)) {
+  G gfb;
+  if (!pack(t.fb, &gfb, t.n_lu)) {
     *err = "LU schedule exceeds the 16-bit table encodings";
     return false;
+  }
+  // the solves as rounds of 32 targets, longest first within a level, so
+  // that a round's targets have similar lengths and its padding stays small
+  std::vector<uint32_t> sv_rec, sv_ext;
+  const uint32_t no_pair = (uint32_t)t.n_lu | ((uint32_t)n << 16);
+  int n_srounds = 0;
+  for (const Tables::Grouped* g : {&t.fwd, &t.bwd}) {
+    for (int l = 0; l < g->n_levels; ++l) {
+      std::vector<int> us;
+      for (int u = g->lane_ptr[33 * l]; u < g->lane_ptr[33 * l + kLanes]; ++u) us.push_back(u);
+      std::stable_sort(us.begin(), us.end(), [&](int a, int b) {
+        return g->unit_count[a] > g->unit_count[b];
+      });
+      for (size_t r = 0; r < us.size(); r += kLanes, ++n_srounds) {
+        const int cnt = std::max(1, g->unit_count[us[r]]);
+        auto pair = [&](size_t k, int j) {
+          if (k >= us.size() || j >= g->unit_count[us[k]]) return no_pair;
+          const int p = g->unit_begin[us[k]] + j;
+          return (uint32_t)g->pair_a[p] | ((uint32_t)g->pair_b[p] << 16);
+        };
+        for (size_t k = r; k < r + kLanes; ++k) {
+          sv_rec.push_back(pair(k, 0));
+          const uint32_t tgt = k < us.size() ? (uint32_t)g->unit_target[us[k]] : (uint32_t)n;
+          const bool fin = k < us.size() && g->unit_recip[us[k]] > 0;
+          sv_rec.push_back(tgt | ((uint32_t)cnt << 16) | (fin ? 0x80000000u : 0u));
+        }
+        for (int j = 1; j < cnt; ++j)
+          for (size_t k = r; k < r + kLanes; ++k) sv_ext.push_back(pair(k, j));
+      }
+    }
+  }
+  for (int k = 0; k < 2 * kLanes; ++k) {  // read ahead, never run
+    sv_rec.push_back(no_pair);
+    sv_rec.push_back((uint32_t)n | (1u << 16));
   }
 
   Writer w;
@@ -420,19 +454,16 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     }
   }
   o.n_plev = t.n_plev;
-  o.lu_perm = w.put(u16(t.lu_perm));
+  o.lu_iperm = w.put(u16(t.lu_iperm));
   o.lu_src = w.put(lu_src);
   o.fa_ptr = w.put(u16(t.fa_ptr));
   o.fa = w.put(fa);
   o.fb_lane = w.put(gfb.rnd);
   o.fb_unit = w.put(gfb.rec);
   o.fb_pair = w.put(gfb.pair);
-  o.fw_lane = w.put(gfw.rnd);
-  o.fw_unit = w.put(gfw.rec);
-  o.fw_pair = w.put(gfw.pair);
-  o.bw_lane = w.put(gbw.rnd);
-  o.bw_unit = w.put(gbw.rec);
-  o.bw_pair = w.put(gbw.pair);
+  o.n_srounds = n_srounds;
+  o.sv_rec = w.put(sv_rec);
+  o.sv_ext = w.put(sv_ext);
   o.dep_state = w.put(u16(t.dep_state));
   o.atol = w.put(atol_dep);
   // the one-lane LU tables come last: the level-scheduled mode stages only

@@ -28,20 +28,26 @@ struct BlobOff {
   // J gather: w0 = part | coef<<16, w1 = independent species + 1 (0 = loss
   // entry); per slot: entry pointer, LU position, row; lane slot lists
   int jg_w0, jg_w1, jg_ptr, jg_mid, jg_lupos, jg_row, jg_lane, jg_slots;
-  // LU: perm, diag (uint16); factorization by pivot level: scaled L entries
-  // (fa_ptr uint16, fa = pos | pivot<<16), Schur updates grouped by target
-  // with the reciprocal pivots taken in the same phase (fb); forward solve
-  // (fw); backward solve updates with the pivots finalised in the same
-  // phase (bw).  A grouped phase G has round pointers per level (uint16,
-  // levels + 1; the *_lane fields), one record per lane and round (the
-  // *_unit fields: uint32 target | count<<16, uint32 first pair |
-  // (pivot+1)<<16, pivot 0 = none; a no-op record targets the spare slot
-  // past the accumulator) and pairs (uint32 a | b<<16).
-  int lu_perm, lu_diag, lu_src;
+  // LU: dependent index -> pivot row (iperm), diag (uint16); factorization by
+  // pivot level: scaled L entries (fa_ptr uint16, fa = pos | pivot<<16),
+  // Schur updates grouped by target with the reciprocal pivots taken in the
+  // same phase (fb).  The grouped phase fb has round pointers per level
+  // (uint16, levels + 1; fb_lane), one record per lane and round (fb_unit:
+  // uint32 target | count<<16, uint32 first pair | (pivot+1)<<16, pivot 0 =
+  // none; a no-op record targets the spare slot past the accumulator) and
+  // pairs (uint32 a | b<<16).
+  int lu_iperm, lu_diag, lu_src;
   int fa_ptr, fa;
   int fb_lane, fb_unit, fb_pair;
-  int fw_lane, fw_unit, fw_pair;
-  int bw_lane, bw_unit, bw_pair;
+  // triangular solves: n_srounds rounds, forward then backward.  A round
+  // gives every lane one target z[tgt] -= sum LU[a] z[x] (backward: then
+  // times its reciprocal pivot when bit 31 of the second word is set): record
+  // uint32 a | x<<16, uint32 tgt | cnt<<16 | finish<<31 (sv_rec, 32 records
+  // per round and two rounds of padding at the end), the first pair in the
+  // record, cnt - 1 more per lane in sv_ext (uint32 a | x<<16, 32 per step).
+  // cnt is the round's largest, the same in every lane: shorter targets and
+  // idle lanes are padded with the spare slots LU[n_lu] = z[n] = 0.
+  int n_srounds, sv_rec, sv_ext;
   // row-wise LU for the sequential (one-lane) mode: J slot -> LU position
   // (jg_lupos), diagonal positions, rowptr, col (uint16), update pointer per
   // L entry (uint32) and updates (src | dst<<16); staged only in that mode

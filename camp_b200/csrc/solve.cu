@@ -130,14 +130,10 @@ struct Tab {
   const uint16_t *fg_unit, *fg_lane, *fg_split;
   const uint32_t* jg_w0;
   const uint16_t *jg_w1, *jg_ptr, *jg_mid, *jg_lupos, *jg_row, *jg_lane, *jg_slots;
-  const uint16_t *lu_perm, *lu_diag, *lu_src, *fa_ptr;
+  const uint16_t *lu_iperm, *lu_diag, *lu_src, *fa_ptr;
   const uint32_t* fa;
   const uint16_t* fb_lane;
   const uint32_t *fb_unit, *fb_pair;
-  const uint16_t* fw_lane;
-  const uint32_t *fw_unit, *fw_pair;
-  const uint16_t *bw_lane;
-  const uint32_t *bw_unit, *bw_pair;
   const uint16_t* dep_state;
   const double* atol;
   const uint16_t *lu_rowptr, *lu_col;
@@ -165,7 +161,7 @@ __device__ __forceinline__ Tab make_tab(const char* b) {
   t.jg_row = (const uint16_t*)(b + o.jg_row);
   t.jg_lane = (const uint16_t*)(b + o.jg_lane);
   t.jg_slots = (const uint16_t*)(b + o.jg_slots);
-  t.lu_perm = (const uint16_t*)(b + o.lu_perm);
+  t.lu_iperm = (const uint16_t*)(b + o.lu_iperm);
   t.lu_diag = (const uint16_t*)(b + o.lu_diag);
   t.lu_src = (const uint16_t*)(b + o.lu_src);
   t.fa_ptr = (const uint16_t*)(b + o.fa_ptr);
@@ -186,12 +182,6 @@ __device__ __forceinline__ Tab make_tab(const char* b) {
   t.fb_lane = (const uint16_t*)(b + o.fb_lane);
   t.fb_unit = (const uint32_t*)(b + o.fb_unit);
   t.fb_pair = (const uint32_t*)(b + o.fb_pair);
-  t.fw_lane = (const uint16_t*)(b + o.fw_lane);
-  t.fw_unit = (const uint32_t*)(b + o.fw_unit);
-  t.fw_pair = (const uint32_t*)(b + o.fw_pair);
-  t.bw_lane = (const uint16_t*)(b + o.bw_lane);
-  t.bw_unit = (const uint32_t*)(b + o.bw_unit);
-  t.bw_pair = (const uint32_t*)(b + o.bw_pair);
   t.dep_state = (const uint16_t*)(b + o.dep_state);
   t.atol = (const double*)(b + o.atol);
   t.lu_rowptr = (const uint16_t*)(b + o.lu_rowptr);
@@ -975,20 +965,17 @@ __device__ __forceinline__ bool has_simpol(const char* tb) {
 // ---------------------------------------------------------------------------
 // LU of M = I - gamma*J on the fixed order, and the triangular solves
 // ---------------------------------------------------------------------------
-// One level of a grouped phase: every unit of this lane subtracts its pair
-// products from its target, acc[target] -= sum a[pa] * x[pb].  A unit that
-// carries a pivot (factorization only) then stores the reciprocal of its
-// final value, the pivot, in dinv; the return value flags a zero or
-// non-finite pivot.
-template <int MODE, typename LT, typename XT>
+// One level of the factorization: every unit of this lane subtracts its pair
+// products from its target, LU[target] -= sum LU[pa] * LU[pb].  A unit that
+// carries a pivot then stores the reciprocal of its final value, the pivot,
+// in dinv; the return value flags a zero or non-finite pivot.
+template <typename LT>
 __device__ __forceinline__ bool grouped_level(const uint16_t* rnd, const uint32_t* rec,
-                                              const uint32_t* pair, int level, LT* acc,
-                                              const LT* a, const XT* x, LT* dinv, int lane) {
-  // MODE 0: plain; 1: a unit carrying pivot k stores dinv[k] = 1 / (its
-  // final value) (factorization); 2: a unit carrying pivot k scales its final
-  // value by dinv[k] (backward substitution).  Round r hands this lane the
-  // record rec[32 r + lane]; a no-op record targets the spare accumulator
-  // slot with no pairs and no pivot, so every lane runs the same code.
+                                              const uint32_t* pair, int level, LT* LU, LT* dinv,
+                                              int lane) {
+  // Round r hands this lane the record rec[32 r + lane]; a no-op record
+  // targets the spare slot with no pairs and no pivot, so every lane runs the
+  // same code.
   bool bad = false;
   const uint2* rec2 = (const uint2*)rec;
   const int r1 = rnd[level + 1];
@@ -997,26 +984,25 @@ __device__ __forceinline__ bool grouped_level(const uint16_t* rnd, const uint32_
     const uint2 w = rec2[32 * r + lane];
     const int tgt = w.x & 0xFFFFu, cnt = w.x >> 16;
     const int p0 = w.y & 0xFFFFu, piv = w.y >> 16;
-    LT s0 = acc[tgt], s1 = (LT)0;
+    LT s0 = LU[tgt], s1 = (LT)0;
     int p = p0;
     #pragma unroll 1
     for (; p + 1 < p0 + cnt; p += 2) {
       const uint32_t q0 = pair[p], q1 = pair[p + 1];
-      s0 -= a[q0 & 0xFFFFu] * (LT)x[q0 >> 16];
-      s1 -= a[q1 & 0xFFFFu] * (LT)x[q1 >> 16];
+      s0 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
+      s1 -= LU[q1 & 0xFFFFu] * LU[q1 >> 16];
     }
     if (p < p0 + cnt) {
       const uint32_t q0 = pair[p];
-      s0 -= a[q0 & 0xFFFFu] * (LT)x[q0 >> 16];
+      s0 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
     }
     LT s = s0 + s1;
-    if (MODE == 1 && piv) {
+    if (piv) {
       const bool pbad = (s == (LT)0) || !isfinite((double)s);
       bad |= pbad;
       dinv[piv - 1] = pbad ? (LT)0 : (LT)1 / s;
     }
-    if (MODE == 2 && piv) s *= dinv[piv - 1];
-    acc[tgt] = s;
+    LU[tgt] = s;
   }
   return bad;
 }
@@ -1039,7 +1025,7 @@ __device__ __noinline__ bool dev_form_factor(const char* tb, const LT* J, double
     LU[q] = v;
   }
   __syncwarp();
-  bool bad = grouped_level<1, LT, LT>(t.fb_lane, t.fb_unit, t.fb_pair, 0, LU, LU, LU, dinv, lane);
+  bool bad = grouped_level<LT>(t.fb_lane, t.fb_unit, t.fb_pair, 0, LU, dinv, lane);
   __syncwarp();
   #pragma unroll 1
   for (int lv = 0; lv < t.n_plev; ++lv) {
@@ -1050,33 +1036,65 @@ __device__ __noinline__ bool dev_form_factor(const char* tb, const LT* J, double
       LU[w & 0xFFFFu] *= dinv[w >> 16];
     }
     __syncwarp();
-    bad |= grouped_level<1, LT, LT>(t.fb_lane, t.fb_unit, t.fb_pair, lv + 1, LU, LU, LU, dinv, lane);
+    bad |= grouped_level<LT>(t.fb_lane, t.fb_unit, t.fb_pair, lv + 1, LU, dinv, lane);
     __syncwarp();
   }
   return !warp_any(bad);
 }
 
-// b (original variable order, FP64) <- M^{-1} b
+// The spare slots that the padding of the solve rounds reads and writes.
 template <typename LT>
-__device__ __noinline__ void dev_lsolve(const char* tb, const LT* LU, const LT* dinv,
-                                        double* b, LT* z, int lane) {
-  const Tab t = make_tab(tb);
-  #pragma unroll 1
-  for (int k = lane; k < t.n; k += 32) z[k] = (LT)b[t.lu_perm[k]];
+__device__ __forceinline__ void clear_spare(const char* tb, LT* LU, LT* z, int lane) {
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  if (lane == 0) LU[o.n_lu] = z[o.n] = (LT)0;
   __syncwarp();
+}
+
+// z (in pivot order) <- M^{-1} z.
+// Bound by latency: some thirty levels in a row (cb05cl_ae5: 14 forward, 16
+// backward), each a handful of dependent steps on at most 32 targets.  So a
+// round is one record load per lane and as few instructions as will do: the
+// record holds its first pair (the only one in most rounds), the next
+// round's L / U value and the record after that are loaded while this round
+// runs, and the pair count is the same in every lane.
+template <typename LT>
+__device__ __noinline__ void dev_lsolve(const char* tb, const LT* LU, const LT* dinv, LT* z,
+                                        int lane) {
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  const uint2* rec = (const uint2*)(tb + o.sv_rec) + lane;
+  const uint32_t* ext = (const uint32_t*)(tb + o.sv_ext) + lane;
+  const uint2* const end = rec + 32 * o.n_srounds;
+  uint2 w = rec[0], wn = rec[32];
+  LT a = LU[w.x & 0xFFFFu];
   #pragma unroll 1
-  for (int lv = 0; lv < t.n_flev; ++lv) {
-    grouped_level<0, LT, LT>(t.fw_lane, t.fw_unit, t.fw_pair, lv, z, LU, z, (LT*)nullptr, lane);
+  for (; rec < end; rec += 32) {
+    const uint2 wnn = rec[64];
+    const LT an = LU[wn.x & 0xFFFFu];
+    const int tgt = w.y & 0xFFFFu, cnt = (w.y >> 16) & 0x7FFFu;
+    LT s0 = z[tgt], s1 = (LT)0;
+    s0 -= a * z[w.x >> 16];
+    if (cnt > 1) {
+      int p = 1;
+      #pragma unroll 1
+      for (; p + 1 < cnt; p += 2, ext += 64) {
+        const uint32_t q0 = ext[0], q1 = ext[32];
+        s1 -= LU[q0 & 0xFFFFu] * z[q0 >> 16];
+        s0 -= LU[q1 & 0xFFFFu] * z[q1 >> 16];
+      }
+      if (p < cnt) {
+        const uint32_t q0 = ext[0];
+        s1 -= LU[q0 & 0xFFFFu] * z[q0 >> 16];
+        ext += 32;
+      }
+    }
+    LT s = s0 + s1;
+    if ((int)w.y < 0) s *= dinv[tgt];
+    z[tgt] = s;
     __syncwarp();
+    w = wn;
+    wn = wnn;
+    a = an;
   }
-  #pragma unroll 1
-  for (int g = 0; g < t.n_blev; ++g) {
-    grouped_level<2, LT, LT>(t.bw_lane, t.bw_unit, t.bw_pair, g, z, LU, z, (LT*)dinv, lane);
-    __syncwarp();
-  }
-  #pragma unroll 1
-  for (int k = lane; k < t.n; k += 32) b[t.lu_perm[k]] = (double)z[k];
-  __syncwarp();
 }
 
 // Sequential mode: lane 0 factors row by row (IKJ order, the same update
@@ -1135,12 +1153,9 @@ __device__ __noinline__ bool dev_form_factor_seq(const char* tb, const LT* J, do
 }
 
 template <typename LT>
-__device__ __noinline__ void dev_lsolve_seq(const char* tb, const LT* LU, const LT* dinv,
-                                            double* b, LT* z, int lane) {
+__device__ __noinline__ void dev_lsolve_seq(const char* tb, const LT* LU, const LT* dinv, LT* z,
+                                            int lane) {
   const Tab t = make_tab(tb);
-  #pragma unroll 1
-  for (int k = lane; k < t.n; k += 32) z[k] = (LT)b[t.lu_perm[k]];
-  __syncwarp();
   if (lane == 0) {
     #pragma unroll 1
     for (int i = 0; i < t.n; ++i) {
@@ -1170,9 +1185,6 @@ __device__ __noinline__ void dev_lsolve_seq(const char* tb, const LT* LU, const 
     }
   }
   __syncwarp();
-  #pragma unroll 1
-  for (int k = lane; k < t.n; k += 32) b[t.lu_perm[k]] = (double)z[k];
-  __syncwarp();
 }
 
 // ---------------------------------------------------------------------------
@@ -1187,6 +1199,7 @@ __device__ __noinline__ void dev_lsolve_seq(const char* tb, const LT* LU, const 
 template <typename LT, bool AERO, bool BLK = false>
 struct Cell {
   const char* tb;     // shared-memory tables
+  const uint16_t* iperm;  // dependent index -> pivot row
   blk::Cmd* cmd;      // CTA form: the command slot and the operations' arrays
   const blk::Ctx<LT>* bx;
   const double* atol;
@@ -1428,30 +1441,46 @@ struct Cell {
   __device__ int newton(bool projected) {
     int mm = 0;
     double del, delp = 0.0;
+    // the correction of a matrix whose gamma has moved since (1.0: not moved)
+    const double corr = gamrat != 1.0 ? ddiv(2.0, 1.0 + gamrat) : 1.0;
     #pragma unroll 1
     for (;;) {
+      // right-hand side, solve, then scaling, norm and update in one pass:
+      // the warp form writes the right-hand side straight into pivot order
+      // and reads the solution back from it
       #pragma unroll 1
-      for (int i = lane; i < n; i += 32)
-        tempv[i] = gamma * ftemp[i] - (rl1 * (zb + (1) * n)[i] + acor[i]);
+      for (int i = lane; i < n; i += 32) {
+        const double r = gamma * ftemp[i] - (rl1 * (zb + (1) * n)[i] + acor[i]);
+        if constexpr (BLK)
+          tempv[i] = r;
+        else
+          z[iperm[i]] = (LT)r;
+      }
       __syncwarp();
       if constexpr (BLK)
         blk::call<LT>(cmd, *bx, blk::OP_SOLVE, nullptr, nullptr, 0.0);
       else if (lu_mode)
-        dev_lsolve_seq<LT>(tb, LU, dinv, tempv, z, lane);
+        dev_lsolve_seq<LT>(tb, LU, dinv, z, lane);
       else
-        dev_lsolve<LT>(tb, LU, dinv, tempv, z, lane);
-      if (gamrat != 1.0) {
-        double s = ddiv(2.0, 1.0 + gamrat);
-        #pragma unroll 1
-        for (int i = lane; i < n; i += 32) tempv[i] *= s;
-      }
+        dev_lsolve<LT>(tb, LU, dinv, z, lane);
       nni++;
-      del = wrms(tempv);
+      double sum = 0.0;
       #pragma unroll 1
       for (int i = lane; i < n; i += 32) {
-        acor[i] += tempv[i];
-        y[i] = (zb + (0) * n)[i] + acor[i];
+        double v;
+        if constexpr (BLK)
+          v = tempv[i];
+        else
+          v = (double)z[iperm[i]];
+        // rounded by itself, as when it was stored, not fused into the sum
+        const double d = __dmul_rn(v, corr);
+        const double t = d * ewt[i];
+        sum += t * t;
+        const double a = acor[i] + d;
+        acor[i] = a;
+        y[i] = (zb + (0) * n)[i] + a;
       }
+      del = dsqrt(ddiv(warp_sum(sum), (double)n));
       __syncwarp();
       if (mm > 0) crate = fmax(CRDOWN * crate, ddiv(del, delp));
       double dcon = ddiv(del * fmin(1.0, crate), tq[4]);
@@ -1781,6 +1810,7 @@ __device__ void bind_cell(Cell<LT, AERO>& c, const SolveArgs& a, const char* tab
                           int gwarp, int lane) {
   c.tb = tab;
   c.atol = make_tab(tab).atol;
+  c.iperm = make_tab(tab).lu_iperm;
   c.lane = lane;
   c.n = a.off.n;
   // per-warp global slab: [Nordsieck history when it is not in shared
@@ -1826,6 +1856,7 @@ __global__ void __launch_bounds__(32 * (AERO ? kMaxCellsAero : kMaxCellsPerBlock
   char* base = smem + a.tab_bytes + (size_t)wib * a.lay.bytes;
   Cell<LT, AERO> c;
   bind_cell<LT, AERO>(c, a, smem, base, gwarp, lane);
+  clear_spare<LT>(smem, c.LU, c.z, lane);
   const DevMech& m = a.m;
   const uint16_t* dep_state = make_tab(smem).dep_state;
   #pragma unroll 1
@@ -1981,6 +2012,7 @@ __global__ void __launch_bounds__(blk::kThreads, sizeof(LT) == 4 ? 2 : 1)
     }
     Cell<LT, false, true> c;
     c.tb = nullptr;
+    c.iperm = nullptr;
     c.cmd = &cmd;
     c.bx = cx;
     c.atol = cx->t.atol;
@@ -2279,11 +2311,11 @@ __global__ void precision_kernel(PrecArgs p) {
   double* y = (double*)(base + a.lay.y);
   double* rates = (double*)(base + a.lay.rates);
   double* keff = (double*)(base + a.lay.keff);
-  double* b = (double*)(base + a.lay.tempv);
   LT* LU = (LT*)(base + a.lay.lu);
   LT* z = (LT*)(base + a.lay.z);
   LT* dinv = (LT*)(base + a.lay.dinv);
   LT* J = (LT*)p.jbuf + (size_t)cell * t.n_jac;
+  clear_spare<LT>(smem, LU, z, lane);
   const double* st = a.state + (size_t)cell * m.n_state;
   #pragma unroll 1
   for (int i = lane; i < t.n; i += 32) y[i] = st[t.dep_state[i]];
@@ -2297,12 +2329,13 @@ __global__ void precision_kernel(PrecArgs p) {
     #pragma unroll 1
     for (int i = lane; i < t.n; i += 32) {
       const double s = p.rtol * fabs(y[i]) + t.atol[i];
-      b[i] = ((i * 2654435761u) >> 13) & 1u ? s : -s;
+      z[t.lu_iperm[i]] = (LT)(((i * 2654435761u) >> 13) & 1u ? s : -s);
     }
     __syncwarp();
-    dev_lsolve<LT>(smem, LU, dinv, b, z, lane);
+    dev_lsolve<LT>(smem, LU, dinv, z, lane);
     #pragma unroll 1
-    for (int i = lane; i < t.n; i += 32) p.x[(size_t)cell * t.n + i] = b[i];
+    for (int i = lane; i < t.n; i += 32)
+      p.x[(size_t)cell * t.n + i] = (double)z[t.lu_iperm[i]];
   }
   if (lane == 0) p.bad[cell] = ok ? 0 : 1;
 }
