@@ -251,79 +251,76 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   };
   std::vector<uint32_t> fa(t.fa_pos.size());
   for (size_t i = 0; i < fa.size(); ++i) fa[i] = (uint32_t)t.fa_pos[i] | ((uint32_t)t.fa_piv[i] << 16);
-  // A grouped phase is stored as rounds: level l runs rounds
-  // [rnd[l], rnd[l + 1]); round r gives lane k the record rec[32 r + k] of
-  // its r-th unit (units of a lane in decreasing size) or, when the lane has
-  // fewer units, a no-op record whose target is the spare slot `dummy` past
-  // the end of the accumulator.  Records: target | count<<16, first pair |
-  // (pivot+1)<<16.
-  struct G {
-    std::vector<uint16_t> rnd;
-    std::vector<uint32_t> rec, pair;
+  // Grouped phases as rounds of 32 targets, longest first within a level, so
+  // that a round's targets have similar lengths and its padding stays small.
+  // Per round its pair count, whether it is the last of its level, 32 records
+  // (first pair, target, pivot or finish mark) and its further pairs.
+  struct Rounds {
+    std::vector<uint32_t> pair0, target, recip, ext;
+    std::vector<int> cnt, last;
   };
-  auto pack = [&](const Tables::Grouped& g, G* o, int dummy) {
-    o->rnd.assign(1, 0);
-    o->rec.clear();
+  auto rounds_of = [&](const Tables::Grouped& g, Rounds* o, uint32_t no_pair, int spare,
+                       bool keep_empty) {
     for (int l = 0; l < g.n_levels; ++l) {
-      int rounds = 0;
-      for (int k = 0; k < kLanes; ++k)
-        rounds = std::max(rounds, g.lane_ptr[33 * l + k + 1] - g.lane_ptr[33 * l + k]);
-      for (int r = 0; r < rounds; ++r)
-        for (int k = 0; k < kLanes; ++k) {
-          const int u = g.lane_ptr[33 * l + k] + r;
-          if (u < g.lane_ptr[33 * l + k + 1]) {
-            o->rec.push_back((uint32_t)g.unit_target[u] | ((uint32_t)g.unit_count[u] << 16));
-            o->rec.push_back((uint32_t)g.unit_begin[u] | ((uint32_t)g.unit_recip[u] << 16));
-          } else {
-            o->rec.push_back((uint32_t)dummy);
-            o->rec.push_back(0u);
-          }
-        }
-      o->rnd.push_back((uint16_t)(o->rnd.back() + rounds));
-    }
-    o->pair.resize(g.pair_a.size());
-    for (size_t p = 0; p < g.pair_a.size(); ++p)
-      o->pair[p] = (uint32_t)g.pair_a[p] | ((uint32_t)g.pair_b[p] << 16);
-    return g.unit_target.size() <= 65535 && g.pair_a.size() <= 65535 && dummy <= 65535 &&
-           o->rec.size() / 2 / kLanes <= 65535;
-  };
-  G gfb;
-  if (!pack(t.fb, &gfb, t.n_lu)) {
-    *err = "LU schedule exceeds the 16-bit table encodings";
-    return false;
-  }
-  // the solves as rounds of 32 targets, longest first within a level, so
-  // that a round's targets have similar lengths and its padding stays small
-  std::vector<uint32_t> sv_rec, sv_ext;
-  const uint32_t no_pair = (uint32_t)t.n_lu | ((uint32_t)n << 16);
-  int n_srounds = 0;
-  for (const Tables::Grouped* g : {&t.fwd, &t.bwd}) {
-    for (int l = 0; l < g->n_levels; ++l) {
       std::vector<int> us;
-      for (int u = g->lane_ptr[33 * l]; u < g->lane_ptr[33 * l + kLanes]; ++u) us.push_back(u);
+      for (int u = g.lane_ptr[33 * l]; u < g.lane_ptr[33 * l + kLanes]; ++u) us.push_back(u);
       std::stable_sort(us.begin(), us.end(), [&](int a, int b) {
-        return g->unit_count[a] > g->unit_count[b];
+        return g.unit_count[a] > g.unit_count[b];
       });
-      for (size_t r = 0; r < us.size(); r += kLanes, ++n_srounds) {
-        const int cnt = std::max(1, g->unit_count[us[r]]);
+      const size_t n_r = std::max<size_t>(keep_empty ? 1 : 0, (us.size() + kLanes - 1) / kLanes);
+      for (size_t r = 0; r < n_r; ++r) {
         auto pair = [&](size_t k, int j) {
-          if (k >= us.size() || j >= g->unit_count[us[k]]) return no_pair;
-          const int p = g->unit_begin[us[k]] + j;
-          return (uint32_t)g->pair_a[p] | ((uint32_t)g->pair_b[p] << 16);
+          if (k >= us.size() || j >= g.unit_count[us[k]]) return no_pair;
+          const int p = g.unit_begin[us[k]] + j;
+          return (uint32_t)g.pair_a[p] | ((uint32_t)g.pair_b[p] << 16);
         };
-        for (size_t k = r; k < r + kLanes; ++k) {
-          sv_rec.push_back(pair(k, 0));
-          const uint32_t tgt = k < us.size() ? (uint32_t)g->unit_target[us[k]] : (uint32_t)n;
-          const bool fin = k < us.size() && g->unit_recip[us[k]] > 0;
-          sv_rec.push_back(tgt | ((uint32_t)cnt << 16) | (fin ? 0x80000000u : 0u));
+        const size_t k0 = r * kLanes;
+        const int cnt = k0 < us.size() ? std::max(1, g.unit_count[us[k0]]) : 1;
+        o->cnt.push_back(cnt);
+        o->last.push_back(r + 1 == n_r);
+        for (size_t k = k0; k < k0 + kLanes; ++k) {
+          const bool real = k < us.size();
+          o->pair0.push_back(pair(k, 0));
+          o->target.push_back(real ? (uint32_t)g.unit_target[us[k]] : (uint32_t)spare);
+          o->recip.push_back(real ? (uint32_t)g.unit_recip[us[k]] : 0u);
         }
         for (int j = 1; j < cnt; ++j)
-          for (size_t k = r; k < r + kLanes; ++k) sv_ext.push_back(pair(k, j));
+          for (size_t k = k0; k < k0 + kLanes; ++k) o->ext.push_back(pair(k, j));
       }
     }
+  };
+  for (const Tables::Grouped* g : {&t.fb, &t.fwd, &t.bwd})
+    if (g->unit_target.size() > 65535 || g->pair_a.size() > 65535) {
+      *err = "LU schedule exceeds the 16-bit table encodings";
+      return false;
+    }
+  Rounds fbr, svr;
+  const uint32_t lu_none = (uint32_t)t.n_lu | ((uint32_t)t.n_lu << 16);
+  const uint32_t sv_none = (uint32_t)t.n_lu | ((uint32_t)n << 16);
+  rounds_of(t.fb, &fbr, lu_none, t.n_lu, true);
+  rounds_of(t.fwd, &svr, sv_none, n, false);
+  rounds_of(t.bwd, &svr, sv_none, n, false);
+  std::vector<uint32_t> fb_rec, sv_rec;
+  std::vector<uint16_t> fb_hdr;
+  for (size_t r = 0; r < fbr.cnt.size(); ++r)
+    fb_hdr.push_back((uint16_t)(fbr.cnt[r] | (fbr.last[r] ? 0x8000 : 0)));
+  fb_hdr.push_back(1);  // read ahead, never run
+  for (size_t k = 0; k < fbr.pair0.size(); ++k) {
+    fb_rec.push_back(fbr.pair0[k]);
+    fb_rec.push_back(fbr.target[k] | (fbr.recip[k] << 16));
   }
-  for (int k = 0; k < 2 * kLanes; ++k) {  // read ahead, never run
-    sv_rec.push_back(no_pair);
+  for (int k = 0; k < kLanes; ++k) {
+    fb_rec.push_back(lu_none);
+    fb_rec.push_back((uint32_t)t.n_lu);
+  }
+  const int n_srounds = (int)svr.cnt.size();
+  for (size_t k = 0; k < svr.pair0.size(); ++k) {
+    sv_rec.push_back(svr.pair0[k]);
+    sv_rec.push_back(svr.target[k] | ((uint32_t)svr.cnt[k / kLanes] << 16) |
+                     (svr.recip[k] ? 0x80000000u : 0u));
+  }
+  for (int k = 0; k < 2 * kLanes; ++k) {
+    sv_rec.push_back(sv_none);
     sv_rec.push_back((uint32_t)n | (1u << 16));
   }
 
@@ -458,12 +455,12 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   o.lu_src = w.put(lu_src);
   o.fa_ptr = w.put(u16(t.fa_ptr));
   o.fa = w.put(fa);
-  o.fb_lane = w.put(gfb.rnd);
-  o.fb_unit = w.put(gfb.rec);
-  o.fb_pair = w.put(gfb.pair);
+  o.fb_hdr = w.put(fb_hdr);
+  o.fb_rec = w.put(fb_rec);
+  o.fb_ext = w.put(fbr.ext);
   o.n_srounds = n_srounds;
   o.sv_rec = w.put(sv_rec);
-  o.sv_ext = w.put(sv_ext);
+  o.sv_ext = w.put(svr.ext);
   o.dep_state = w.put(u16(t.dep_state));
   o.atol = w.put(atol_dep);
   // the one-lane LU tables come last: the level-scheduled mode stages only

@@ -31,14 +31,15 @@ struct BlobOff {
   // LU: dependent index -> pivot row (iperm), diag (uint16); factorization by
   // pivot level: scaled L entries (fa_ptr uint16, fa = pos | pivot<<16),
   // Schur updates grouped by target with the reciprocal pivots taken in the
-  // same phase (fb).  The grouped phase fb has round pointers per level
-  // (uint16, levels + 1; fb_lane), one record per lane and round (fb_unit:
-  // uint32 target | count<<16, uint32 first pair | (pivot+1)<<16, pivot 0 =
-  // none; a no-op record targets the spare slot past the accumulator) and
-  // pairs (uint32 a | b<<16).
+  // same phase, as rounds (n_plev + 1 phases).  A round gives every lane one
+  // target LU[tgt] -= sum LU[a] LU[b]: record uint32 a | b<<16, uint32 tgt |
+  // (pivot+1)<<16 (pivot 0 = none; fb_rec, 32 records per round and one round
+  // of padding at the end), the first pair in the record, the round's
+  // cnt - 1 more per lane in fb_ext; fb_hdr (uint16 per round): cnt | last
+  // round of its phase<<15.  Padding as in the solves.
   int lu_iperm, lu_diag, lu_src;
   int fa_ptr, fa;
-  int fb_lane, fb_unit, fb_pair;
+  int fb_hdr, fb_rec, fb_ext;
   // triangular solves: n_srounds rounds, forward then backward.  A round
   // gives every lane one target z[tgt] -= sum LU[a] z[x] (backward: then
   // times its reciprocal pivot when bit 31 of the second word is set): record

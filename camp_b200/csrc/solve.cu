@@ -130,17 +130,14 @@ struct Tab {
   const uint16_t *fg_unit, *fg_lane, *fg_split;
   const uint32_t* jg_w0;
   const uint16_t *jg_w1, *jg_ptr, *jg_mid, *jg_lupos, *jg_row, *jg_lane, *jg_slots;
-  const uint16_t *lu_iperm, *lu_diag, *lu_src, *fa_ptr;
-  const uint32_t* fa;
-  const uint16_t* fb_lane;
-  const uint32_t *fb_unit, *fb_pair;
+  const uint16_t *lu_iperm, *lu_diag;
   const uint16_t* dep_state;
   const double* atol;
   const uint16_t *lu_rowptr, *lu_col;
   const uint32_t *upd_ptr, *upd;
   const uint16_t *si_rec, *si_elem, *jg_umid, *aq_rec, *aq_sp, *aq_cp;
   const double *si_ef, *aq_sm, *aq_cpm, *aq_sim;
-  int n, n_rxn, n_jac, n_lu, n_fsplit, n_plev, n_flev, n_blev, n_simpol, has_ug, n_aq;
+  int n, n_rxn, n_jac, n_lu, n_fsplit, n_simpol, has_ug, n_aq;
 };
 
 __device__ __forceinline__ Tab make_tab(const char* b) {
@@ -163,9 +160,6 @@ __device__ __forceinline__ Tab make_tab(const char* b) {
   t.jg_slots = (const uint16_t*)(b + o.jg_slots);
   t.lu_iperm = (const uint16_t*)(b + o.lu_iperm);
   t.lu_diag = (const uint16_t*)(b + o.lu_diag);
-  t.lu_src = (const uint16_t*)(b + o.lu_src);
-  t.fa_ptr = (const uint16_t*)(b + o.fa_ptr);
-  t.fa = (const uint32_t*)(b + o.fa);
   t.si_rec = (const uint16_t*)(b + o.si_rec);
   t.si_elem = (const uint16_t*)(b + o.si_elem);
   t.si_ef = (const double*)(b + o.si_ef);
@@ -179,9 +173,6 @@ __device__ __forceinline__ Tab make_tab(const char* b) {
   t.aq_cp = (const uint16_t*)(b + o.aq_cp);
   t.aq_cpm = (const double*)(b + o.aq_cpm);
   t.n_aq = o.n_aq;
-  t.fb_lane = (const uint16_t*)(b + o.fb_lane);
-  t.fb_unit = (const uint32_t*)(b + o.fb_unit);
-  t.fb_pair = (const uint32_t*)(b + o.fb_pair);
   t.dep_state = (const uint16_t*)(b + o.dep_state);
   t.atol = (const double*)(b + o.atol);
   t.lu_rowptr = (const uint16_t*)(b + o.lu_rowptr);
@@ -193,9 +184,6 @@ __device__ __forceinline__ Tab make_tab(const char* b) {
   t.n_jac = o.n_jac;
   t.n_lu = o.n_lu;
   t.n_fsplit = o.n_fsplit;
-  t.n_plev = o.n_plev;
-  t.n_flev = o.n_flev;
-  t.n_blev = o.n_blev;
   return t;
 }
 
@@ -965,84 +953,105 @@ __device__ __forceinline__ bool has_simpol(const char* tb) {
 // ---------------------------------------------------------------------------
 // LU of M = I - gamma*J on the fixed order, and the triangular solves
 // ---------------------------------------------------------------------------
-// One level of the factorization: every unit of this lane subtracts its pair
-// products from its target, LU[target] -= sum LU[pa] * LU[pb].  A unit that
-// carries a pivot then stores the reciprocal of its final value, the pivot,
-// in dinv; the return value flags a zero or non-finite pivot.
-template <typename LT>
-__device__ __forceinline__ bool grouped_level(const uint16_t* rnd, const uint32_t* rec,
-                                              const uint32_t* pair, int level, LT* LU, LT* dinv,
-                                              int lane) {
-  // Round r hands this lane the record rec[32 r + lane]; a no-op record
-  // targets the spare slot with no pairs and no pivot, so every lane runs the
-  // same code.
-  bool bad = false;
-  const uint2* rec2 = (const uint2*)rec;
-  const int r1 = rnd[level + 1];
-  #pragma unroll 1
-  for (int r = rnd[level]; r < r1; ++r) {
-    const uint2 w = rec2[32 * r + lane];
-    const int tgt = w.x & 0xFFFFu, cnt = w.x >> 16;
-    const int p0 = w.y & 0xFFFFu, piv = w.y >> 16;
-    LT s0 = LU[tgt], s1 = (LT)0;
-    int p = p0;
-    #pragma unroll 1
-    for (; p + 1 < p0 + cnt; p += 2) {
-      const uint32_t q0 = pair[p], q1 = pair[p + 1];
-      s0 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
-      s1 -= LU[q1 & 0xFFFFu] * LU[q1 >> 16];
-    }
-    if (p < p0 + cnt) {
-      const uint32_t q0 = pair[p];
-      s0 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
-    }
-    LT s = s0 + s1;
-    if (piv) {
-      const bool pbad = (s == (LT)0) || !isfinite((double)s);
-      bad |= pbad;
-      dinv[piv - 1] = pbad ? (LT)0 : (LT)1 / s;
-    }
-    LU[tgt] = s;
-  }
-  return bad;
-}
-
 // M = I - gamma*J scattered into the LU pattern, then a right-looking
-// factorization level by level: reciprocal pivots of the level, scaled L
-// columns, Schur updates grouped by target.  Returns false on a zero or
-// non-finite pivot.
+// factorization level by level: L columns scaled by the level's reciprocal
+// pivots, then its Schur updates grouped by target, a target that becomes a
+// pivot of the next level storing its reciprocal in dinv.  Returns false on a
+// zero or non-finite pivot.
+// Bound by latency and instruction count (cb05cl_ae5: 23 levels, 60 rounds of
+// at most 32 targets, mostly of one pair), so a round is one record load per
+// lane, loaded one round ahead, the first pair in the record and the pair
+// count in a header that every lane reads.
 template <typename LT>
 __device__ __noinline__ bool dev_form_factor(const char* tb, const LT* J, double gamma,
                                              LT* LU, LT* dinv, int lane) {
-  const Tab t = make_tab(tb);
-  // M = I - gamma*J in one pass over the LU positions (fill-in starts at 0)
-  #pragma unroll 1
-  for (int q = lane; q < t.n_lu; q += 32) {
-    const uint32_t src = t.lu_src[q];
-    const int e = (int)(src & 0x7FFFu) - 1;
-    LT v = e >= 0 ? (LT)(-gamma * (double)J[e]) : (LT)0;
-    if (src & 0x8000u) v += (LT)1;
-    LU[q] = v;
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  // M = I - gamma*J in one pass over the LU positions (fill-in starts at 0),
+  // four loads of J (global memory) in flight
+  {
+    const uint16_t* lu_src = (const uint16_t*)(tb + o.lu_src);
+    const int n_lu = o.n_lu;
+    #pragma unroll 1
+    for (int q = lane; q < n_lu; q += 128) {
+      uint32_t src[4];
+      LT v[4];
+      #pragma unroll
+      for (int k = 0; k < 4; ++k) src[k] = q + 32 * k < n_lu ? lu_src[q + 32 * k] : 0u;
+      #pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = (src[k] & 0x7FFFu) ? J[(src[k] & 0x7FFFu) - 1] : (LT)0;
+      #pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (q + 32 * k < n_lu) {
+          LT m = (src[k] & 0x7FFFu) ? (LT)(-gamma * (double)v[k]) : (LT)0;
+          if (src[k] & 0x8000u) m += (LT)1;
+          LU[q + 32 * k] = m;
+        }
+    }
   }
   __syncwarp();
-  bool bad = grouped_level<LT>(t.fb_lane, t.fb_unit, t.fb_pair, 0, LU, dinv, lane);
-  __syncwarp();
+  const uint16_t* hdr = (const uint16_t*)(tb + o.fb_hdr);
+  const uint2* rec = (const uint2*)(tb + o.fb_rec) + lane;
+  const uint32_t* ext = (const uint32_t*)(tb + o.fb_ext) + lane;
+  const uint16_t* fa_ptr = (const uint16_t*)(tb + o.fa_ptr);
+  const uint32_t* fa = (const uint32_t*)(tb + o.fa);
+  const int n_plev = o.n_plev;
+  bool bad = false;
+  uint2 w = *rec;
+  unsigned h = *hdr;
+  int fa0 = 0;
   #pragma unroll 1
-  for (int lv = 0; lv < t.n_plev; ++lv) {
-    const int a1 = t.fa_ptr[lv + 1];
+  for (int lv = 0;; ++lv) {
+    unsigned last;
     #pragma unroll 1
-    for (int i = t.fa_ptr[lv] + lane; i < a1; i += 32) {
-      const uint32_t w = t.fa[i];
-      LU[w & 0xFFFFu] *= dinv[w >> 16];
-    }
+    do {
+      rec += 32;
+      ++hdr;
+      const uint2 wn = *rec;
+      const unsigned hn = *hdr;
+      const int tgt = w.y & 0xFFFFu, piv = w.y >> 16, cnt = h & 0x7FFFu;
+      LT s0 = LU[tgt], s1 = (LT)0;
+      s0 -= LU[w.x & 0xFFFFu] * LU[w.x >> 16];
+      if (cnt > 1) {
+        int p = 1;
+        #pragma unroll 1
+        for (; p + 1 < cnt; p += 2, ext += 64) {
+          const uint32_t q0 = ext[0], q1 = ext[32];
+          s1 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
+          s0 -= LU[q1 & 0xFFFFu] * LU[q1 >> 16];
+        }
+        if (p < cnt) {
+          const uint32_t q0 = ext[0];
+          s1 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
+          ext += 32;
+        }
+      }
+      const LT s = s0 + s1;
+      if (piv) {
+        const bool pbad = (s == (LT)0) || !isfinite((double)s);
+        bad |= pbad;
+        dinv[piv - 1] = pbad ? (LT)0 : (LT)1 / s;
+      }
+      LU[tgt] = s;
+      last = h & 0x8000u;
+      w = wn;
+      h = hn;
+    } while (!last);
     __syncwarp();
-    bad |= grouped_level<LT>(t.fb_lane, t.fb_unit, t.fb_pair, lv + 1, LU, dinv, lane);
+    if (lv == n_plev) break;
+    const int fa1 = fa_ptr[lv + 1];
+    #pragma unroll 1
+    for (int i = fa0 + lane; i < fa1; i += 32) {
+      const uint32_t e = fa[i];
+      LU[e & 0xFFFFu] *= dinv[e >> 16];
+    }
+    fa0 = fa1;
     __syncwarp();
   }
   return !warp_any(bad);
 }
 
-// The spare slots that the padding of the solve rounds reads and writes.
+// The spare slots that the padding of the rounds reads and writes (zero, and
+// zero minus products of zeros stays zero).
 template <typename LT>
 __device__ __forceinline__ void clear_spare(const char* tb, LT* LU, LT* z, int lane) {
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
