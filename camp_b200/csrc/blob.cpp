@@ -43,6 +43,133 @@ std::vector<std::vector<int>> lpt(const std::vector<long>& weight) {
   return lanes;
 }
 
+// One item of the f or J gather: index | coef<<16 entries of its sums (a loss
+// or an unguarded product carries the coefficient 1)
+struct GatherItem {
+  int id = 0, tag = 0xFFFF;
+  std::vector<uint32_t> lead, loss, prod;
+  std::vector<uint32_t> neg;  // f: guarded losses, after the others into L1
+  // the four chains: losses alternate between L0 and L1, products between P0,
+  // which starts with the unguarded ones, and P1
+  std::vector<uint32_t> chain(int c) const {
+    std::vector<uint32_t> o;
+    const std::vector<uint32_t>& v = c < 2 ? loss : prod;
+    if (c == 2) o = lead;
+    for (size_t k = c & 1; k < v.size(); k += 2) o.push_back(v[k]);
+    if (c == 1) o.insert(o.end(), neg.begin(), neg.end());
+    return o;
+  }
+  int longest() const {
+    size_t m = 0;
+    for (int c = 0; c < 4; ++c) m = std::max(m, chain(c).size());
+    return (int)m;
+  }
+};
+
+struct GatherTables {
+  std::vector<uint32_t> a_rec, a_ent, b_hdr, b_id, b_ent, neg;
+};
+
+// Splits the items into rounds of eight with a lane per chain and rounds of 32
+// with a lane per item (blob.hpp).  A chain round costs its longest chain (11
+// instructions an entry, 45 for the reduction), an item round its longest
+// lists (9 a word, 30 besides) and their padded words; with the longest chains
+// first, the number of chain rounds with the least sum is taken,
+// `bytes_per_inst` table bytes counting as one instruction.
+void pack_gather(std::vector<GatherItem> items, uint32_t zero, int bytes_per_inst,
+                 GatherTables* o) {
+  std::stable_sort(items.begin(), items.end(), [](const GatherItem& a, const GatherItem& b) {
+    return !a.neg.empty() != !b.neg.empty() ? !a.neg.empty() : a.longest() > b.longest();
+  });
+  auto half = [](size_t n) { return (int)(n + 1) / 2; };
+  auto up = [](int n, int m) { return (n + m - 1) / m * m; };
+  // the items from `first` on in rounds of 32, similar lists together
+  auto rest = [&](size_t first) {
+    std::vector<const GatherItem*> r;
+    for (size_t k = first; k < items.size(); ++k) r.push_back(&items[k]);
+    std::stable_sort(r.begin(), r.end(), [&](const GatherItem* a, const GatherItem* b) {
+      auto w = [&](const GatherItem* x) {
+        return up(half(x->loss.size()), 2) + up((int)x->prod.size(), 2) + (int)x->lead.size();
+      };
+      return w(a) > w(b);
+    });
+    return r;
+  };
+  struct Steps {
+    int u = 0, l = 0, p = 0;
+  };
+  auto steps = [&](const std::vector<const GatherItem*>& r, size_t k0) {
+    Steps s;
+    for (size_t k = k0; k < std::min(r.size(), k0 + kLanes); ++k) {
+      s.u = std::max(s.u, (int)r[k]->lead.size());
+      s.l = std::max(s.l, half(r[k]->loss.size()));
+      s.p = std::max(s.p, (int)r[k]->prod.size());
+    }
+    s.l = s.l > 1 ? up(s.l, 2) : s.l;
+    s.p = s.p > 1 ? up(s.p, 2) : s.p;
+    return s;
+  };
+  size_t n_neg = 0;
+  while (n_neg < items.size() && !items[n_neg].neg.empty()) ++n_neg;
+  const size_t r_min = (n_neg + 7) / 8;
+  size_t best_r = r_min;
+  long best = -1, chains = 0;
+  for (size_t ra = 0; ra * 8 < items.size() + 8; ++ra) {
+    if (ra > 0 && (ra - 1) * 8 < items.size()) {
+      long len = 0, bytes = 32 * 8;
+      for (size_t k = 8 * (ra - 1); k < std::min(items.size(), 8 * ra); ++k) {
+        len = std::max(len, (long)up(items[k].longest(), 4));
+        for (int c = 0; c < 4; ++c) bytes += 4 * up((int)items[k].chain(c).size(), 4);
+      }
+      chains += 45 + 11 * len + bytes / bytes_per_inst;
+    }
+    if (ra < r_min) continue;
+    const auto r = rest(8 * ra);
+    long cost = chains;
+    for (size_t k = 0; k < r.size(); k += kLanes) {
+      const Steps s = steps(r, k);
+      cost += 30 + 9 * (s.u + s.l + s.p) + 128L * (1 + s.u + s.l + s.p) / bytes_per_inst;
+    }
+    if (best < 0 || cost < best) {
+      best = cost;
+      best_r = ra;
+    }
+  }
+  for (size_t k = 0; k < 8 * best_r; ++k) {
+    for (int c = 0; c < 4; ++c) {
+      std::vector<uint32_t> e;
+      if (k < items.size()) e = items[k].chain(c);
+      e.resize(up((int)e.size(), 4), zero);
+      o->a_rec.push_back((uint32_t)o->a_ent.size() | ((uint32_t)e.size() << 16));
+      o->a_rec.push_back(k < items.size()
+                             ? (uint32_t)items[k].id | ((uint32_t)items[k].tag << 16)
+                             : 0xFFFFu);
+      o->a_ent.insert(o->a_ent.end(), e.begin(), e.end());
+    }
+  }
+  const auto r = rest(8 * best_r);
+  for (size_t k0 = 0; k0 < r.size(); k0 += kLanes) {
+    const Steps s = steps(r, k0);
+    o->b_hdr.push_back((uint32_t)s.l | ((uint32_t)s.p << 16));
+    o->b_hdr.push_back((uint32_t)s.u);
+    auto at = [&](const std::vector<uint32_t> GatherItem::*list, size_t k, size_t j) {
+      return k < r.size() && j < (r[k]->*list).size() ? (r[k]->*list)[j] : zero;
+    };
+    for (size_t k = k0; k < k0 + kLanes; ++k)
+      o->b_id.push_back(k < r.size() ? (uint32_t)r[k]->id | ((uint32_t)r[k]->tag << 16) : 0xFFFFu);
+    for (int j = 0; j < s.u; ++j)
+      for (size_t k = k0; k < k0 + kLanes; ++k) o->b_ent.push_back(at(&GatherItem::lead, k, j));
+    for (int j = 0; j < s.l; ++j)
+      for (size_t k = k0; k < k0 + kLanes; ++k)
+        o->b_ent.push_back((at(&GatherItem::loss, k, 2 * j) & 0xFFFFu) |
+                           (at(&GatherItem::loss, k, 2 * j + 1) << 16));
+    for (int j = 0; j < s.p; ++j)
+      for (size_t k = k0; k < k0 + kLanes; ++k) o->b_ent.push_back(at(&GatherItem::prod, k, j));
+  }
+  o->a_ent.resize(o->a_ent.size() + 4, zero);  // read ahead, never used
+  o->b_ent.resize(o->b_ent.size() + 2 * kLanes, zero);
+}
+
 }  // namespace
 
 bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vector<uint8_t>* blob,
@@ -52,7 +179,8 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     *err = "more than 1023 dependent variables";
     return false;
   }
-  if (t.n_rates > 65535 || t.n_keff > 65535 || t.n_part_all > 65535 || t.n_lu > 65535 ||
+  if (t.n_rates + t.n_cv > 65535 || t.n_keff > 65535 ||
+      t.n_part_all + t.n_cv + t.n_pj + t.n_virt > 65535 || t.n_lu > 65535 ||
       t.n_jac > 65535 ||
       (int)t.fg_rxn.size() > 65535 || (int)t.jg_part.size() > 65535 ||
       (int)t.fa_pos.size() > 65535) {
@@ -83,6 +211,7 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     }
     uint32_t w = (uint32_t)(v1 - v0) << 30;
     for (int k = 0; k < v1 - v0; ++k) w |= (uint32_t)t.rx_vdep[v0 + k] << (10 * k);
+    for (int k = v1 - v0; k < 2; ++k) w |= (uint32_t)n << (10 * k);
     rx_word[r] = w;
     rx_vptr[r] = (uint16_t)v0;
   }
@@ -155,6 +284,29 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     }
   }
   fg_lane[kLanes] = (uint16_t)(fg_unit.size() / 8);
+  // the same units as chains and rounds (blob.hpp)
+  const uint32_t one = (uint32_t)coef_id(1.0) << 16;
+  const int f_zero = t.n_rates + t.n_cv;
+  GatherTables fgt;
+  {
+    std::vector<GatherItem> items;
+    for (const Unit& x : units) {
+      const int m1 = clampi(grp_end[2 * x.sp], x.b, x.e);
+      const int m2 = clampi(grp_end[2 * x.sp + 1], x.b, x.e);
+      GatherItem it;
+      it.id = x.sp;
+      it.tag = x.slot;
+      for (int k = x.b; k < m1; ++k) it.loss.push_back((fg_ent[k] & 0xFFFFu) | one);
+      for (int k = m1; k < m2; ++k) it.prod.push_back(fg_ent[k] & 0x7FFFFFFFu);
+      for (int k = m2; k < x.e; ++k) {
+        fgt.neg.push_back(fg_ent[k] & 0x7FFFFFFFu);
+        fgt.neg.push_back((uint32_t)x.sp);
+        it.neg.push_back((uint32_t)(f_zero + (int)fgt.neg.size() / 2) | one);
+      }
+      items.push_back(it);
+    }
+    pack_gather(items, (uint32_t)f_zero, 16, &fgt);
+  }
   // J gather: each slot's partials regrouped: unguarded products (SIMPOL,
   // into the production part), losses (into the loss part) and guarded
   // products (into the production part); jg_umid[e] / jg_mid[e] are the
@@ -243,6 +395,37 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     for (int e : s) jg_slots.push_back((uint16_t)e);
   }
   jg_lane[kLanes] = (uint16_t)jg_slots.size();
+  // the same slots as chains and rounds (blob.hpp); a Jacobian is evaluated a
+  // few times less often than f, so its table bytes weigh more
+  const int j_zero = t.n_part_all + t.n_cv + t.n_pj + t.n_virt;
+  GatherTables jgt;
+  {
+    std::vector<GatherItem> items;
+    for (int e = 0; e < t.n_jac; ++e) {
+      GatherItem it;
+      it.id = e;
+      for (int g = t.jg_ptr[e]; g < jg_umid[e]; ++g)
+        it.lead.push_back((jg_w0[g] & 0xFFFFu) | one);
+      for (int g = jg_umid[e]; g < jg_mid[e]; ++g)
+        it.loss.push_back((jg_w0[g] & 0xFFFFu) | one);
+      for (int g = jg_mid[e]; g < t.jg_ptr[e + 1]; ++g) {
+        if (coef[jg_w0[g] >> 16] >= 0.0) {
+          it.prod.push_back(jg_w0[g]);
+          continue;
+        }
+        jgt.neg.push_back(jg_w0[g]);
+        jgt.neg.push_back((uint32_t)(jg_w1[g] - 1) | ((uint32_t)t.jg_row[e] << 16));
+        it.prod.push_back((uint32_t)(j_zero + (int)jgt.neg.size() / 2) | one);
+      }
+      items.push_back(it);
+    }
+    pack_gather(items, (uint32_t)j_zero, 8, &jgt);
+  }
+  if (fgt.a_ent.size() > 65535 || jgt.a_ent.size() > 65535 ||
+      f_zero + fgt.neg.size() / 2 > 65535 || j_zero + jgt.neg.size() / 2 > 65535) {
+    *err = "mechanism exceeds the 16-bit table encodings";
+    return false;
+  }
   // LU
   auto u16 = [](const std::vector<int>& v) {
     std::vector<uint16_t> o(v.size());
@@ -342,21 +525,25 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   o.n_flev = t.n_flev;
   o.n_blev = t.n_blev;
   o.rx_word = w.put(rx_word);
-  o.rx_vptr = w.put(rx_vptr);
   o.coef = w.put(coef);
-  o.fg_ent = w.put(fg_ent);
-  o.fg_unit = w.put(fg_unit);
-  o.fg_lane = w.put(fg_lane);
   o.fg_split = w.put(split);
-  o.jg_w0 = w.put(jg_w0);
-  o.jg_w1 = w.put(jg_w1);
-  o.jg_ptr = w.put(jg_ptr);
-  o.jg_mid = w.put(jg_mid);
-  o.jg_row = w.put(jg_row);
-  o.jg_lane = w.put(jg_lane);
-  o.jg_slots = w.put(jg_slots);
+  o.rx_vptr = w.put(rx_vptr);
+  for (int k = 0; k < 2; ++k) {
+    GatherTables& x = k == 0 ? fgt : jgt;
+    BlobOff::Gather& g = o.g[k];
+    g.n_a = (int)x.a_rec.size() / (2 * kLanes);
+    g.n_b = (int)x.b_hdr.size() / 2;
+    g.n_neg = (int)x.neg.size() / 2;
+    g.zero = k == 0 ? f_zero : j_zero;
+    g.a_rec = w.put(x.a_rec);
+    g.a_ent = w.put(x.a_ent);
+    g.b_hdr = w.put(x.b_hdr);
+    g.b_id = k == 0 ? w.put(x.b_id)
+                    : w.put(std::vector<uint16_t>(x.b_id.begin(), x.b_id.end()));
+    g.b_ent = w.put(x.b_ent);
+    g.neg = w.put(x.neg);
+  }
   o.has_ug = has_ug ? 1 : 0;
-  o.jg_umid = w.put(jg_umid);
   o.n_simpol = t.n_simpol;
   o.n_keff = t.n_keff;
   o.n_rates = t.n_rates;
@@ -463,8 +650,9 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   o.sv_ext = w.put(svr.ext);
   o.dep_state = w.put(u16(t.dep_state));
   o.atol = w.put(atol_dep);
-  // the one-lane LU tables come last: the level-scheduled mode stages only
-  // the bytes before them into shared memory
+  // the level-scheduled mode stages only the bytes up to here into shared
+  // memory, the one-lane LU mode its LU tables too; the f gather for any
+  // signs and the J gather come last and stay in global memory
   w.buf.resize((w.buf.size() + 15) & ~size_t(15), 0);
   o.stage_bytes = (int)w.buf.size();
   {
@@ -478,6 +666,19 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     o.upd_ptr = w.put(up);
     o.upd = w.put(ud);
   }
+  w.buf.resize((w.buf.size() + 15) & ~size_t(15), 0);
+  o.seq_bytes = (int)w.buf.size();
+  o.fg_ent = w.put(fg_ent);
+  o.fg_unit = w.put(fg_unit);
+  o.fg_lane = w.put(fg_lane);
+  o.jg_w0 = w.put(jg_w0);
+  o.jg_w1 = w.put(jg_w1);
+  o.jg_ptr = w.put(jg_ptr);
+  o.jg_mid = w.put(jg_mid);
+  o.jg_row = w.put(jg_row);
+  o.jg_lane = w.put(jg_lane);
+  o.jg_slots = w.put(jg_slots);
+  o.jg_umid = w.put(jg_umid);
   w.buf.resize((w.buf.size() + 15) & ~size_t(15), 0);
   o.bytes = (int)w.buf.size();
   memcpy(w.buf.data(), &o, sizeof(o));

@@ -13,20 +13,46 @@ namespace campb {
 
 struct BlobOff {
   int bytes;        // whole blob
-  int stage_bytes;  // prefix the level-scheduled mode stages (all but the one-lane LU)
+  int stage_bytes;  // prefix the level-scheduled mode stages
+  int seq_bytes;    // prefix the one-lane LU mode stages (its LU tables too)
   // counts
   int n, n_rxn, n_part, n_jac, n_lu, n_coef, n_funits, n_fsplit, n_fscratch;
   int n_plev, n_flev, n_blev;
-  // reactions: variable reactants packed (nv<<30 | d2<<20 | d1<<10 | d0), partial base
+  // reactions: variable reactants packed (nv<<30 | d2<<20 | d1<<10 | d0; d0
+  // and d1 default to n, where y holds 1), partial base
   int rx_word, rx_vptr;
   // coefficient table (double)
   int coef;
-  // f gather: entries (rxn | coef<<16 | prod<<31), units (species, begin, end,
-  // slot) as 4 x uint16, lane pointers (33 x uint16), split species (species,
-  // first slot, count) as 3 x uint16
+  // f gather for any signs: entries (rxn | coef<<16 | prod<<31), units
+  // (species, begin, end of losses, end of non-negative-yield products, end,
+  // slot) as 8 x uint16, lane pointers (33 x uint16); read from the blob in
+  // global memory (self).  Split species (species, first slot, count) as 3 x
+  // uint16
   int fg_ent, fg_unit, fg_lane, fg_split;
-  // J gather: w0 = part | coef<<16, w1 = independent species + 1 (0 = loss
-  // entry); per slot: entry pointer, LU position, row; lane slot lists
+  // f (g[0]) and J (g[1]) gathers where no rate (partial), concentration or
+  // step is negative; every item is a unit of the f gather or a slot of the
+  // solver Jacobian, its sums L0, L1, P0 and P1 four chains of entries (uint32
+  // index | coef<<16).  Long items come first, as n_a rounds of eight items
+  // with one lane per chain: per lane a_rec (uint32 first entry | entries<<16,
+  // id | tag<<16) into a_ent (lists of a multiple of four).  The rest follows
+  // as n_b rounds of 32 items, one lane each: per round b_hdr (uint32 x 2:
+  // words of loss pairs | products<<16, leading unguarded products), per lane
+  // b_id (f: uint32 id | tag<<16, J: uint16 id), and in b_ent, 32 lanes at a
+  // time, the unguarded products, the loss pairs (uint32 index | index<<16) and
+  // the products, both a multiple of two.  Padding uses an index that the
+  // gather keeps at zero; four entries and two rows are read ahead of the ends.
+  // Terms with a negative yield are evaluated before the gather, n_neg records
+  // (uint32 index | coef<<16; f: species, J: guard species | row<<16), into
+  // the slots after that zero.
+  // f: id species, tag split slot (0xFFFF none); J: id slot; idle lanes have
+  // id 0xFFFF.
+  struct Gather {
+    int n_a, n_b, n_neg, zero, a_rec, a_ent, b_hdr, b_id, b_ent, neg;
+  } g[2];
+  unsigned long long self;  // the blob's own address in global memory
+  // J gather for any signs: w0 = part | coef<<16, w1 = independent species + 1
+  // (0 = loss entry); per slot: entry pointer, LU position, row; lane slot
+  // lists.  Read from the blob in global memory (self).
   int jg_w0, jg_w1, jg_ptr, jg_mid, jg_lupos, jg_row, jg_lane, jg_slots;
   // LU: dependent index -> pivot row (iperm), diag (uint16); factorization by
   // pivot level: scaled L entries (fa_ptr uint16, fa = pos | pivot<<16),

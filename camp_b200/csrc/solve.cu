@@ -103,10 +103,29 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// The block's dynamic shared memory: the staged tables, then a slab per cell.
+extern __shared__ __align__(16) char g_smem[];
+
+// A pointer into it, told to the compiler as such: the device functions below
+// are compiled out of line, and without this the address space of their
+// arguments is known only as far as it happens to be inferred.
+template <typename T>
+__device__ __forceinline__ T* sh(T* p) {
+  return (T*)(g_smem + ((unsigned)__cvta_generic_to_shared(p) -
+                        (unsigned)__cvta_generic_to_shared(g_smem)));
+}
+
 // value the reference's f sees for a solver variable: y above -SMALL is used
 // as is, anything else (only exactly -SMALL reaches here) becomes TINY
 // (src/camp_solver.c:805-833)
 __device__ __forceinline__ double state_of(double y) { return y > -kSmall ? y : kTiny; }
+
+// y[n] = 1: the absent reactants of f's rates (the concentrations themselves
+// never reach y[n])
+__device__ __forceinline__ void set_unit(double* y, int n, int lane) {
+  if (lane == 0) y[n] = 1.0;
+  __syncwarp();
+}
 
 // Device loops carry `#pragma unroll 1` unless unrolling is wanted: the
 // solve kernel is bound by instruction fetch (a warp per cell, each at its own
@@ -117,6 +136,32 @@ __device__ __forceinline__ double state_of(double y) { return y > -kSmall ? y : 
 __device__ __noinline__ double dpow(double x, double y) { return pow(x, y); }
 __device__ __noinline__ double ddiv(double a, double b) { return a / b; }
 __device__ __noinline__ double dsqrt(double a) { return sqrt(a); }
+
+// sqrt(s / n) with n a small whole number and rn = 1 / n rounded to nearest:
+// one residual step makes s * rn the correctly rounded quotient (Markstein,
+// IBM J. Res. Dev. 34, 1990) at a fifth of a division's latency, away from
+// the ends of the exponent range
+__device__ __noinline__ double rms(double s, double n, double rn) {
+  double q = s * rn;
+  q = fma(fma(-q, n, s), rn, q);
+  if (!(s > 1.0e-250 && s < 1.0e250)) q = s / n;
+  return sqrt(q);
+}
+
+// 1 / j for j = 0..7 (0: unused) and the sum -1 - 1/2 - ... - 1/q for
+// q = 0..5, each term subtracted in turn: the divisions of the method's
+// coefficients by whole numbers, with their roundings
+__constant__ double kInvInt[8] = {0.0,       1.0,       1.0 / 2.0, 1.0 / 3.0,
+                                  1.0 / 4.0, 1.0 / 5.0, 1.0 / 6.0, 1.0 / 7.0};
+__constant__ double kAlpha0[6] = {
+    -1.0, -1.0, -1.0 - 1.0 / 2.0, -1.0 - 1.0 / 2.0 - 1.0 / 3.0,
+    -1.0 - 1.0 / 2.0 - 1.0 / 3.0 - 1.0 / 4.0,
+    -1.0 - 1.0 / 2.0 - 1.0 / 3.0 - 1.0 / 4.0 - 1.0 / 5.0};
+// above kNoGrowth[k], x^(1/k) + ADDON is certainly above 1 / THRESH, so a step
+// size ratio 1 / (x^(1/k) + ADDON) is below THRESH and leaves the step as it is
+// (0.66667^k; 1 / THRESH - ADDON = 0.6666657)
+__constant__ double kNoGrowth[8] = {0.0,         0.66667,    0.44444889, 0.29630075,
+                                    0.19753482, 0.13169054, 0.08779414, 0.0};
 
 
 // ---------------------------------------------------------------------------
@@ -142,28 +187,29 @@ struct Tab {
 
 __device__ __forceinline__ Tab make_tab(const char* b) {
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(b);
+  const char* g = (const char*)o.self;  // the tables that are not staged
   Tab t;
   t.rx_word = (const uint32_t*)(b + o.rx_word);
   t.rx_vptr = (const uint16_t*)(b + o.rx_vptr);
   t.coef = (const double*)(b + o.coef);
-  t.fg_ent = (const uint32_t*)(b + o.fg_ent);
-  t.fg_unit = (const uint16_t*)(b + o.fg_unit);
-  t.fg_lane = (const uint16_t*)(b + o.fg_lane);
+  t.fg_ent = (const uint32_t*)(g + o.fg_ent);
+  t.fg_unit = (const uint16_t*)(g + o.fg_unit);
+  t.fg_lane = (const uint16_t*)(g + o.fg_lane);
   t.fg_split = (const uint16_t*)(b + o.fg_split);
-  t.jg_w0 = (const uint32_t*)(b + o.jg_w0);
-  t.jg_w1 = (const uint16_t*)(b + o.jg_w1);
-  t.jg_ptr = (const uint16_t*)(b + o.jg_ptr);
-  t.jg_mid = (const uint16_t*)(b + o.jg_mid);
+  t.jg_w0 = (const uint32_t*)(g + o.jg_w0);
+  t.jg_w1 = (const uint16_t*)(g + o.jg_w1);
+  t.jg_ptr = (const uint16_t*)(g + o.jg_ptr);
+  t.jg_mid = (const uint16_t*)(g + o.jg_mid);
   t.jg_lupos = (const uint16_t*)(b + o.jg_lupos);
-  t.jg_row = (const uint16_t*)(b + o.jg_row);
-  t.jg_lane = (const uint16_t*)(b + o.jg_lane);
-  t.jg_slots = (const uint16_t*)(b + o.jg_slots);
+  t.jg_row = (const uint16_t*)(g + o.jg_row);
+  t.jg_lane = (const uint16_t*)(g + o.jg_lane);
+  t.jg_slots = (const uint16_t*)(g + o.jg_slots);
   t.lu_iperm = (const uint16_t*)(b + o.lu_iperm);
   t.lu_diag = (const uint16_t*)(b + o.lu_diag);
   t.si_rec = (const uint16_t*)(b + o.si_rec);
   t.si_elem = (const uint16_t*)(b + o.si_elem);
   t.si_ef = (const double*)(b + o.si_ef);
-  t.jg_umid = (const uint16_t*)(b + o.jg_umid);
+  t.jg_umid = (const uint16_t*)(g + o.jg_umid);
   t.n_simpol = o.n_simpol;
   t.has_ug = o.has_ug;
   t.aq_rec = (const uint16_t*)(b + o.aq_rec);
@@ -689,14 +735,32 @@ __device__ __noinline__ void aero_partials(const char* tb, const double* y, cons
   aq_partials(tb, y, keff, cv, part, lane);
 }
 
-// Returns 1 (recoverable) when some y < -SMALL, else writes f into out.
-// When rp/rl are given, the production and loss sums are written too.
-// Species lists are processed in lane-balanced units; lists split over
-// several units are added up in a combine pass (fscr holds their partials).
-__device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
-                                  const double* keff, double* rates, double* fscr,
-                                  double* out, int lane, double* rp = nullptr,
-                                  double* rl = nullptr, bool neg_extra = false) {
+// the species whose lists were split over several units
+__device__ __forceinline__ void f_combine(const char* tb, const double* fscr, double* out,
+                                          int lane, double* rp, double* rl) {
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  const uint16_t* split = (const uint16_t*)(tb + o.fg_split);
+  #pragma unroll 1
+  for (int s = lane; s < o.n_fsplit; s += 32) {
+    const int sp = split[3 * s], first = split[3 * s + 1], cnt = split[3 * s + 2];
+    double P = 0.0, L = 0.0;
+    #pragma unroll 1
+    for (int j = 0; j < cnt; ++j) {
+      P += fscr[2 * (first + j)];
+      L += fscr[2 * (first + j) + 1];
+    }
+    out[sp] = (P + L != 0.0) ? P - L : 0.0;
+    if (rp) rp[sp] = P;
+    if (rl) rl[sp] = L;
+  }
+  __syncwarp();
+}
+
+// f with any signs; see dev_f
+__device__ __noinline__ int dev_f_any(const char* tb, const double* y, double h,
+                                      const double* keff, double* rates, double* fscr,
+                                      double* out, int lane, double* rp, double* rl,
+                                      bool neg_extra) {
   const Tab t = make_tab(tb);
   bool bad = false;
   #pragma unroll 1
@@ -778,26 +842,185 @@ __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
     }
   }
   __syncwarp();
-  #pragma unroll 1
-  for (int s = lane; s < t.n_fsplit; s += 32) {
-    const int sp = t.fg_split[3 * s], first = t.fg_split[3 * s + 1], cnt = t.fg_split[3 * s + 2];
-    double P = 0.0, L = 0.0;
-    #pragma unroll 1
-    for (int j = 0; j < cnt; ++j) {
-      P += fscr[2 * (first + j)];
-      L += fscr[2 * (first + j) + 1];
-    }
-    out[sp] = (P + L != 0.0) ? P - L : 0.0;
-    if (rp) rp[sp] = P;
-    if (rl) rl[sp] = L;
-  }
-  __syncwarp();
+  f_combine(tb, fscr, out, lane, rp, rl);
   return 0;
 }
 
-// Solver Jacobian values into Jout (indexed by CSC entry; each lane writes the
-// entries of its balanced slot list); production and loss parts into jp/jl
-// when given (src/rxns/rxn_arrhenius.c:178-212).
+// Sums of every item of the f (k = 0) or J (k = 1) gather (blob.hpp) from the
+// terms in src, f into out (fscr for the parts of a split species), J into
+// Jout by CSC entry; production and loss parts into rp / rl when given.
+//
+// No term here is negative, so each one's sum is known, and the step counts of
+// a round are the same in every lane: the long lists (some tens of terms) a
+// chain of sums per lane, the short ones an item per lane (the split is chosen
+// in blob.cpp).  Bound by shared-memory latency: the loads of several entries
+// are issued together, their words a step ahead.  One copy of the code for f
+// and J, as the kernel is short of instruction cache.
+template <typename JT>
+__device__ __noinline__ void gather(int k, const double* src, double* out, double* fscr,
+                                    JT* Jout, int lane, double* rp, double* rl) {
+  src = sh(src);
+  const char* const tb = g_smem;
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  const BlobOff::Gather& g = o.g[k];
+  const double* coef = (const double*)(tb + o.coef);
+  auto term = [&](uint32_t q) { return __dmul_rn(src[q & 0xFFFFu], coef[q >> 16]); };
+  auto put = [&](int id, int tag, double P, double L) {
+    if (k) {
+      Jout[id] = (JT)(P - L);
+    } else if (tag == 0xFFFF) {
+      sh(out)[id] = (P + L != 0.0) ? P - L : 0.0;
+    } else {
+      sh(fscr)[2 * tag] = P;
+      sh(fscr)[2 * tag + 1] = L;
+      return;
+    }
+    if (rp) rp[id] = P;
+    if (rl) rl[id] = L;
+  };
+  {
+    const uint2* rec = (const uint2*)(tb + g.a_rec) + lane;
+    const uint32_t* ent = (const uint32_t*)(tb + g.a_ent);
+    #pragma unroll 1
+    for (int r = g.n_a; r > 0; --r, rec += 32) {
+      const uint2 w = *rec;
+      const uint32_t* e = ent + (w.x & 0xFFFFu);
+      uint32_t q0 = e[0], q1 = e[1], q2 = e[2], q3 = e[3];
+      double s = 0.0;
+      #pragma unroll 1
+      for (int c = w.x >> 16; c > 0; c -= 4) {
+        e += 4;
+        const double v0 = term(q0), v1 = term(q1), v2 = term(q2), v3 = term(q3);
+        q0 = e[0];
+        q1 = e[1];
+        q2 = e[2];
+        q3 = e[3];
+        s += v0;
+        s += v1;
+        s += v2;
+        s += v3;
+      }
+      __syncwarp();
+      s += __shfl_xor_sync(FULLMASK, s, 1);  // L0 + L1, P0 + P1
+      const double P = __shfl_xor_sync(FULLMASK, s, 2);
+      const int id = w.y & 0xFFFFu;
+      if (id != 0xFFFF && (lane & 3) == 0) put(id, w.y >> 16, P, s);
+    }
+  }
+  const uint2* hdr = (const uint2*)(tb + g.b_hdr);
+  const uint32_t* st = (const uint32_t*)(tb + g.b_ent) + lane;
+  uint32_t q0 = st[0], q1 = st[32];
+  #pragma unroll 1
+  for (int r = 0; r < g.n_b; ++r) {
+    const uint2 hd = hdr[r];
+    const uint32_t idw = k ? ((const uint16_t*)(tb + g.b_id))[32 * r + lane]
+                           : ((const uint32_t*)(tb + g.b_id))[32 * r + lane];
+    double P0 = 0.0, L0 = 0.0, P1 = 0.0, L1 = 0.0;
+    #pragma unroll 1
+    for (int c = hd.y; c > 0; --c) {
+      P0 += src[q0 & 0xFFFFu];
+      q0 = q1;
+      q1 = st[64];
+      st += 32;
+    }
+    int c = hd.x & 0xFFFFu;
+    if (c == 1) {
+      L0 += src[q0 & 0xFFFFu];
+      L1 += src[q0 >> 16];
+      q0 = q1;
+      q1 = st[64];
+      st += 32;
+    } else {
+      #pragma unroll 1
+      for (; c > 0; c -= 2) {
+        const double a0 = src[q0 & 0xFFFFu], a1 = src[q0 >> 16];
+        const double b0 = src[q1 & 0xFFFFu], b1 = src[q1 >> 16];
+        q0 = st[64];
+        q1 = st[96];
+        st += 64;
+        L0 += a0;
+        L1 += a1;
+        L0 += b0;
+        L1 += b1;
+      }
+    }
+    c = hd.x >> 16;
+    if (c == 1) {
+      P0 += term(q0);
+      q0 = q1;
+      q1 = st[64];
+      st += 32;
+    } else {
+      #pragma unroll 1
+      for (; c > 0; c -= 2) {
+        const double v0 = term(q0), v1 = term(q1);
+        q0 = st[64];
+        q1 = st[96];
+        st += 64;
+        P0 += v0;
+        P1 += v1;
+      }
+    }
+    const int id = idw & 0xFFFFu;
+    if (id != 0xFFFF) put(id, idw >> 16, P0 + P1, L0 + L1);
+  }
+  __syncwarp();
+}
+
+// Returns 1 (recoverable) when some y < -SMALL, else writes f into out.
+// When rp/rl are given, the production and loss sums are written too.
+//
+// Nearly every call has no negative rate, concentration or step.  Then a state
+// value is used as it is and only terms with a negative yield need their guard,
+// one lane each, before the gather.  Everything else (also a NaN) takes
+// dev_f_any, which classifies and guards term by term; the sums' order is the
+// same.
+template <typename LT>
+__device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
+                                  const double* keff, double* rates, double* fscr,
+                                  double* out, int lane, double* rp = nullptr,
+                                  double* rl = nullptr, bool neg_extra = false) {
+  tb = g_smem;
+  y = sh(y);
+  keff = sh(keff);
+  rates = sh(rates);
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  bool odd = neg_extra || !(h >= 0.0);
+  const int n = o.n, n_rxn = o.n_rxn;
+  #pragma unroll 1
+  for (int i = lane; i < n; i += 32) odd |= !(y[i] >= 0.0);
+  const uint32_t* rx_word = (const uint32_t*)(tb + o.rx_word);
+  #pragma unroll 2
+  for (int r = lane; r < n_rxn; r += 32) {
+    const uint32_t w = rx_word[r];
+    double rate = keff[r];
+    rate *= y[w & 1023u];  // y[n] = 1
+    rate *= y[(w >> 10) & 1023u];
+    if (w >= 0xC0000000u) rate *= y[(w >> 20) & 1023u];
+    rates[r] = rate;
+    odd |= !(rate >= 0.0);
+  }
+  if (warp_any(odd))
+    return dev_f_any(tb, y, h, keff, rates, fscr, out, lane, rp, rl, neg_extra);
+  const BlobOff::Gather& g = o.g[0];
+  if (lane == 0) rates[g.zero] = 0.0;
+  __syncwarp();
+  // a term with a negative yield counts as a loss while its guard lets it
+  // apply (src/rxns/rxn_arrhenius.c:153-160)
+  const double* coef = (const double*)(tb + o.coef);
+  const uint2* neg = (const uint2*)(tb + g.neg);
+  #pragma unroll 1
+  for (int j = lane; j < g.n_neg; j += 32) {
+    const uint2 q = neg[j];
+    const double v = __dmul_rn(rates[q.x & 0xFFFFu], -coef[q.x >> 16]);
+    rates[g.zero + 1 + j] = v * h <= y[q.y] ? v : 0.0;
+  }
+  __syncwarp();
+  gather<LT>(0, rates, out, fscr, nullptr, lane, rp, rl);
+  f_combine(tb, sh(fscr), sh(out), lane, rp, rl);
+  return 0;
+}
+
 // One product entry of a solver-Jacobian slot: the partial times its yield
 // adds to the production part when the negative-yield guard lets the product
 // term apply (src/rxns/rxn_arrhenius.c:201-207).
@@ -810,10 +1033,12 @@ __device__ __forceinline__ double jac_prod(const Tab& t, const double* part, con
   return -p * yi * c * h <= yrow ? __dmul_rn(c, p) : 0.0;
 }
 
+// the Jacobian with any signs (each lane writes the slots of its balanced
+// list); see dev_jac
 template <typename JT>
-__device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
-                                    const double* keff, double* part, JT* Jout, int lane,
-                                    double* jp = nullptr, double* jl = nullptr) {
+__device__ __noinline__ int dev_jac_any(const char* tb, const double* y, double h,
+                                        const double* keff, double* part, JT* Jout, int lane,
+                                        double* jp, double* jl) {
   const Tab t = make_tab(tb);
   bool bad = false;
   #pragma unroll 1
@@ -877,6 +1102,72 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
   return 0;
 }
 
+// Solver Jacobian values into Jout (indexed by CSC entry); production and
+// loss parts into jp / jl when given (src/rxns/rxn_arrhenius.c:178-212).
+// Returns 1 (recoverable) when some y < -SMALL.
+//
+// As in dev_f, nearly every call has no negative or non-finite partial,
+// concentration or step: then a product with a non-negative yield always
+// passes its guard; anything else takes dev_jac_any, with the sums in the same
+// order.
+template <typename JT>
+__device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
+                                    const double* keff, double* part, JT* Jout, int lane,
+                                    double* jp = nullptr, double* jl = nullptr) {
+  tb = g_smem;
+  y = sh(y);
+  keff = sh(keff);
+  part = sh(part);
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  bool odd = !(h >= 0.0);
+  const int n = o.n, n_rxn = o.n_rxn;
+  #pragma unroll 1
+  for (int i = lane; i < n; i += 32) odd |= !(y[i] >= 0.0);
+  // d rate / d y_k for every variable reactant occurrence k
+  const uint32_t* rx_word = (const uint32_t*)(tb + o.rx_word);
+  const uint16_t* rx_vptr = (const uint16_t*)(tb + o.rx_vptr);
+  auto is_odd = [](double v) { return !(v >= 0.0 && v <= 1.7976931348623157e308); };
+  #pragma unroll 1
+  for (int r = lane; r < n_rxn; r += 32) {
+    const uint32_t w = rx_word[r];
+    const int nv = w >> 30, base = rx_vptr[r];
+    const double k = keff[r], y0 = y[w & 1023u], y1 = y[(w >> 10) & 1023u];  // y[n] = 1
+    if (nv == 3) {
+      const double y2 = y[(w >> 20) & 1023u];
+      const double p0 = k * y1 * y2, p1 = k * y0 * y2, p2 = k * y0 * y1;
+      part[base] = p0;
+      part[base + 1] = p1;
+      part[base + 2] = p2;
+      odd |= is_odd(p0) | is_odd(p1) | is_odd(p2);
+    } else if (nv > 0) {
+      const double p0 = k * y1, p1 = k * y0;
+      part[base] = p0;
+      odd |= is_odd(p0);
+      if (nv > 1) {
+        part[base + 1] = p1;
+        odd |= is_odd(p1);
+      }
+    }
+  }
+  if (warp_any(odd)) return dev_jac_any<JT>(tb, y, h, keff, part, Jout, lane, jp, jl);
+  const BlobOff::Gather& g = o.g[1];
+  if (lane == 0) part[g.zero] = 0.0;
+  __syncwarp();
+  // the negative-yield guard (src/rxns/rxn_arrhenius.c:201-207)
+  const double* coef = (const double*)(tb + o.coef);
+  const uint2* neg = (const uint2*)(tb + g.neg);
+  #pragma unroll 1
+  for (int j = lane; j < g.n_neg; j += 32) {
+    const uint2 q = neg[j];
+    const double p = part[q.x & 0xFFFFu], c = coef[q.x >> 16];
+    part[g.zero + 1 + j] =
+        -p * y[q.y & 0xFFFFu] * c * h <= y[q.y >> 16] ? __dmul_rn(c, p) : 0.0;
+  }
+  __syncwarp();
+  gather<JT>(1, part, nullptr, nullptr, Jout, lane, jp, jl);
+  return 0;
+}
+
 // f and J of a mechanism with SIMPOL, HL or aqueous equilibrium instances:
 // their pseudo-rates or
 // partials first (slots after the terms', which the mass-action passes do
@@ -891,6 +1182,7 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
 // J[row][j] += V[row][c] * P[c][j] (src/camp_solver.c:1063-1106).  Where
 // the production / loss split jp / jl is asked for, each chained term adds to
 // the production part when positive and to the loss part when negative.
+template <typename LT>
 __device__ __noinline__ int dev_f_aero(const char* tb, const double* y, double h,
                                        const double* keff, double* rates, double* fscr,
                                        double* out, int lane, double* rp = nullptr,
@@ -899,7 +1191,7 @@ __device__ __noinline__ int dev_f_aero(const char* tb, const double* y, double h
   double* cv = rates + o.n_rates;
   if (o.n_cv > 0) sub_model_eval(tb, y, keff, cv, nullptr, lane);
   const bool neg = aero_rates(tb, y, keff, cv, rates, lane);
-  return dev_f(tb, y, h, keff, rates, fscr, out, lane, rp, rl, neg);
+  return dev_f<LT>(tb, y, h, keff, rates, fscr, out, lane, rp, rl, neg);
 }
 template <typename JT>
 __device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double h,
@@ -1050,12 +1342,14 @@ __device__ __noinline__ bool dev_form_factor(const char* tb, const LT* J, double
   return !warp_any(bad);
 }
 
-// The spare slots that the padding of the rounds reads and writes (zero, and
-// zero minus products of zeros stays zero).
+// The spare slot LU[n_lu] that the padding of the rounds reads and writes
+// (zero, and zero minus products of zeros stays zero).  Its counterpart z[n]
+// is set with each right-hand side: z lies over the rates' scratch, which no
+// solve needs.
 template <typename LT>
-__device__ __forceinline__ void clear_spare(const char* tb, LT* LU, LT* z, int lane) {
+__device__ __forceinline__ void clear_spare(const char* tb, LT* LU, int lane) {
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
-  if (lane == 0) LU[o.n_lu] = z[o.n] = (LT)0;
+  if (lane == 0) LU[o.n_lu] = (LT)0;
   __syncwarp();
 }
 
@@ -1215,9 +1509,10 @@ struct Cell {
   int lu_mode;        // 0 = level schedule over the lanes, 1 = one lane
   int lane, n;
   double* zb;  // Nordsieck history: column j at zb + j*n
-  double *ewt, *acor, *y, *ftemp, *tempv, *rates, *keff, *fscr;
+  double *ewt, *acor, *y, *ftemp, *rates, *keff, *fscr;
+  double* tempv;  // CTA form: the solves' right-hand side and solution
   LT *LU, *z, *J, *dinv;
-  double rtol;
+  double rtol, rn;  // rn: 1 / n
   int max_steps, maxncf, maxnef;
   double h0;
   // method state
@@ -1225,7 +1520,6 @@ struct Cell {
   double h, hprime, hscale, eta, etamax, hu, next_h, tn;
   double *tau, *tq, *l;  // per-warp shared scalars (all lanes hold equal values)
   double rl1, gamma, gammap, gamrat, crate, acnrm, saved_tq5;
-  double etaqm1, etaq, etaqp1;
   int nst, nfe, nsetups, netf, nni, ncfn, nje, nstlp, nstlj;
 
   __device__ double wrms(const double* v) const {
@@ -1235,7 +1529,7 @@ struct Cell {
       double t = v[i] * ewt[i];
       s += t * t;
     }
-    return dsqrt(ddiv(warp_sum(s), (double)n));
+    return rms(warp_sum(s), (double)n, rn);
   }
   __device__ int f(const double* yy, double* out) {
     if constexpr (BLK) {
@@ -1246,9 +1540,9 @@ struct Cell {
       blk::call<LT>(cmd, *bx, blk::OP_F, yy, out, h > 0.0 ? h : h0);
       return 0;
     } else if constexpr (AERO)
-      return dev_f_aero(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane);
+      return dev_f_aero<LT>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane);
     else
-      return dev_f(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane);
+      return dev_f<LT>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane);
   }
   __device__ bool set_ewt(const double* yy) {
     bool bad = false;
@@ -1256,10 +1550,25 @@ struct Cell {
     for (int i = lane; i < n; i += 32) {
       double w = rtol * fabs(yy[i]) + atol[i];
       bad |= !(w > 0.0);
-      ewt[i] = ddiv(1.0, w);
+      ewt[i] = __drcp_rn(w);
     }
     __syncwarp();
     return !warp_any(bad);
+  }
+  // set_ewt of zn[0] and the test UROUND * wrms(zn[0]) <= 1 in one pass: true
+  // when both surely pass (no weighted value near 1 / UROUND); otherwise the
+  // caller takes them one by one
+  __device__ bool weights_pass() {
+    bool odd = false;
+    #pragma unroll 1
+    for (int i = lane; i < n; i += 32) {
+      const double v = zb[i], w = rtol * fabs(v) + atol[i];
+      const double e = __drcp_rn(w), t = v * e;
+      ewt[i] = e;
+      odd |= !(w > 0.0) || !(t * t < 1.0e25);
+    }
+    __syncwarp();
+    return !warp_any(odd);
   }
   __device__ void rescale() {
     double factor = eta;
@@ -1302,57 +1611,76 @@ struct Cell {
     tn = saved_t;
     pascal(-1.0);
   }
-  // l and tq of the fixed-leading-coefficient BDF formula
+  // l and tq of the fixed-leading-coefficient BDF formula.  Its dozen
+  // divisions are a serial chain only in part: they are taken in three turns,
+  // a quotient per lane, and handed round (3 500 -> 900 cycles at one warp).
   __device__ void set() {
-    double alpha0, alpha0_hat, xi_inv, xistar_inv, hsum;
-    l[0] = l[1] = xi_inv = xistar_inv = 1.0;
+    // xi_j = h / (h + tau_1 + ... + tau_(j-1)) in lane j, the sum in this order
+    double hsum = h;
     #pragma unroll 1
-    for (int i = 2; i <= q; ++i) l[i] = 0.0;
-    alpha0 = alpha0_hat = -1.0;
-    hsum = h;
+    for (int j = 1; j <= q; ++j) hsum += lane > j ? tau[j] : 0.0;
+    const double xi = h / hsum;
+    double c[LMAX];
+    c[0] = c[1] = 1.0;
+#pragma unroll
+    for (int i = 2; i < LMAX; ++i) c[i] = 0.0;
+    const double alpha0 = kAlpha0[q];
+    double alpha0_hat = -1.0, xi_inv = 1.0, xistar_inv = 1.0;
     if (q > 1) {
-      #pragma unroll 1
-      for (int j = 2; j < q; ++j) {
-        hsum += tau[j - 1];
-        xi_inv = ddiv(h, hsum);
-        alpha0 -= ddiv(1.0, (double)j);
-        #pragma unroll 1
-        for (int i = j; i >= 1; --i) l[i] += l[i - 1] * xi_inv;
-      }
-      alpha0 -= ddiv(1.0, (double)q);
-      xistar_inv = -l[1] - alpha0;
-      hsum += tau[q - 1];
-      xi_inv = ddiv(h, hsum);
-      alpha0_hat = -l[1] - xi_inv;
-      #pragma unroll 1
-      for (int i = q; i >= 1; --i) l[i] += l[i - 1] * xistar_inv;
+#pragma unroll
+      for (int j = 2; j < QMAX; ++j)
+        if (j < q) {
+          const double x = __shfl_sync(FULLMASK, xi, j);
+#pragma unroll
+          for (int i = j; i >= 1; --i) c[i] += c[i - 1] * x;
+        }
+      xistar_inv = -c[1] - alpha0;
+      xi_inv = __shfl_sync(FULLMASK, xi, q);
+      alpha0_hat = -c[1] - xi_inv;
+#pragma unroll
+      for (int i = QMAX; i >= 1; --i)
+        if (i <= q) c[i] += c[i - 1] * xistar_inv;
     }
-    double A1 = 1.0 - alpha0_hat + alpha0;
-    double A2 = 1.0 + q * A1;
-    tq[2] = fabs(ddiv(A1, alpha0 * A2));
-    tq[5] = fabs(ddiv(A2 * xistar_inv, l[q] * xi_inv));
-    if (qwait == 1) {
-      if (q > 1) {
-        double C = ddiv(xistar_inv, l[q]);
-        double A3 = alpha0 + ddiv(1.0, (double)q);
-        double A4 = alpha0_hat + xi_inv;
-        double Cpinv = ddiv(1.0 - A4 + A3, A3);
-        tq[1] = fabs(C * Cpinv);
-      } else {
-        tq[1] = 1.0;
-      }
-      hsum += tau[q];
-      xi_inv = ddiv(h, hsum);
-      double A5 = alpha0 - ddiv(1.0, (double)(q + 1));
-      double A6 = alpha0_hat - xi_inv;
-      double Cppinv = ddiv(1.0 - A6 + A5, A2);
-      tq[3] = fabs(ddiv(Cppinv, xi_inv * (q + 2) * A5));
+    double cq = c[1];
+#pragma unroll
+    for (int i = 0; i < LMAX; ++i) {
+      if (i == q) cq = c[i];
+      if (i <= q) l[i] = c[i];
     }
-    tq[4] = ddiv(NLSCOEF, tq[2]);
-    rl1 = ddiv(1.0, l[1]);
+    const double A1 = 1.0 - alpha0_hat + alpha0;
+    const double A2 = 1.0 + q * A1;
+    const bool next_order = qwait == 1;
+    const double xi_next = next_order ? __shfl_sync(FULLMASK, xi, q + 1) : 1.0;
+    const double A3 = alpha0 + kInvInt[q], A4 = alpha0_hat + xi_inv;
+    const double A5 = alpha0 - kInvInt[q + 1], A6 = alpha0_hat - xi_next;
+    double num = A1, den = alpha0 * A2;
+    if (lane == 1) num = A2 * xistar_inv, den = cq * xi_inv;
+    if (lane == 2) num = 1.0, den = c[1];
+    if (lane == 3) num = xistar_inv, den = cq;
+    if (lane == 4) num = 1.0 - A4 + A3, den = A3;
+    if (lane == 5) num = 1.0 - A6 + A5, den = A2;
+    const double r = num / den;
+    const double tq2 = fabs(__shfl_sync(FULLMASK, r, 0));
+    const double tq5 = fabs(__shfl_sync(FULLMASK, r, 1));
+    rl1 = __shfl_sync(FULLMASK, r, 2);
     gamma = h * rl1;
     if (nst == 0) gammap = gamma;
-    gamrat = (nst > 0) ? ddiv(gamma, gammap) : 1.0;
+    num = NLSCOEF;
+    den = tq2;
+    if (lane == 1) num = gamma, den = gammap;
+    if (next_order) {
+      const double C = __shfl_sync(FULLMASK, r, 3), Cpinv = __shfl_sync(FULLMASK, r, 4);
+      const double Cppinv = __shfl_sync(FULLMASK, r, 5);
+      tq[1] = q > 1 ? fabs(C * Cpinv) : 1.0;
+      if (lane == 2) num = Cppinv, den = xi_next * (q + 2) * A5;
+    }
+    const double s = num / den;
+    tq[2] = tq2;
+    tq[5] = tq5;
+    tq[4] = __shfl_sync(FULLMASK, s, 0);
+    const double ratio = __shfl_sync(FULLMASK, s, 1);
+    gamrat = (nst > 0) ? ratio : 1.0;
+    if (next_order) tq[3] = fabs(__shfl_sync(FULLMASK, s, 2));
   }
   __device__ void increase_order() {
     #pragma unroll 1
@@ -1465,6 +1793,8 @@ struct Cell {
         else
           z[iperm[i]] = (LT)r;
       }
+      if constexpr (!BLK)
+        if (lane == 0) z[n] = (LT)0;
       __syncwarp();
       if constexpr (BLK)
         blk::call<LT>(cmd, *bx, blk::OP_SOLVE, nullptr, nullptr, 0.0);
@@ -1489,11 +1819,11 @@ struct Cell {
         acor[i] = a;
         y[i] = (zb + (0) * n)[i] + a;
       }
-      del = dsqrt(ddiv(warp_sum(sum), (double)n));
+      del = rms(warp_sum(sum), (double)n, rn);
       __syncwarp();
       if (mm > 0) crate = fmax(CRDOWN * crate, ddiv(del, delp));
-      double dcon = ddiv(del * fmin(1.0, crate), tq[4]);
-      if (dcon <= 1.0) {
+      // del * min(1, crate) / tq[4] <= 1 (tq[4] > 0: the same without dividing)
+      if (del * fmin(1.0, crate) <= tq[4]) {
         acnrm = (mm == 0 && !projected) ? del : wrms(acor);
         jcur = 0;
         return NL_OK;
@@ -1520,7 +1850,7 @@ struct Cell {
         s += t * t;
       }
     if (!warp_any(viol)) return NL_OK;
-    double vnorm = dsqrt(ddiv(warp_sum(s), (double)n));
+    double vnorm = rms(warp_sum(s), (double)n, rn);
     if (vnorm <= tq[4]) {
       #pragma unroll 1
       for (int i = lane; i < n; i += 32)
@@ -1605,7 +1935,7 @@ struct Cell {
     if (*nef == maxnef) return ERR_FAILURE;
     etamax = 1.0;
     if (*nef <= MXNEF1) {
-      eta = ddiv(1.0, dpow(BIAS2 * *dsm, ddiv(1.0, (double)L)) + ADDON);
+      eta = ddiv(1.0, dpow(BIAS2 * *dsm, kInvInt[L]) + ADDON);
       eta = fmax(ETAMIN, eta);
       if (*nef >= SMALL_NEF) eta = fmin(eta, ETAMXF);
       rescale();
@@ -1628,11 +1958,11 @@ struct Cell {
     #pragma unroll 1
     for (int i = lane; i < n; i += 32) y[i] = zb[i];
     __syncwarp();
-    int r = f(y, tempv);
+    int r = f(y, ftemp);
     nfe++;
     if (r > 0) return UNREC_RHSFUNC_ERR;
     #pragma unroll 1
-    for (int i = lane; i < n; i += 32) (zb + (1) * n)[i] = h * tempv[i];
+    for (int i = lane; i < n; i += 32) (zb + (1) * n)[i] = h * ftemp[i];
     __syncwarp();
     return TRY_AGAIN;
   }
@@ -1647,8 +1977,13 @@ struct Cell {
     #pragma unroll 1
     for (int i = lane; i < n; i += 32) {
       const double a = acor[i];
-      #pragma unroll 1
-      for (int j = 0; j <= q; ++j) (zb + (j) * n)[i] += l[j] * a;
+      double v[LMAX];
+#pragma unroll
+      for (int j = 0; j < LMAX; ++j)
+        if (j <= q) v[j] = zb[j * n + i];
+#pragma unroll
+      for (int j = 0; j < LMAX; ++j)
+        if (j <= q) zb[j * n + i] = v[j] + l[j] * a;
       if (save) (zb + (QMAX) * n)[i] = a;
     }
     __syncwarp();
@@ -1674,27 +2009,42 @@ struct Cell {
       eta = 1.0;
       return;
     }
-    etaq = ddiv(1.0, dpow(BIAS2 * dsm, ddiv(1.0, (double)L)) + ADDON);
+    // Most steps keep their size, and that shows without the powers: a ratio
+    // below THRESH counts as 1 whatever its value.
+    const bool no_q = BIAS2 * dsm > kNoGrowth[L];
     if (qwait != 0) {
-      eta = etaq;
       qprime = q;
+      eta = no_q ? 1.0
+                 : ddiv(1.0, dpow(BIAS2 * dsm, kInvInt[L]) + ADDON);
       set_eta();
       return;
     }
     qwait = 2;
-    etaqm1 = 0.0;
+    double ddn = 0.0, dup = 0.0;
+    bool no_any = no_q;
     if (q > 1) {
-      double ddn = wrms((zb + (q) * n)) * tq[1];
-      etaqm1 = ddiv(1.0, dpow(BIAS1 * ddn, ddiv(1.0, (double)q)) + ADDON);
+      ddn = wrms((zb + (q) * n)) * tq[1];
+      no_any &= BIAS1 * ddn > kNoGrowth[q];
     }
-    etaqp1 = 0.0;
-    if (q != QMAX && saved_tq5 != 0.0) {
-      double cquot = ddiv(tq[5], saved_tq5) * dpow(ddiv(h, tau[2]), (double)L);
+    const bool up = q != QMAX && saved_tq5 != 0.0;
+    if (up) {
+      const double ratio = ddiv(h, tau[2]);
+      const double cquot = ddiv(tq[5], saved_tq5) * (ratio == 1.0 ? 1.0 : dpow(ratio, (double)L));
       #pragma unroll 1
-      for (int i = lane; i < n; i += 32) tempv[i] = acor[i] - cquot * (zb + (QMAX) * n)[i];
-      double dup = wrms(tempv) * tq[3];
-      etaqp1 = ddiv(1.0, dpow(BIAS3 * dup, ddiv(1.0, (double)(L + 1))) + ADDON);
+      for (int i = lane; i < n; i += 32) ftemp[i] = acor[i] - cquot * (zb + (QMAX) * n)[i];
+      dup = wrms(ftemp) * tq[3];
+      no_any &= BIAS3 * dup > kNoGrowth[L + 1];
     }
+    if (no_any) {
+      eta = 1.0;
+      qprime = q;
+      set_eta();
+      return;
+    }
+    const double etaq = ddiv(1.0, dpow(BIAS2 * dsm, kInvInt[L]) + ADDON);
+    double etaqm1 = 0.0, etaqp1 = 0.0;
+    if (q > 1) etaqm1 = ddiv(1.0, dpow(BIAS1 * ddn, kInvInt[q]) + ADDON);
+    if (up) etaqp1 = ddiv(1.0, dpow(BIAS3 * dup, kInvInt[L + 1]) + ADDON);
     double etam = fmax(etaqm1, fmax(etaq, etaqp1));
     if (etam < THRESH) {
       eta = 1.0;
@@ -1734,9 +2084,6 @@ struct Cell {
     complete_step();
     prepare_next_step(dsm);
     etamax = (nst <= SMALL_NST) ? ETAMX2 : ETAMX3;
-    #pragma unroll 1
-    for (int i = lane; i < n; i += 32) acor[i] *= tq[2];
-    __syncwarp();
     return OK;
   }
   // CVodeReInit + CVodeSetInitStep(h0) + CVode(tout, CV_NORMAL); y (shared)
@@ -1771,7 +2118,7 @@ struct Cell {
     __syncwarp();
     if (!set_ewt((zb + (0) * n))) return ILL_INPUT;
     next_h = 0.0;
-    if (f(y, (zb + (1) * n))) return REPTD_RHSFUNC_ERR;
+    if (f(y, ftemp)) return REPTD_RHSFUNC_ERR;
     nfe++;
     h = h0;
     // a zero initial step makes CVODE estimate one (cvHin), which refuses an
@@ -1781,16 +2128,16 @@ struct Cell {
     hscale = h;
     hprime = h;
     #pragma unroll 1
-    for (int i = lane; i < n; i += 32) (zb + (1) * n)[i] *= h;
+    for (int i = lane; i < n; i += 32) (zb + (1) * n)[i] = ftemp[i] * h;
     __syncwarp();
     int nstloc = 0;
     #pragma unroll 1
     for (;;) {
       next_h = h;
-      if (nst > 0 && !set_ewt((zb + (0) * n))) return ILL_INPUT;
+      const bool pass = nst > 0 && weights_pass();
+      if (!pass && nst > 0 && !set_ewt((zb + (0) * n))) return ILL_INPUT;
       if (max_steps > 0 && nstloc >= max_steps) return TOO_MUCH_WORK;
-      double tolsf = UROUND * wrms((zb + (0) * n));
-      if (tolsf > 1.0) return TOO_MUCH_ACC;
+      if (!pass && UROUND * wrms((zb + (0) * n)) > 1.0) return TOO_MUCH_ACC;
       int kflag = step();
       if (kflag != OK) return kflag;
       nstloc++;
@@ -1822,8 +2169,8 @@ __device__ void bind_cell(Cell<LT, AERO>& c, const SolveArgs& a, const char* tab
   c.iperm = make_tab(tab).lu_iperm;
   c.lane = lane;
   c.n = a.off.n;
-  // per-warp global slab: [Nordsieck history when it is not in shared
-  // memory] [rate constants when they are not in shared memory]
+  c.rn = 1.0 / (double)a.off.n;
+  // per-warp global slab: the Nordsieck history when it is not in shared memory
   double* slab = a.hist ? a.hist + (size_t)gwarp * a.hist_stride : nullptr;
   c.zb = a.lay.zn >= 0 ? (double*)(base + a.lay.zn) : slab;
   double* ctl = (double*)(base + a.lay.ctl);
@@ -1834,10 +2181,9 @@ __device__ void bind_cell(Cell<LT, AERO>& c, const SolveArgs& a, const char* tab
   c.acor = (double*)(base + a.lay.acor);
   c.y = (double*)(base + a.lay.y);
   c.ftemp = (double*)(base + a.lay.ftemp);
-  c.tempv = (double*)(base + a.lay.tempv);
+  c.tempv = nullptr;
   c.rates = (double*)(base + a.lay.rates);
-  c.keff = a.lay.keff >= 0 ? (double*)(base + a.lay.keff)
-                           : slab + (a.lay.zn >= 0 ? 0 : (size_t)LMAX * a.off.n);
+  c.keff = (double*)(base + a.lay.keff);
   c.fscr = (double*)(base + a.lay.fscr);
   c.LU = (LT*)(base + a.lay.lu);
   c.z = (LT*)(base + a.lay.z);
@@ -1856,7 +2202,7 @@ __device__ void bind_cell(Cell<LT, AERO>& c, const SolveArgs& a, const char* tab
 template <typename LT, bool AERO>
 __global__ void __launch_bounds__(32 * (AERO ? kMaxCellsAero : kMaxCellsPerBlock), 1)
     solve_kernel(SolveArgs a) {
-  extern __shared__ __align__(16) char smem[];
+  char* const smem = g_smem;
   __shared__ unsigned long long tma_bar;
   if (!stage_tables(smem, a.blob, a.stage_bytes, &tma_bar, a.err)) return;
   const int lane = threadIdx.x & 31;
@@ -1865,7 +2211,8 @@ __global__ void __launch_bounds__(32 * (AERO ? kMaxCellsAero : kMaxCellsPerBlock
   char* base = smem + a.tab_bytes + (size_t)wib * a.lay.bytes;
   Cell<LT, AERO> c;
   bind_cell<LT, AERO>(c, a, smem, base, gwarp, lane);
-  clear_spare<LT>(smem, c.LU, c.z, lane);
+  clear_spare<LT>(smem, c.LU, lane);
+  set_unit(c.y, c.n, lane);
   const DevMech& m = a.m;
   const uint16_t* dep_state = make_tab(smem).dep_state;
   #pragma unroll 1
@@ -1964,7 +2311,7 @@ struct BlkArgs {
 template <typename LT>
 __global__ void __launch_bounds__(blk::kThreads, sizeof(LT) == 4 ? 2 : 1)
     block_kernel(BlkArgs a) {
-  extern __shared__ __align__(16) char smem[];
+  char* const smem = g_smem;
   __shared__ blk::Cmd cmd;
   __shared__ int s_idx;
   const BlkLayout& L = a.lay;
@@ -2027,6 +2374,7 @@ __global__ void __launch_bounds__(blk::kThreads, sizeof(LT) == 4 ? 2 : 1)
     c.atol = cx->t.atol;
     c.lane = lane;
     c.n = cx->t.n;
+    c.rn = 1.0 / (double)cx->t.n;
     c.zb = L.zn >= 0 ? (double*)(smem + L.zn) : a.hist + (size_t)blockIdx.x * a.hist_stride;
     double* ctl = (double*)(smem + L.ctl);
     c.tau = ctl;
@@ -2114,7 +2462,7 @@ struct EvalArgs {
 };
 
 __global__ void eval_kernel(EvalArgs a) {
-  extern __shared__ __align__(16) char smem[];
+  char* const smem = g_smem;
   __shared__ unsigned long long tma_bar;
   if (!stage_tables(smem, a.blob, a.stage_bytes, &tma_bar, a.err)) return;
   const int lane = threadIdx.x & 31;
@@ -2131,16 +2479,16 @@ __global__ void eval_kernel(EvalArgs a) {
   const double* st = a.state + (size_t)cell * m.n_state;
   #pragma unroll 1
   for (int i = lane; i < t.n; i += 32) y[i] = st[t.dep_state[i]];
-  __syncwarp();
+  set_unit(y, t.n, lane);
   compute_keff(m, st, a.env[2 * cell], a.env[2 * cell + 1],
                a.photo ? a.photo + (size_t)cell * m.n_photo : nullptr, keff, lane);
   if (!a.do_jac) {
     double* out = (double*)(base + a.lay.ftemp);
     if (has_simpol(smem))
-      dev_f_aero(smem, y, a.h, keff, rates, fscr, out, lane, a.rp + (size_t)cell * t.n,
+      dev_f_aero<double>(smem, y, a.h, keff, rates, fscr, out, lane, a.rp + (size_t)cell * t.n,
                  a.rl + (size_t)cell * t.n);
     else
-      dev_f(smem, y, a.h, keff, rates, fscr, out, lane, a.rp + (size_t)cell * t.n,
+      dev_f<double>(smem, y, a.h, keff, rates, fscr, out, lane, a.rp + (size_t)cell * t.n,
             a.rl + (size_t)cell * t.n);
     #pragma unroll 1
     for (int i = lane; i < t.n; i += 32) a.f[(size_t)cell * t.n + i] = out[i];
@@ -2177,7 +2525,7 @@ struct CheckArgs {
 };
 
 __global__ void jac_check_kernel(CheckArgs c) {
-  extern __shared__ __align__(16) char smem[];
+  char* const smem = g_smem;
   __shared__ unsigned long long tma_bar;
   const EvalArgs& a = c.e;
   if (!stage_tables(smem, a.blob, a.stage_bytes, &tma_bar, a.err)) return;
@@ -2202,11 +2550,11 @@ __global__ void jac_check_kernel(CheckArgs c) {
   const double* st = a.state + (size_t)cell * m.n_state;
   #pragma unroll 1
   for (int i = lane; i < t.n; i += 32) y[i] = st[t.dep_state[i]];
-  __syncwarp();
+  set_unit(y, t.n, lane);
   compute_keff(m, st, a.env[2 * cell], a.env[2 * cell + 1],
                a.photo ? a.photo + (size_t)cell * m.n_photo : nullptr, keff, lane);
   const bool aero = has_simpol(smem);
-  if (dev_f_aero(smem, y, a.h, keff, rates, fscr, f0, lane, rp0, rl0) ||
+  if (dev_f_aero<double>(smem, y, a.h, keff, rates, fscr, f0, lane, rp0, rl0) ||
       (aero ? dev_jac_aero<double>(smem, y, a.h, keff, rates, J, lane)
             : dev_jac<double>(smem, y, a.h, keff, rates, J, lane))) {
     if (lane == 0) {
@@ -2231,10 +2579,10 @@ __global__ void jac_check_kernel(CheckArgs c) {
       const double dx = x * scale;
       if (lane == 0) y[j] = x + dx;
       __syncwarp();
-      int r = dev_f_aero(smem, y, a.h, keff, rates, fscr, f1, lane);
+      int r = dev_f_aero<double>(smem, y, a.h, keff, rates, fscr, f1, lane);
       if (lane == 0) y[j] = x + 0.5 * dx;
       __syncwarp();
-      r |= dev_f_aero(smem, y, a.h, keff, rates, fscr, f2, lane);
+      r |= dev_f_aero<double>(smem, y, a.h, keff, rates, fscr, f2, lane);
       if (lane == 0) y[j] = x;
       __syncwarp();
       if (r) continue;
@@ -2306,7 +2654,7 @@ struct PrecArgs {
 
 template <typename LT>
 __global__ void precision_kernel(PrecArgs p) {
-  extern __shared__ __align__(16) char smem[];
+  char* const smem = g_smem;
   __shared__ unsigned long long tma_bar;
   const EvalArgs& a = p.e;
   if (!stage_tables(smem, a.blob, a.stage_bytes, &tma_bar, a.err)) return;
@@ -2324,11 +2672,11 @@ __global__ void precision_kernel(PrecArgs p) {
   LT* z = (LT*)(base + a.lay.z);
   LT* dinv = (LT*)(base + a.lay.dinv);
   LT* J = (LT*)p.jbuf + (size_t)cell * t.n_jac;
-  clear_spare<LT>(smem, LU, z, lane);
+  clear_spare<LT>(smem, LU, lane);
   const double* st = a.state + (size_t)cell * m.n_state;
   #pragma unroll 1
   for (int i = lane; i < t.n; i += 32) y[i] = st[t.dep_state[i]];
-  __syncwarp();
+  set_unit(y, t.n, lane);
   compute_keff(m, st, a.env[2 * cell], a.env[2 * cell + 1],
                a.photo ? a.photo + (size_t)cell * m.n_photo : nullptr, keff, lane);
   int r = has_simpol(smem) ? dev_jac_aero<LT>(smem, y, a.h, keff, rates, J, lane)
@@ -2340,6 +2688,7 @@ __global__ void precision_kernel(PrecArgs p) {
       const double s = p.rtol * fabs(y[i]) + t.atol[i];
       z[t.lu_iperm[i]] = (LT)(((i * 2654435761u) >> 13) & 1u ? s : -s);
     }
+    if (lane == 0) z[t.n] = (LT)0;
     __syncwarp();
     dev_lsolve<LT>(smem, LU, dinv, z, lane);
     #pragma unroll 1
@@ -2577,6 +2926,8 @@ bool Engine::init(const Model& model, const std::vector<double>& atol_dep, int c
   I->warp_ok = build_blob(t, atol_dep, &blob, &I->off, &I->warp_why);
   if (I->warp_ok) {
     CK(cudaMalloc(&I->d_blob, blob.size()));
+    I->off.self = (unsigned long long)(uintptr_t)I->d_blob;
+    memcpy(blob.data(), &I->off, sizeof(I->off));
     CK(cudaMemcpy(I->d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice));
   }
   std::vector<uint8_t> lblob;
@@ -2617,7 +2968,7 @@ bool Engine::init(const Model& model, const std::vector<double>& atol_dep, int c
 // and the rate constants in global memory (with_hist = false), which leaves
 // room for more resident cells
 static Layout make_layout(const BlobOff& o, int lt_size, bool with_hist,
-                          bool keff_in_smem) {
+                          bool with_tempv) {
   Layout L{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -2629,18 +2980,18 @@ static Layout make_layout(const BlobOff& o, int lt_size, bool with_hist,
   L.zn = with_hist ? take(vec * LMAX) : -1;
   L.ewt = take(vec);
   L.acor = take(vec);
-  L.y = take(vec);
+  L.y = take(vec + sizeof(double));  // y[n]: see set_unit
   L.ftemp = take(vec);
-  L.tempv = take(vec);
-  // the f scratch (pseudo-rates, then the computed species) and the J
-  // scratch (partials, computed species, parameter partials, virtual slots)
-  L.rates = take(sizeof(double) * std::max(o.n_rates + o.n_cv,
-                                           o.n_part_all + o.n_cv + o.n_pj + o.n_virt));
-  L.keff = keff_in_smem ? take(sizeof(double) * o.n_keff) : -1;
+  L.tempv = with_tempv ? take(vec) : -1;
+  // the f scratch (pseudo-rates, then the computed species, a zero and the guarded terms) and
+  // the J scratch (partials, computed species, parameter partials, virtual
+  // slots, a zero and the guarded terms); the solves' vector lies over them
+  const int n_scr = std::max(o.g[0].zero + 1 + o.g[0].n_neg, o.g[1].zero + 1 + o.g[1].n_neg);
+  L.rates = L.z = take(std::max(sizeof(double) * n_scr, (size_t)lt_size * (o.n + 1)));
+  L.keff = take(sizeof(double) * o.n_keff);
   L.fscr = take(sizeof(double) * 2 * std::max(1, o.n_fscratch));
-  // one spare slot each: the target of the grouped phases' no-op records
+  // a spare slot: see clear_spare
   L.lu = take((size_t)lt_size * (o.n_lu + 1));
-  L.z = take((size_t)lt_size * (o.n + 1));
   L.dinv = take((size_t)lt_size * o.n);
   // control block: tau[LMAX + 2], tq[8], l[LMAX + 1]
   L.ctl = take(sizeof(double) * (LMAX + 2 + 8 + LMAX + 1));
@@ -2651,7 +3002,7 @@ static Layout make_layout(const BlobOff& o, int lt_size, bool with_hist,
 // shared-memory bytes of the staged tables: the one-lane LU mode also needs
 // the row-wise LU tables at the end of the blob
 static int stage_bytes_of(const BlobOff& o, int lu_mode) {
-  return lu_mode ? o.bytes : o.stage_bytes;
+  return lu_mode ? o.seq_bytes : o.stage_bytes;
 }
 static int tab_bytes_of(const BlobOff& o, int lu_mode) {
   return (stage_bytes_of(o, lu_mode) + 127) & ~127;
@@ -2681,7 +3032,7 @@ static bool plan_warp_launch(const BlobOff& off, int sm_count, int max_smem,
                              const SolveSettings& s, int n_cells, int max_blocks,
                              WarpLaunch* w, std::string* err) {
   w->lt = s.precision == 1 ? 4 : 8;
-  w->lay = make_layout(off, w->lt, s.hist_global == 0, true);
+  w->lay = make_layout(off, w->lt, s.hist_global == 0, false);
   w->tab = tab_bytes_of(off, s.lu_mode);
   int max_warps = (max_smem - w->tab) / w->lay.bytes;
   if (max_warps < 1) {
@@ -3050,7 +3401,7 @@ int Engine::max_cells_per_block(const SolveSettings& s) const {
   const Impl* I = impl_;
   if (s.kernel != 0 || !I->warp_ok) return 0;
   const int lt = s.precision == 1 ? 4 : 8;
-  const Layout lay = make_layout(I->off, lt, s.hist_global == 0, true);
+  const Layout lay = make_layout(I->off, lt, s.hist_global == 0, false);
   return std::min(max_cells_of(I->off),
                   std::max(0, (I->max_smem - tab_bytes_of(I->off, s.lu_mode)) / lay.bytes));
 }
@@ -3142,8 +3493,8 @@ bool Engine::eval_deriv(const double* h_state, const double* h_env, const double
   a.m = m;
   a.off = I->off;
   a.blob = I->d_blob;
-  a.tab_bytes = tab_bytes_of(I->off, 1);
-  a.stage_bytes = I->off.bytes;
+  a.tab_bytes = tab_bytes_of(I->off, 0);
+  a.stage_bytes = I->off.stage_bytes;
   a.err = I->d_counter + 1;
   a.lay = make_layout(I->off, 8, true, true);
   a.state = ds;
@@ -3188,8 +3539,8 @@ bool Engine::eval_jac(const double* h_state, const double* h_env, const double* 
   a.m = m;
   a.off = I->off;
   a.blob = I->d_blob;
-  a.tab_bytes = tab_bytes_of(I->off, 1);
-  a.stage_bytes = I->off.bytes;
+  a.tab_bytes = tab_bytes_of(I->off, 0);
+  a.stage_bytes = I->off.stage_bytes;
   a.err = I->d_counter + 1;
   a.lay = make_layout(I->off, 8, true, true);
   a.state = ds;
@@ -3239,8 +3590,8 @@ bool Engine::check_precision(const double* h_state, const double* h_env,
     a.m = m;
     a.off = I->off;
     a.blob = I->d_blob;
-    a.tab_bytes = tab_bytes_of(I->off, 1);
-    a.stage_bytes = I->off.bytes;
+    a.tab_bytes = tab_bytes_of(I->off, 0);
+    a.stage_bytes = I->off.stage_bytes;
     a.err = I->d_counter + 1;
     a.lay = make_layout(I->off, pass == 0 ? 8 : 4, true, true);
     a.state = bs.p;
@@ -3328,8 +3679,8 @@ bool Engine::check_jac(const double* h_state, const double* h_env, const double*
     a.m = m;
     a.off = I->off;
     a.blob = I->d_blob;
-    a.tab_bytes = tab_bytes_of(I->off, 1);
-    a.stage_bytes = I->off.bytes;
+    a.tab_bytes = tab_bytes_of(I->off, 0);
+    a.stage_bytes = I->off.stage_bytes;
     a.err = I->d_counter + 1;
     a.lay = make_layout(I->off, 8, true, true);
     a.state = ds;
@@ -3433,7 +3784,7 @@ bool Engine::run_solve_static(double* d_state, const double* d_env, const double
   }
   cudaStream_t st = (cudaStream_t)stream;
   const int lt = s.precision == 1 ? 4 : 8;
-  Layout lay = make_layout(I->off, lt, true, true);
+  Layout lay = make_layout(I->off, lt, true, false);
   const int tab = tab_bytes_of(I->off, s.lu_mode);
   int warps = (I->max_smem - tab) / lay.bytes;
   if (warps < 1) {
