@@ -376,9 +376,18 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     *err = "too many Jacobian elements for the table encoding";
     return false;
   }
+  std::vector<int> jslot(t.n_jac);  // J slot of each CSC entry: by LU position
+  {
+    std::vector<int> at(t.n_lu, 0);
+    for (int e = 0; e < t.n_jac; ++e) at[t.jg_lupos[e]] = e + 1;
+    for (int q = 0, k = 0; q < t.n_lu; ++q)
+      if (at[q]) jslot[at[q] - 1] = k++;
+  }
   std::vector<uint16_t> lu_src(t.n_lu, 0);
-  for (int e = 0; e < t.n_jac; ++e) lu_src[t.jg_lupos[e]] = (uint16_t)(e + 1);
+  for (int e = 0; e < t.n_jac; ++e) lu_src[t.jg_lupos[e]] = (uint16_t)(jslot[e] + 1);
   for (int i = 0; i < n; ++i) lu_src[t.lu_diag[i]] |= 0x8000u;
+  std::vector<int> jcsc(t.n_jac);
+  for (int e = 0; e < t.n_jac; ++e) jcsc[jslot[e]] = e;
   std::vector<long> jw(t.n_jac);
   for (int e = 0; e < t.n_jac; ++e) jw[e] = 2 + (t.jg_ptr[e + 1] - t.jg_ptr[e]);
   auto jlanes = lpt(jw);
@@ -403,7 +412,7 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     std::vector<GatherItem> items;
     for (int e = 0; e < t.n_jac; ++e) {
       GatherItem it;
-      it.id = e;
+      it.id = jslot[e];
       for (int g = t.jg_ptr[e]; g < jg_umid[e]; ++g)
         it.lead.push_back((jg_w0[g] & 0xFFFFu) | one);
       for (int g = jg_umid[e]; g < jg_mid[e]; ++g)
@@ -432,35 +441,32 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     for (size_t i = 0; i < v.size(); ++i) o[i] = (uint16_t)v[i];
     return o;
   };
-  std::vector<uint32_t> fa(t.fa_pos.size());
-  for (size_t i = 0; i < fa.size(); ++i) fa[i] = (uint32_t)t.fa_pos[i] | ((uint32_t)t.fa_piv[i] << 16);
   // Grouped phases as rounds of 32 targets, longest first within a level, so
   // that a round's targets have similar lengths and its padding stays small.
-  // Per round its pair count, whether it is the last of its level, 32 records
-  // (first pair, target, pivot or finish mark) and its further pairs.
+  // Per round its pair count, 32 records (first pair, target, pivot or finish
+  // mark) and its further pairs.
   struct Rounds {
     std::vector<uint32_t> pair0, target, recip, ext;
-    std::vector<int> cnt, last;
+    std::vector<int> cnt, level;
   };
   auto rounds_of = [&](const Tables::Grouped& g, Rounds* o, uint32_t no_pair, int spare,
-                       bool keep_empty) {
+                       bool with_empty) {
     for (int l = 0; l < g.n_levels; ++l) {
       std::vector<int> us;
-      for (int u = g.lane_ptr[33 * l]; u < g.lane_ptr[33 * l + kLanes]; ++u) us.push_back(u);
+      for (int u = g.lane_ptr[33 * l]; u < g.lane_ptr[33 * l + kLanes]; ++u)
+        if (with_empty || g.unit_count[u] > 0) us.push_back(u);
       std::stable_sort(us.begin(), us.end(), [&](int a, int b) {
         return g.unit_count[a] > g.unit_count[b];
       });
-      const size_t n_r = std::max<size_t>(keep_empty ? 1 : 0, (us.size() + kLanes - 1) / kLanes);
-      for (size_t r = 0; r < n_r; ++r) {
+      for (size_t k0 = 0; k0 < us.size(); k0 += kLanes) {
         auto pair = [&](size_t k, int j) {
           if (k >= us.size() || j >= g.unit_count[us[k]]) return no_pair;
           const int p = g.unit_begin[us[k]] + j;
           return (uint32_t)g.pair_a[p] | ((uint32_t)g.pair_b[p] << 16);
         };
-        const size_t k0 = r * kLanes;
-        const int cnt = k0 < us.size() ? std::max(1, g.unit_count[us[k0]]) : 1;
+        const int cnt = std::max(1, g.unit_count[us[k0]]);
         o->cnt.push_back(cnt);
-        o->last.push_back(r + 1 == n_r);
+        o->level.push_back(l);
         for (size_t k = k0; k < k0 + kLanes; ++k) {
           const bool real = k < us.size();
           o->pair0.push_back(pair(k, 0));
@@ -480,27 +486,53 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   Rounds fbr, svr;
   const uint32_t lu_none = (uint32_t)t.n_lu | ((uint32_t)t.n_lu << 16);
   const uint32_t sv_none = (uint32_t)t.n_lu | ((uint32_t)n << 16);
-  rounds_of(t.fb, &fbr, lu_none, t.n_lu, true);
-  rounds_of(t.fwd, &svr, sv_none, n, false);
-  rounds_of(t.bwd, &svr, sv_none, n, false);
-  std::vector<uint32_t> fb_rec, sv_rec;
-  std::vector<uint16_t> fb_hdr;
+  // the factorization takes reciprocal pivots with the scaling, so its units
+  // without pairs drop out (the schedule's phase g holds level g - 1's updates)
+  rounds_of(t.fb, &fbr, lu_none, t.n_lu, false);
+  rounds_of(t.fwd, &svr, sv_none, n, true);
+  const int n_fwd = (int)svr.cnt.size();
+  rounds_of(t.bwd, &svr, sv_none, n, true);
+  std::vector<uint32_t> fb_rec, sv_rec, fs_rec;
+  std::vector<uint16_t> fl_hdr(2 * t.n_plev, 0);
   for (size_t r = 0; r < fbr.cnt.size(); ++r)
-    fb_hdr.push_back((uint16_t)(fbr.cnt[r] | (fbr.last[r] ? 0x8000 : 0)));
-  fb_hdr.push_back(1);  // read ahead, never run
+    fl_hdr[2 * (fbr.level[r] - 1) + 1]++;
   for (size_t k = 0; k < fbr.pair0.size(); ++k) {
     fb_rec.push_back(fbr.pair0[k]);
-    fb_rec.push_back(fbr.target[k] | (fbr.recip[k] << 16));
+    fb_rec.push_back(fbr.target[k] | ((uint32_t)fbr.cnt[k / kLanes] << 16));
   }
-  for (int k = 0; k < kLanes; ++k) {
+  for (int k = 0; k < 2 * kLanes; ++k) {
     fb_rec.push_back(lu_none);
-    fb_rec.push_back((uint32_t)t.n_lu);
+    fb_rec.push_back((uint32_t)t.n_lu | (1u << 16));
   }
-  const int n_srounds = (int)svr.cnt.size();
+  for (int l = 0; l < t.n_plev; ++l) {
+    std::vector<std::pair<int, int>> e;  // L position (n_lu: none), pivot
+    std::vector<char> has(n, 0);
+    for (int i = t.fa_ptr[l]; i < t.fa_ptr[l + 1]; ++i) {
+      e.push_back({t.fa_pos[i], t.fa_piv[i]});
+      has[t.fa_piv[i]] = 1;
+    }
+    // the pivots of a level are those whose reciprocal its phase takes
+    for (int u = t.fb.lane_ptr[33 * l]; u < t.fb.lane_ptr[33 * l + kLanes]; ++u)
+      if (t.fb.unit_recip[u] && !has[t.fb.unit_recip[u] - 1])
+        e.push_back({t.n_lu, t.fb.unit_recip[u] - 1});
+    std::vector<char> stored(n, 0);
+    for (size_t k = 0; k < (e.size() + kLanes - 1) / kLanes * kLanes; ++k) {
+      if (k >= e.size()) {
+        fs_rec.push_back((uint32_t)t.n_lu);
+        fs_rec.push_back(0x7FFFu);
+        continue;
+      }
+      const int piv = e[k].second;
+      fs_rec.push_back((uint32_t)e[k].first | ((uint32_t)t.lu_diag[piv] << 16));
+      fs_rec.push_back((uint32_t)piv | (stored[piv] ? 0u : 0x8000u));
+      stored[piv] = 1;
+    }
+    fl_hdr[2 * l] = (uint16_t)((e.size() + kLanes - 1) / kLanes);
+  }
   for (size_t k = 0; k < svr.pair0.size(); ++k) {
     sv_rec.push_back(svr.pair0[k]);
-    sv_rec.push_back(svr.target[k] | ((uint32_t)svr.cnt[k / kLanes] << 16) |
-                     (svr.recip[k] ? 0x80000000u : 0u));
+    sv_rec.push_back(svr.target[k] | (svr.recip[k] ? 0x8000u : 0u) |
+                     ((uint32_t)svr.cnt[k / kLanes] << 16));
   }
   for (int k = 0; k < 2 * kLanes; ++k) {
     sv_rec.push_back(sv_none);
@@ -625,7 +657,9 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     o.jv_ptr = w.put(u16(t.jv_ptr));
     o.jv_part = w.put(u16(t.jv_part));
     o.n_chain = (int)t.ch_tgt.size();
-    o.ch_tgt = w.put(u16(t.ch_tgt));
+    std::vector<int> tgt;
+    for (int e : t.ch_tgt) tgt.push_back(jslot[e]);
+    o.ch_tgt = w.put(u16(tgt));
     o.ch_ptr = w.put(u16(t.ch_ptr));
     std::vector<uint32_t> ent(t.ch_v.size());
     for (size_t i = 0; i < ent.size(); ++i)
@@ -640,12 +674,12 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   o.n_plev = t.n_plev;
   o.lu_iperm = w.put(u16(t.lu_iperm));
   o.lu_src = w.put(lu_src);
-  o.fa_ptr = w.put(u16(t.fa_ptr));
-  o.fa = w.put(fa);
-  o.fb_hdr = w.put(fb_hdr);
+  o.fl_hdr = w.put(fl_hdr);
+  o.fs_rec = w.put(fs_rec);
   o.fb_rec = w.put(fb_rec);
   o.fb_ext = w.put(fbr.ext);
-  o.n_srounds = n_srounds;
+  o.n_fwd = n_fwd;
+  o.n_bwd = (int)svr.cnt.size() - n_fwd;
   o.sv_rec = w.put(sv_rec);
   o.sv_ext = w.put(svr.ext);
   o.dep_state = w.put(u16(t.dep_state));
@@ -671,6 +705,8 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   o.fg_ent = w.put(fg_ent);
   o.fg_unit = w.put(fg_unit);
   o.fg_lane = w.put(fg_lane);
+  o.j_csc = w.put(u16(jcsc));
+  o.jg_slot = w.put(u16(jslot));
   o.jg_w0 = w.put(jg_w0);
   o.jg_w1 = w.put(jg_w1);
   o.jg_ptr = w.put(jg_ptr);

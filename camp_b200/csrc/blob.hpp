@@ -39,8 +39,9 @@ struct BlobOff {
   // words of loss pairs | products<<16, leading unguarded products), per lane
   // b_id (f: uint32 id | tag<<16, J: uint16 id), and in b_ent, 32 lanes at a
   // time, the unguarded products, the loss pairs (uint32 index | index<<16) and
-  // the products, both a multiple of two.  Padding uses an index that the
-  // gather keeps at zero; four entries and two rows are read ahead of the ends.
+  // the products, both one or a multiple of two.  Padding uses an index that
+  // the gather keeps at zero; four entries and two rows are read ahead of the
+  // ends.
   // Terms with a negative yield are evaluated before the gather, n_neg records
   // (uint32 index | coef<<16; f: species, J: guard species | row<<16), into
   // the slots after that zero.
@@ -54,27 +55,30 @@ struct BlobOff {
   // (0 = loss entry); per slot: entry pointer, LU position, row; lane slot
   // lists.  Read from the blob in global memory (self).
   int jg_w0, jg_w1, jg_ptr, jg_mid, jg_lupos, jg_row, jg_lane, jg_slots;
-  // LU: dependent index -> pivot row (iperm), diag (uint16); factorization by
-  // pivot level: scaled L entries (fa_ptr uint16, fa = pos | pivot<<16),
-  // Schur updates grouped by target with the reciprocal pivots taken in the
-  // same phase, as rounds (n_plev + 1 phases).  A round gives every lane one
-  // target LU[tgt] -= sum LU[a] LU[b]: record uint32 a | b<<16, uint32 tgt |
-  // (pivot+1)<<16 (pivot 0 = none; fb_rec, 32 records per round and one round
-  // of padding at the end), the first pair in the record, the round's
-  // cnt - 1 more per lane in fb_ext; fb_hdr (uint16 per round): cnt | last
-  // round of its phase<<15.  Padding as in the solves.
+  // device J slots are numbered by LU position; CSC entry of each slot and
+  // slot of each CSC entry (uint16; self)
+  int j_csc, jg_slot;
+  // LU: dependent index -> pivot row (iperm), diag (uint16); per LU position
+  // the J slot that fills it + 1 (0 = none; slots are numbered by LU position)
+  // | diagonal<<15.
   int lu_iperm, lu_diag, lu_src;
-  int fa_ptr, fa;
-  int fb_hdr, fb_rec, fb_ext;
-  // triangular solves: n_srounds rounds, forward then backward.  A round
-  // gives every lane one target z[tgt] -= sum LU[a] z[x] (backward: then
-  // times its reciprocal pivot when bit 31 of the second word is set): record
-  // uint32 a | x<<16, uint32 tgt | cnt<<16 | finish<<31 (sv_rec, 32 records
-  // per round and two rounds of padding at the end), the first pair in the
-  // record, cnt - 1 more per lane in sv_ext (uint32 a | x<<16, 32 per step).
-  // cnt is the round's largest, the same in every lane: shorter targets and
-  // idle lanes are padded with the spare slots LU[n_lu] = z[n] = 0.
-  int n_srounds, sv_rec, sv_ext;
+  // factorization by pivot level (n_plev): fl_hdr (uint16 x 2 per level):
+  // rounds of scaled L entries, rounds of updates.  A scaling round gives every lane fs_rec (uint32 L position |
+  // diagonal position<<16, uint32 pivot | store its reciprocal<<15; pivot
+  // 0x7FFF idle lane, L position n_lu nothing to scale).  An update round gives
+  // every lane one target LU[tgt] -= sum LU[a] LU[b]: record uint32 a | b<<16,
+  // uint32 tgt | cnt<<16 (fb_rec), the first pair in the record, cnt - 1 more
+  // per lane in fb_ext (uint32 a | b<<16, 32 per step).  cnt is the round's
+  // largest, the same in every lane: shorter targets and idle lanes are padded
+  // with the spare slot LU[n_lu] = 0.
+  int fl_hdr, fs_rec, fb_rec, fb_ext;
+  // triangular solves: n_fwd rounds forward, then n_bwd backward.  A round
+  // gives every lane one target z[tgt] -= sum LU[a] z[x] (backward: then times
+  // its reciprocal pivot when bit 15 of the second word is set): record
+  // uint32 a | x<<16, uint32 tgt | finish<<15 | cnt<<16 (sv_rec), further pairs
+  // in sv_ext (uint32 a | x<<16) as for the updates, padded with LU[n_lu] and
+  // z[n] = 0.  Two rounds of records are read ahead of the ends.
+  int n_fwd, n_bwd, sv_rec, sv_ext;
   // row-wise LU for the sequential (one-lane) mode: J slot -> LU position
   // (jg_lupos), diagonal positions, rowptr, col (uint16), update pointer per
   // L entry (uint32) and updates (src | dst<<16); staged only in that mode

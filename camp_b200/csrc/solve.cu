@@ -120,6 +120,18 @@ __device__ __forceinline__ T* sh(T* p) {
 // (src/camp_solver.c:805-833)
 __device__ __forceinline__ double state_of(double y) { return y > -kSmall ? y : kTiny; }
 
+// flags of a Newton iterate: made non-negative, holding a value that is not a
+// number >= 0 (both per lane), with a negative aerosol pseudo-rate (per warp)
+constexpr int kProjected = 1, kOdd = 2, kNegRate = 4;
+
+// whether some value of this lane is not a number >= 0
+__device__ __noinline__ int vec_odd(const double* y, int n, int lane) {
+  bool odd = false;
+  #pragma unroll 1
+  for (int i = lane; i < n; i += 32) odd |= !(y[i] >= 0.0);
+  return odd ? kOdd : 0;
+}
+
 // y[n] = 1: the absent reactants of f's rates (the concentrations themselves
 // never reach y[n])
 __device__ __forceinline__ void set_unit(double* y, int n, int lane) {
@@ -137,14 +149,16 @@ __device__ __noinline__ double dpow(double x, double y) { return pow(x, y); }
 __device__ __noinline__ double ddiv(double a, double b) { return a / b; }
 __device__ __noinline__ double dsqrt(double a) { return sqrt(a); }
 
-// sqrt(s / n) with n a small whole number and rn = 1 / n rounded to nearest:
-// one residual step makes s * rn the correctly rounded quotient (Markstein,
-// IBM J. Res. Dev. 34, 1990) at a fifth of a division's latency, away from
-// the ends of the exponent range
-__device__ __noinline__ double rms(double s, double n, double rn) {
+// sqrt(sum of s over the lanes / n) with n a small whole number and rn = 1 / n
+// rounded to nearest: one residual step makes sum * rn the correctly rounded
+// quotient (Markstein, IBM J. Res. Dev. 34, 1990) at a fifth of a division's
+// latency, away from the ends of the exponent range
+__device__ __noinline__ double warp_rms(double s, int n, double rn) {
+  s = warp_sum(s);
+  const double d = (double)n;
   double q = s * rn;
-  q = fma(fma(-q, n, s), rn, q);
-  if (!(s > 1.0e-250 && s < 1.0e250)) q = s / n;
+  q = fma(fma(-q, d, s), rn, q);
+  if (!(s > 1.0e-250 && s < 1.0e250)) q = ddiv(s, d);
   return sqrt(q);
 }
 
@@ -180,6 +194,7 @@ struct Tab {
   const double* atol;
   const uint16_t *lu_rowptr, *lu_col;
   const uint32_t *upd_ptr, *upd;
+  const uint16_t* jg_slot;
   const uint16_t *si_rec, *si_elem, *jg_umid, *aq_rec, *aq_sp, *aq_cp;
   const double *si_ef, *aq_sm, *aq_cpm, *aq_sim;
   int n, n_rxn, n_jac, n_lu, n_fsplit, n_simpol, has_ug, n_aq;
@@ -196,6 +211,7 @@ __device__ __forceinline__ Tab make_tab(const char* b) {
   t.fg_unit = (const uint16_t*)(g + o.fg_unit);
   t.fg_lane = (const uint16_t*)(g + o.fg_lane);
   t.fg_split = (const uint16_t*)(b + o.fg_split);
+  t.jg_slot = (const uint16_t*)(g + o.jg_slot);
   t.jg_w0 = (const uint32_t*)(g + o.jg_w0);
   t.jg_w1 = (const uint16_t*)(g + o.jg_w1);
   t.jg_ptr = (const uint16_t*)(g + o.jg_ptr);
@@ -736,22 +752,24 @@ __device__ __noinline__ void aero_partials(const char* tb, const double* y, cons
 }
 
 // the species whose lists were split over several units
+template <bool EV>
 __device__ __forceinline__ void f_combine(const char* tb, const double* fscr, double* out,
                                           int lane, double* rp, double* rl) {
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
   const uint16_t* split = (const uint16_t*)(tb + o.fg_split);
   #pragma unroll 1
   for (int s = lane; s < o.n_fsplit; s += 32) {
-    const int sp = split[3 * s], first = split[3 * s + 1], cnt = split[3 * s + 2];
+    const int sp = split[3 * s];
+    const double* v = fscr + 2 * split[3 * s + 1];
     double P = 0.0, L = 0.0;
     #pragma unroll 1
-    for (int j = 0; j < cnt; ++j) {
-      P += fscr[2 * (first + j)];
-      L += fscr[2 * (first + j) + 1];
+    for (int j = split[3 * s + 2]; j > 0; --j, v += 2) {
+      P += v[0];
+      L += v[1];
     }
     out[sp] = (P + L != 0.0) ? P - L : 0.0;
-    if (rp) rp[sp] = P;
-    if (rl) rl[sp] = L;
+    if (EV && rp) rp[sp] = P;
+    if (EV && rl) rl[sp] = L;
   }
   __syncwarp();
 }
@@ -842,13 +860,14 @@ __device__ __noinline__ int dev_f_any(const char* tb, const double* y, double h,
     }
   }
   __syncwarp();
-  f_combine(tb, fscr, out, lane, rp, rl);
+  f_combine<true>(tb, fscr, out, lane, rp, rl);
   return 0;
 }
 
 // Sums of every item of the f (k = 0) or J (k = 1) gather (blob.hpp) from the
 // terms in src, f into out (fscr for the parts of a split species), J into
-// Jout by CSC entry; production and loss parts into rp / rl when given.
+// Jout by slot.  The evaluation hooks' form (EV) writes J by CSC entry when csc
+// gives each slot's, and production and loss parts into rp / rl.
 //
 // No term here is negative, so each one's sum is known, and the step counts of
 // a round are the same in every lane: the long lists (some tens of terms) a
@@ -856,9 +875,10 @@ __device__ __noinline__ int dev_f_any(const char* tb, const double* y, double h,
 // in blob.cpp).  Bound by shared-memory latency: the loads of several entries
 // are issued together, their words a step ahead.  One copy of the code for f
 // and J, as the kernel is short of instruction cache.
-template <typename JT>
+template <typename JT, bool EV>
 __device__ __noinline__ void gather(int k, const double* src, double* out, double* fscr,
-                                    JT* Jout, int lane, double* rp, double* rl) {
+                                    JT* Jout, int lane, const uint16_t* csc = nullptr,
+                                    double* rp = nullptr, double* rl = nullptr) {
   src = sh(src);
   const char* const tb = g_smem;
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
@@ -867,6 +887,7 @@ __device__ __noinline__ void gather(int k, const double* src, double* out, doubl
   auto term = [&](uint32_t q) { return __dmul_rn(src[q & 0xFFFFu], coef[q >> 16]); };
   auto put = [&](int id, int tag, double P, double L) {
     if (k) {
+      if (EV && csc) id = csc[id];
       Jout[id] = (JT)(P - L);
     } else if (tag == 0xFFFF) {
       sh(out)[id] = (P + L != 0.0) ? P - L : 0.0;
@@ -875,8 +896,8 @@ __device__ __noinline__ void gather(int k, const double* src, double* out, doubl
       sh(fscr)[2 * tag + 1] = L;
       return;
     }
-    if (rp) rp[id] = P;
-    if (rl) rl[id] = L;
+    if (EV && rp) rp[id] = P;
+    if (EV && rl) rl[id] = L;
   };
   {
     const uint2* rec = (const uint2*)(tb + g.a_rec) + lane;
@@ -972,25 +993,25 @@ __device__ __noinline__ void gather(int k, const double* src, double* out, doubl
 //
 // Nearly every call has no negative rate, concentration or step.  Then a state
 // value is used as it is and only terms with a negative yield need their guard,
-// one lane each, before the gather.  Everything else (also a NaN) takes
+// one lane each, before the gather; flags tells whether this lane's share of y
+// has a value that is not a number >= 0 (kOdd) and, in every lane, whether an
+// aerosol pseudo-rate is negative (kNegRate).  Everything else (also a NaN) takes
 // dev_f_any, which classifies and guards term by term; the sums' order is the
 // same.
-template <typename LT>
+template <typename LT, bool EV = false>
 __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
                                   const double* keff, double* rates, double* fscr,
-                                  double* out, int lane, double* rp = nullptr,
-                                  double* rl = nullptr, bool neg_extra = false) {
+                                  double* out, int lane, int flags, double* rp = nullptr,
+                                  double* rl = nullptr) {
   tb = g_smem;
   y = sh(y);
   keff = sh(keff);
   rates = sh(rates);
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
-  bool odd = neg_extra || !(h >= 0.0);
-  const int n = o.n, n_rxn = o.n_rxn;
-  #pragma unroll 1
-  for (int i = lane; i < n; i += 32) odd |= !(y[i] >= 0.0);
+  bool odd = flags != 0 || !(h >= 0.0);
+  const int n_rxn = o.n_rxn;
   const uint32_t* rx_word = (const uint32_t*)(tb + o.rx_word);
-  #pragma unroll 2
+  #pragma unroll 1
   for (int r = lane; r < n_rxn; r += 32) {
     const uint32_t w = rx_word[r];
     double rate = keff[r];
@@ -1001,7 +1022,8 @@ __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
     odd |= !(rate >= 0.0);
   }
   if (warp_any(odd))
-    return dev_f_any(tb, y, h, keff, rates, fscr, out, lane, rp, rl, neg_extra);
+    return dev_f_any(tb, y, h, keff, rates, fscr, out, lane, EV ? rp : nullptr,
+                     EV ? rl : nullptr, (flags & kNegRate) != 0);
   const BlobOff::Gather& g = o.g[0];
   if (lane == 0) rates[g.zero] = 0.0;
   __syncwarp();
@@ -1016,8 +1038,9 @@ __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
     rates[g.zero + 1 + j] = v * h <= y[q.y] ? v : 0.0;
   }
   __syncwarp();
-  gather<LT>(0, rates, out, fscr, nullptr, lane, rp, rl);
-  f_combine(tb, sh(fscr), sh(out), lane, rp, rl);
+  gather<LT, EV>(0, rates, out, fscr, nullptr, lane, nullptr, EV ? rp : nullptr,
+                 EV ? rl : nullptr);
+  f_combine<EV>(tb, sh(fscr), sh(out), lane, rp, rl);
   return 0;
 }
 
@@ -1038,7 +1061,7 @@ __device__ __forceinline__ double jac_prod(const Tab& t, const double* part, con
 template <typename JT>
 __device__ __noinline__ int dev_jac_any(const char* tb, const double* y, double h,
                                         const double* keff, double* part, JT* Jout, int lane,
-                                        double* jp, double* jl) {
+                                        const uint16_t* csc, double* jp, double* jl) {
   const Tab t = make_tab(tb);
   bool bad = false;
   #pragma unroll 1
@@ -1094,7 +1117,7 @@ __device__ __noinline__ int dev_jac_any(const char* tb, const double* y, double 
     }
     if (g < g1) P0 += jac_prod(t, part, y, yrow, h, g);
     const double P = P0 + P1, L = L0 + L1;
-    Jout[e] = (JT)(P - L);
+    Jout[csc ? e : t.jg_slot[e]] = (JT)(P - L);
     if (jp) jp[e] = P;
     if (jl) jl[e] = L;
   }
@@ -1102,27 +1125,27 @@ __device__ __noinline__ int dev_jac_any(const char* tb, const double* y, double 
   return 0;
 }
 
-// Solver Jacobian values into Jout (indexed by CSC entry); production and
-// loss parts into jp / jl when given (src/rxns/rxn_arrhenius.c:178-212).
+// Solver Jacobian values into Jout, by slot (in the order of the LU positions)
+// or, with csc, by CSC entry; production and loss parts into jp / jl when
+// given (src/rxns/rxn_arrhenius.c:178-212).
 // Returns 1 (recoverable) when some y < -SMALL.
 //
 // As in dev_f, nearly every call has no negative or non-finite partial,
 // concentration or step: then a product with a non-negative yield always
 // passes its guard; anything else takes dev_jac_any, with the sums in the same
 // order.
-template <typename JT>
+template <typename JT, bool EV = false>
 __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
-                                    const double* keff, double* part, JT* Jout, int lane,
-                                    double* jp = nullptr, double* jl = nullptr) {
+                                    const double* keff, double* part, JT* Jout, int lane, int flags,
+                                    const uint16_t* csc = nullptr, double* jp = nullptr,
+                                    double* jl = nullptr) {
   tb = g_smem;
   y = sh(y);
   keff = sh(keff);
   part = sh(part);
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
-  bool odd = !(h >= 0.0);
-  const int n = o.n, n_rxn = o.n_rxn;
-  #pragma unroll 1
-  for (int i = lane; i < n; i += 32) odd |= !(y[i] >= 0.0);
+  bool odd = flags != 0 || !(h >= 0.0);
+  const int n_rxn = o.n_rxn;
   // d rate / d y_k for every variable reactant occurrence k
   const uint32_t* rx_word = (const uint32_t*)(tb + o.rx_word);
   const uint16_t* rx_vptr = (const uint16_t*)(tb + o.rx_vptr);
@@ -1149,7 +1172,9 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
       }
     }
   }
-  if (warp_any(odd)) return dev_jac_any<JT>(tb, y, h, keff, part, Jout, lane, jp, jl);
+  if (warp_any(odd))
+    return dev_jac_any<JT>(tb, y, h, keff, part, Jout, lane, EV ? csc : nullptr,
+                           EV ? jp : nullptr, EV ? jl : nullptr);
   const BlobOff::Gather& g = o.g[1];
   if (lane == 0) part[g.zero] = 0.0;
   __syncwarp();
@@ -1164,7 +1189,10 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
         -p * y[q.y & 0xFFFFu] * c * h <= y[q.y >> 16] ? __dmul_rn(c, p) : 0.0;
   }
   __syncwarp();
-  gather<JT>(1, part, nullptr, nullptr, Jout, lane, jp, jl);
+  if constexpr (EV)
+    gather<JT, true>(1, part, nullptr, nullptr, Jout, lane, csc, jp, jl);
+  else
+    gather<JT, false>(1, part, nullptr, nullptr, Jout, lane);
   return 0;
 }
 
@@ -1182,28 +1210,30 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
 // J[row][j] += V[row][c] * P[c][j] (src/camp_solver.c:1063-1106).  Where
 // the production / loss split jp / jl is asked for, each chained term adds to
 // the production part when positive and to the loss part when negative.
-template <typename LT>
+template <typename LT, bool EV = false>
 __device__ __noinline__ int dev_f_aero(const char* tb, const double* y, double h,
                                        const double* keff, double* rates, double* fscr,
-                                       double* out, int lane, double* rp = nullptr,
+                                       double* out, int lane, int flags, double* rp = nullptr,
                                        double* rl = nullptr) {
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
   double* cv = rates + o.n_rates;
   if (o.n_cv > 0) sub_model_eval(tb, y, keff, cv, nullptr, lane);
   const bool neg = aero_rates(tb, y, keff, cv, rates, lane);
-  return dev_f<LT>(tb, y, h, keff, rates, fscr, out, lane, rp, rl, neg);
+  return dev_f<LT, EV>(tb, y, h, keff, rates, fscr, out, lane, flags | (neg ? kNegRate : 0), rp,
+                       rl);
 }
-template <typename JT>
+template <typename JT, bool EV = false>
 __device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double h,
-                                         const double* keff, double* part, JT* Jout, int lane,
-                                         double* jp = nullptr, double* jl = nullptr) {
+                                         const double* keff, double* part, JT* Jout, int lane, int flags,
+                                         const uint16_t* csc = nullptr, double* jp = nullptr,
+                                         double* jl = nullptr) {
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
   double* cv = part + o.n_part_all;
   double* P = cv + o.n_cv;
   double* V = P + o.n_pj;
   if (o.n_cv > 0) sub_model_eval(tb, y, keff, cv, P, lane);
   aero_partials(tb, y, keff, cv, part, lane);
-  const int r = dev_jac<JT>(tb, y, h, keff, part, Jout, lane, jp, jl);
+  const int r = dev_jac<JT, EV>(tb, y, h, keff, part, Jout, lane, flags, csc, jp, jl);
   if (r != 0 || o.n_chain == 0) return r;
   const uint16_t* vptr = (const uint16_t*)(tb + o.jv_ptr);
   const uint16_t* vpart = (const uint16_t*)(tb + o.jv_part);
@@ -1220,7 +1250,8 @@ __device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double
   const uint32_t* ent = (const uint32_t*)(tb + o.ch_ent);
   #pragma unroll 1
   for (int g = lane; g < o.n_chain; g += 32) {
-    double s = (double)Jout[tgt[g]], sp = 0.0, sl = 0.0;
+    const int at = EV && csc ? csc[tgt[g]] : tgt[g];
+    double s = (double)Jout[at], sp = 0.0, sl = 0.0;
     #pragma unroll 1
     for (int e = cptr[g]; e < cptr[g + 1]; ++e) {
       const double v = V[ent[e] & 0xFFFFu] * P[ent[e] >> 16];
@@ -1228,10 +1259,10 @@ __device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double
       sp += v > 0.0 ? v : 0.0;
       sl += v < 0.0 ? -v : 0.0;
     }
-    Jout[tgt[g]] = (JT)s;
-    if (jp) {
-      jp[tgt[g]] += sp;
-      jl[tgt[g]] += sl;
+    Jout[at] = (JT)s;
+    if (EV && jp) {
+      jp[at] += sp;
+      jl[at] += sl;
     }
   }
   __syncwarp();
@@ -1245,24 +1276,29 @@ __device__ __forceinline__ bool has_simpol(const char* tb) {
 // ---------------------------------------------------------------------------
 // LU of M = I - gamma*J on the fixed order, and the triangular solves
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
+__device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
+
 // M = I - gamma*J scattered into the LU pattern, then a right-looking
 // factorization level by level: L columns scaled by the level's reciprocal
-// pivots, then its Schur updates grouped by target, a target that becomes a
-// pivot of the next level storing its reciprocal in dinv.  Returns false on a
-// zero or non-finite pivot.
-// Bound by latency and instruction count (cb05cl_ae5: 23 levels, 60 rounds of
-// at most 32 targets, mostly of one pair), so a round is one record load per
-// lane, loaded one round ahead, the first pair in the record and the pair
-// count in a header that every lane reads.
+// pivots (stored in dinv), then its Schur updates grouped by target.  Returns
+// false on a zero or non-finite pivot.
+// Bound by latency and instruction count (cb05cl_ae5: 22 levels, 60 rounds of
+// at most 32 targets, mostly of one pair).  So every lane that scales an entry
+// takes the reciprocal of its pivot itself, which saves a barrier and a trip
+// through shared memory per level; a round of updates is one record per lane,
+// read two rounds ahead.  J is laid out in the order of the LU positions, so
+// that its loads (global memory, four in flight) are nearly contiguous.
 template <typename LT>
 __device__ __noinline__ bool dev_form_factor(const char* tb, const LT* J, double gamma,
                                              LT* LU, LT* dinv, int lane) {
+  tb = g_smem;
+  LU = sh(LU);
+  dinv = sh(dinv);
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
-  // M = I - gamma*J in one pass over the LU positions (fill-in starts at 0),
-  // four loads of J (global memory) in flight
+  const int n_lu = o.n_lu;
   {
     const uint16_t* lu_src = (const uint16_t*)(tb + o.lu_src);
-    const int n_lu = o.n_lu;
     #pragma unroll 1
     for (int q = lane; q < n_lu; q += 128) {
       uint32_t src[4];
@@ -1280,63 +1316,55 @@ __device__ __noinline__ bool dev_form_factor(const char* tb, const LT* J, double
         }
     }
   }
-  __syncwarp();
-  const uint16_t* hdr = (const uint16_t*)(tb + o.fb_hdr);
+  const ushort2* hdr = (const ushort2*)(tb + o.fl_hdr);
+  const uint2* fs = (const uint2*)(tb + o.fs_rec) + lane;
   const uint2* rec = (const uint2*)(tb + o.fb_rec) + lane;
   const uint32_t* ext = (const uint32_t*)(tb + o.fb_ext) + lane;
-  const uint16_t* fa_ptr = (const uint16_t*)(tb + o.fa_ptr);
-  const uint32_t* fa = (const uint32_t*)(tb + o.fa);
-  const int n_plev = o.n_plev;
+  uint2 w = rec[0], wn = rec[32];
+  rec += 64;
   bool bad = false;
-  uint2 w = *rec;
-  unsigned h = *hdr;
-  int fa0 = 0;
+  __syncwarp();
   #pragma unroll 1
-  for (int lv = 0;; ++lv) {
-    unsigned last;
+  for (int lv = o.n_plev; lv > 0; --lv) {
+    const ushort2 hd = *hdr++;
     #pragma unroll 1
-    do {
+    for (int c = hd.x; c > 0; --c, fs += 32) {
+      const uint2 f = *fs;
+      const int piv = f.y & 0x7FFFu, pos = f.x & 0xFFFFu;
+      if (piv != 0x7FFF) {
+        const LT p = LU[f.x >> 16], v = LU[pos];
+        const bool pbad = p == (LT)0 || !isfinite(p);
+        bad |= pbad;
+        const LT d = pbad ? (LT)0 : rcp_rn(p);
+        if (pos != n_lu) LU[pos] = v * d;
+        if (f.y & 0x8000u) dinv[piv] = d;
+      }
+    }
+    __syncwarp();
+    #pragma unroll 1
+    for (int r = hd.y; r > 0; --r) {
+      const int tgt = w.y & 0xFFFFu;
+      LT s = LU[tgt] - LU[w.x & 0xFFFFu] * LU[w.x >> 16];
+      int c = w.y >> 16;
+      w = wn;
+      wn = *rec;
       rec += 32;
-      ++hdr;
-      const uint2 wn = *rec;
-      const unsigned hn = *hdr;
-      const int tgt = w.y & 0xFFFFu, piv = w.y >> 16, cnt = h & 0x7FFFu;
-      LT s0 = LU[tgt], s1 = (LT)0;
-      s0 -= LU[w.x & 0xFFFFu] * LU[w.x >> 16];
-      if (cnt > 1) {
-        int p = 1;
+      if (c > 1) {
+        LT s1 = (LT)0;
         #pragma unroll 1
-        for (; p + 1 < cnt; p += 2, ext += 64) {
+        for (; c > 2; c -= 2, ext += 64) {
           const uint32_t q0 = ext[0], q1 = ext[32];
           s1 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
-          s0 -= LU[q1 & 0xFFFFu] * LU[q1 >> 16];
+          s -= LU[q1 & 0xFFFFu] * LU[q1 >> 16];
         }
-        if (p < cnt) {
-          const uint32_t q0 = ext[0];
-          s1 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
+        if (c > 1) {
+          s1 -= LU[ext[0] & 0xFFFFu] * LU[ext[0] >> 16];
           ext += 32;
         }
-      }
-      const LT s = s0 + s1;
-      if (piv) {
-        const bool pbad = (s == (LT)0) || !isfinite((double)s);
-        bad |= pbad;
-        dinv[piv - 1] = pbad ? (LT)0 : (LT)1 / s;
+        s += s1;
       }
       LU[tgt] = s;
-      last = h & 0x8000u;
-      w = wn;
-      h = hn;
-    } while (!last);
-    __syncwarp();
-    if (lv == n_plev) break;
-    const int fa1 = fa_ptr[lv + 1];
-    #pragma unroll 1
-    for (int i = fa0 + lane; i < fa1; i += 32) {
-      const uint32_t e = fa[i];
-      LU[e & 0xFFFFu] *= dinv[e >> 16];
     }
-    fa0 = fa1;
     __syncwarp();
   }
   return !warp_any(bad);
@@ -1357,46 +1385,48 @@ __device__ __forceinline__ void clear_spare(const char* tb, LT* LU, int lane) {
 // Bound by latency: some thirty levels in a row (cb05cl_ae5: 14 forward, 16
 // backward), each a handful of dependent steps on at most 32 targets.  So a
 // round is one record load per lane and as few instructions as will do: the
-// record holds its first pair (the only one in most rounds), the next
-// round's L / U value and the record after that are loaded while this round
-// runs, and the pair count is the same in every lane.
+// record holds its first pair (the only one in most rounds), it is read two
+// rounds ahead, its L / U value and reciprocal pivot one (1 where there is
+// none: exact), and the pair count is the same in every lane.  One loop for both
+// directions and no unrolling: the code has to stay in the instruction cache.
 template <typename LT>
-__device__ __noinline__ void dev_lsolve(const char* tb, const LT* LU, const LT* dinv, LT* z,
-                                        int lane) {
-  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
-  const uint2* rec = (const uint2*)(tb + o.sv_rec) + lane;
-  const uint32_t* ext = (const uint32_t*)(tb + o.sv_ext) + lane;
-  const uint2* const end = rec + 32 * o.n_srounds;
+__device__ __noinline__ void dev_lsolve(const LT* LU, const LT* dinv, LT* z, int lane) {
+  LU = sh(LU);
+  dinv = sh(dinv);
+  z = sh(z);
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(g_smem);
+  const uint2* rec = (const uint2*)(g_smem + o.sv_rec) + lane;
+  const uint32_t* ext = (const uint32_t*)(g_smem + o.sv_ext) + lane;
   uint2 w = rec[0], wn = rec[32];
-  LT a = LU[w.x & 0xFFFFu];
+  LT a = LU[w.x & 0xFFFFu], d = (LT)1;
+  rec += 64;
   #pragma unroll 1
-  for (; rec < end; rec += 32) {
-    const uint2 wnn = rec[64];
-    const LT an = LU[wn.x & 0xFFFFu];
-    const int tgt = w.y & 0xFFFFu, cnt = (w.y >> 16) & 0x7FFFu;
-    LT s0 = z[tgt], s1 = (LT)0;
-    s0 -= a * z[w.x >> 16];
-    if (cnt > 1) {
-      int p = 1;
+  for (int r = o.n_fwd + o.n_bwd; r > 0; --r) {
+    const int tgt = w.y & 0x7FFFu;
+    LT s = z[tgt] - a * z[w.x >> 16];
+    a = LU[wn.x & 0xFFFFu];
+    int c = w.y >> 16;
+    if (c > 1) {
+      // further pairs into alternating sums
+      LT s1 = (LT)0;
       #pragma unroll 1
-      for (; p + 1 < cnt; p += 2, ext += 64) {
+      for (; c > 2; c -= 2, ext += 64) {
         const uint32_t q0 = ext[0], q1 = ext[32];
         s1 -= LU[q0 & 0xFFFFu] * z[q0 >> 16];
-        s0 -= LU[q1 & 0xFFFFu] * z[q1 >> 16];
+        s -= LU[q1 & 0xFFFFu] * z[q1 >> 16];
       }
-      if (p < cnt) {
-        const uint32_t q0 = ext[0];
-        s1 -= LU[q0 & 0xFFFFu] * z[q0 >> 16];
+      if (c > 1) {
+        s1 -= LU[ext[0] & 0xFFFFu] * z[ext[0] >> 16];
         ext += 32;
       }
+      s += s1;
     }
-    LT s = s0 + s1;
-    if ((int)w.y < 0) s *= dinv[tgt];
-    z[tgt] = s;
+    z[tgt] = s * d;
+    d = (wn.y & 0x8000u) ? dinv[wn.y & 0x7FFFu] : (LT)1;
     __syncwarp();
     w = wn;
-    wn = wnn;
-    a = an;
+    wn = *rec;
+    rec += 32;
   }
 }
 
@@ -1416,7 +1446,7 @@ __device__ __noinline__ bool dev_form_factor_seq(const char* tb, const LT* J, do
   #pragma unroll 1
   for (int s = t.jg_lane[lane]; s < s1; ++s) {
     const int e = t.jg_slots[s];
-    LU[t.jg_lupos[e]] = (LT)(-gamma * (double)J[e]);
+    LU[t.jg_lupos[e]] = (LT)(-gamma * (double)J[t.jg_slot[e]]);
   }
   __syncwarp();
   #pragma unroll 1
@@ -1495,6 +1525,129 @@ __device__ __noinline__ void dev_lsolve_seq(const char* tb, const LT* LU, const 
 // ---------------------------------------------------------------------------
 #include "block.cuh"
 
+// Vector operations of the integrator that have several call sites, one
+// out-of-line copy each: the warps of an SM are at different points of the BDF
+// control flow, so the kernel is bound by instruction fetch as much as by
+// latency, and its throughput follows the size of the code they share.
+__device__ __noinline__ double vec_wrms(const double* v, const double* ewt, int n, double rn,
+                                        int lane) {
+  ewt = sh(ewt);
+  double s = 0.0;
+  #pragma unroll 1
+  for (int i = lane; i < n; i += 32) {
+    double t = v[i] * ewt[i];
+    s += t * t;
+  }
+  return warp_rms(s, n, rn);
+}
+// zn <- zn * Pascal(q) (sign +1) or its inverse (sign -1), one element's
+// q+1 history values at a time in registers: for k = 1..q, j = q..k,
+// zn[j-1] += sign * zn[j].  With acor (a prediction) also the first Newton
+// iterate, see vec_start.
+__device__ __noinline__ int hist_pascal(double* zb, int n, int q, double sign, double* acor,
+                                        double* y, int lane) {
+  int flags = 0;
+  #pragma unroll 1
+  for (int i = lane; i < n; i += 32) {
+    double v[LMAX];
+#pragma unroll
+    for (int j = 0; j < LMAX; ++j) v[j] = (j <= q) ? zb[j * n + i] : 0.0;
+#pragma unroll
+    for (int k = 1; k <= QMAX; ++k)
+#pragma unroll
+      for (int j = QMAX; j >= 1; --j)
+        if (k <= q && j >= k && j <= q) v[j - 1] += sign * v[j];
+#pragma unroll
+    for (int j = 0; j < QMAX; ++j)
+      if (j < q) zb[j * n + i] = v[j];
+    if (acor) {
+      const double a = v[0] < 0.0 ? -v[0] : 0.0, s = v[0] + a;
+      sh(acor)[i] = a;
+      sh(y)[i] = s;
+      flags |= (a != 0.0 ? kProjected : 0) | (s >= 0.0 ? 0 : kOdd);
+    }
+  }
+  __syncwarp();
+  return flags;
+}
+// zn[j] *= eta^j, j = 1..q
+__device__ __noinline__ void hist_rescale(double* zb, int n, int q, double eta, int lane) {
+  double factor = eta;
+  #pragma unroll 1
+  for (int j = 1; j <= q; ++j) {
+    #pragma unroll 1
+    for (int i = lane; i < n; i += 32) zb[j * n + i] *= factor;
+    factor *= eta;
+  }
+  __syncwarp();
+}
+__device__ __noinline__ void hist_increase(double* zb, int n, int q, double hscale,
+                                           const double* tau, double* l, int lane) {
+  tau = sh(tau);
+  l = sh(l);
+  #pragma unroll 1
+  for (int i = 0; i <= QMAX; ++i) l[i] = 0.0;
+  l[2] = 1.0;
+  double alpha1 = 1.0, prod = 1.0, xiold = 1.0, alpha0 = -1.0, hsum = hscale;
+  if (q > 1) {
+    #pragma unroll 1
+    for (int j = 1; j < q; ++j) {
+      hsum += tau[j + 1];
+      double xi = ddiv(hsum, hscale);
+      prod *= xi;
+      alpha0 -= ddiv(1.0, (double)(j + 1));
+      alpha1 += ddiv(1.0, xi);
+      #pragma unroll 1
+      for (int i = j + 2; i >= 2; --i) l[i] = l[i] * xiold + l[i - 1];
+      xiold = xi;
+    }
+  }
+  double A1 = ddiv(-alpha0 - alpha1, prod);
+  #pragma unroll 1
+  for (int i = lane; i < n; i += 32) {
+    double top = A1 * (zb + (QMAX) * n)[i];
+    (zb + (q + 1) * n)[i] = top;
+    #pragma unroll 1
+    for (int j = 2; j <= q; ++j) (zb + (j) * n)[i] += l[j] * top;
+  }
+  __syncwarp();
+}
+__device__ __noinline__ void hist_decrease(double* zb, int n, int q, double hscale,
+                                           const double* tau, double* l, int lane) {
+  tau = sh(tau);
+  l = sh(l);
+  #pragma unroll 1
+  for (int i = 0; i <= QMAX; ++i) l[i] = 0.0;
+  l[2] = 1.0;
+  double hsum = 0.0;
+  #pragma unroll 1
+  for (int j = 1; j <= q - 2; ++j) {
+    hsum += tau[j];
+    double xi = ddiv(hsum, hscale);
+    #pragma unroll 1
+    for (int i = j + 2; i >= 2; --i) l[i] = l[i] * xi + l[i - 1];
+  }
+  #pragma unroll 1
+  for (int i = lane; i < n; i += 32)
+    #pragma unroll 1
+    for (int j = 2; j < q; ++j) (zb + (j) * n)[i] -= l[j] * (zb + (q) * n)[i];
+  __syncwarp();
+}
+// acor and y of the first Newton iterate: the prediction made non-negative;
+// whether this lane changed a value and whether one is not a number >= 0
+__device__ __noinline__ int vec_start(const double* zb, double* acor, double* y, int n,
+                                      int lane) {
+  int flags = 0;
+  #pragma unroll 1
+  for (int i = lane; i < n; i += 32) {
+    const double z = zb[i], a = z < 0.0 ? -z : 0.0, s = z + a;
+    sh(acor)[i] = a;
+    sh(y)[i] = s;
+    flags |= (a != 0.0 ? kProjected : 0) | (s >= 0.0 ? 0 : kOdd);
+  }
+  __syncwarp();
+  return flags;
+}
 // One cell's CVODE BDF integration, run by one warp (lane-strided vector
 // loops, warp reductions).  BLK: the CTA-per-cell form, whose heavy
 // operations (f, J, factorization, solves) run on the whole block through
@@ -1519,19 +1672,13 @@ struct Cell {
   int q, qprime, qwait, L, jcur;
   double h, hprime, hscale, eta, etamax, hu, next_h, tn;
   double *tau, *tq, *l;  // per-warp shared scalars (all lanes hold equal values)
+  double* quot;          // quotients of set()
   double rl1, gamma, gammap, gamrat, crate, acnrm, saved_tq5;
   int nst, nfe, nsetups, netf, nni, ncfn, nje, nstlp, nstlj;
 
-  __device__ double wrms(const double* v) const {
-    double s = 0.0;
-    #pragma unroll 1
-    for (int i = lane; i < n; i += 32) {
-      double t = v[i] * ewt[i];
-      s += t * t;
-    }
-    return rms(warp_sum(s), (double)n, rn);
-  }
-  __device__ int f(const double* yy, double* out) {
+  __device__ double wrms(const double* v) const { return vec_wrms(v, ewt, n, rn, lane); }
+  // flags: kOdd where this lane's share of yy is not all >= 0
+  __device__ int f(const double* yy, double* out, int flags) {
     if constexpr (BLK) {
       bool bad = false;
       #pragma unroll 1
@@ -1540,9 +1687,9 @@ struct Cell {
       blk::call<LT>(cmd, *bx, blk::OP_F, yy, out, h > 0.0 ? h : h0);
       return 0;
     } else if constexpr (AERO)
-      return dev_f_aero<LT>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane);
+      return dev_f_aero<LT>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
     else
-      return dev_f<LT>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane);
+      return dev_f<LT>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
   }
   __device__ bool set_ewt(const double* yy) {
     bool bad = false;
@@ -1571,45 +1718,24 @@ struct Cell {
     return !warp_any(odd);
   }
   __device__ void rescale() {
-    double factor = eta;
-    #pragma unroll 1
-    for (int j = 1; j <= q; ++j) {
-      #pragma unroll 1
-      for (int i = lane; i < n; i += 32) (zb + (j) * n)[i] *= factor;
-      factor *= eta;
-    }
-    __syncwarp();
+    hist_rescale(zb, n, q, eta, lane);
     h = hscale * eta;
     next_h = h;
     hscale = h;
   }
-  // zn <- zn * Pascal(q) (sign +1) or its inverse (sign -1), one element's
-  // q+1 history values at a time in registers: for k = 1..q, j = q..k,
-  // zn[j-1] += sign * zn[j]
-  __device__ void pascal(double sign) {
-    #pragma unroll 1
-    for (int i = lane; i < n; i += 32) {
-      double v[LMAX];
-#pragma unroll
-      for (int j = 0; j < LMAX; ++j) v[j] = (j <= q) ? zb[j * n + i] : 0.0;
-#pragma unroll
-      for (int k = 1; k <= QMAX; ++k)
-#pragma unroll
-        for (int j = QMAX; j >= 1; --j)
-          if (k <= q && j >= k && j <= q) v[j - 1] += sign * v[j];
-#pragma unroll
-      for (int j = 0; j < QMAX; ++j)
-        if (j < q) zb[j * n + i] = v[j];
-    }
-    __syncwarp();
-  }
-  __device__ void predict() {
+  __device__ int predict() {
     tn += h;
-    pascal(1.0);
+    return hist_pascal(zb, n, q, 1.0, acor, y, lane);
   }
   __device__ void restore(double saved_t) {
     tn = saved_t;
-    pascal(-1.0);
+    hist_pascal(zb, n, q, -1.0, nullptr, nullptr, lane);
+  }
+  // one value per lane (the first eight) into quot, for every lane to read
+  __device__ void share(double v) {
+    __syncwarp();
+    if (lane < 8) quot[lane] = v;
+    __syncwarp();
   }
   // l and tq of the fixed-leading-coefficient BDF formula.  Its dozen
   // divisions are a serial chain only in part: they are taken in three turns,
@@ -1619,7 +1745,7 @@ struct Cell {
     double hsum = h;
     #pragma unroll 1
     for (int j = 1; j <= q; ++j) hsum += lane > j ? tau[j] : 0.0;
-    const double xi = h / hsum;
+    share(ddiv(h, hsum));
     double c[LMAX];
     c[0] = c[1] = 1.0;
 #pragma unroll
@@ -1630,12 +1756,12 @@ struct Cell {
 #pragma unroll
       for (int j = 2; j < QMAX; ++j)
         if (j < q) {
-          const double x = __shfl_sync(FULLMASK, xi, j);
+          const double x = quot[j];
 #pragma unroll
           for (int i = j; i >= 1; --i) c[i] += c[i - 1] * x;
         }
       xistar_inv = -c[1] - alpha0;
-      xi_inv = __shfl_sync(FULLMASK, xi, q);
+      xi_inv = quot[q];
       alpha0_hat = -c[1] - xi_inv;
 #pragma unroll
       for (int i = QMAX; i >= 1; --i)
@@ -1650,7 +1776,7 @@ struct Cell {
     const double A1 = 1.0 - alpha0_hat + alpha0;
     const double A2 = 1.0 + q * A1;
     const bool next_order = qwait == 1;
-    const double xi_next = next_order ? __shfl_sync(FULLMASK, xi, q + 1) : 1.0;
+    const double xi_next = next_order ? quot[q + 1] : 1.0;
     const double A3 = alpha0 + kInvInt[q], A4 = alpha0_hat + xi_inv;
     const double A5 = alpha0 - kInvInt[q + 1], A6 = alpha0_hat - xi_next;
     double num = A1, den = alpha0 * A2;
@@ -1659,80 +1785,30 @@ struct Cell {
     if (lane == 3) num = xistar_inv, den = cq;
     if (lane == 4) num = 1.0 - A4 + A3, den = A3;
     if (lane == 5) num = 1.0 - A6 + A5, den = A2;
-    const double r = num / den;
-    const double tq2 = fabs(__shfl_sync(FULLMASK, r, 0));
-    const double tq5 = fabs(__shfl_sync(FULLMASK, r, 1));
-    rl1 = __shfl_sync(FULLMASK, r, 2);
+    share(ddiv(num, den));
+    const double tq2 = fabs(quot[0]);
+    tq[2] = tq2;
+    tq[5] = fabs(quot[1]);
+    rl1 = quot[2];
     gamma = h * rl1;
     if (nst == 0) gammap = gamma;
     num = NLSCOEF;
     den = tq2;
     if (lane == 1) num = gamma, den = gammap;
     if (next_order) {
-      const double C = __shfl_sync(FULLMASK, r, 3), Cpinv = __shfl_sync(FULLMASK, r, 4);
-      const double Cppinv = __shfl_sync(FULLMASK, r, 5);
-      tq[1] = q > 1 ? fabs(C * Cpinv) : 1.0;
-      if (lane == 2) num = Cppinv, den = xi_next * (q + 2) * A5;
+      tq[1] = q > 1 ? fabs(quot[3] * quot[4]) : 1.0;
+      if (lane == 2) num = quot[5], den = xi_next * (q + 2) * A5;
     }
-    const double s = num / den;
-    tq[2] = tq2;
-    tq[5] = tq5;
-    tq[4] = __shfl_sync(FULLMASK, s, 0);
-    const double ratio = __shfl_sync(FULLMASK, s, 1);
-    gamrat = (nst > 0) ? ratio : 1.0;
-    if (next_order) tq[3] = fabs(__shfl_sync(FULLMASK, s, 2));
-  }
-  __device__ void increase_order() {
-    #pragma unroll 1
-    for (int i = 0; i <= QMAX; ++i) l[i] = 0.0;
-    l[2] = 1.0;
-    double alpha1 = 1.0, prod = 1.0, xiold = 1.0, alpha0 = -1.0, hsum = hscale;
-    if (q > 1) {
-      #pragma unroll 1
-      for (int j = 1; j < q; ++j) {
-        hsum += tau[j + 1];
-        double xi = ddiv(hsum, hscale);
-        prod *= xi;
-        alpha0 -= ddiv(1.0, (double)(j + 1));
-        alpha1 += ddiv(1.0, xi);
-        #pragma unroll 1
-        for (int i = j + 2; i >= 2; --i) l[i] = l[i] * xiold + l[i - 1];
-        xiold = xi;
-      }
-    }
-    double A1 = ddiv(-alpha0 - alpha1, prod);
-    #pragma unroll 1
-    for (int i = lane; i < n; i += 32) {
-      double top = A1 * (zb + (QMAX) * n)[i];
-      (zb + (q + 1) * n)[i] = top;
-      #pragma unroll 1
-      for (int j = 2; j <= q; ++j) (zb + (j) * n)[i] += l[j] * top;
-    }
-    __syncwarp();
-  }
-  __device__ void decrease_order() {
-    #pragma unroll 1
-    for (int i = 0; i <= QMAX; ++i) l[i] = 0.0;
-    l[2] = 1.0;
-    double hsum = 0.0;
-    #pragma unroll 1
-    for (int j = 1; j <= q - 2; ++j) {
-      hsum += tau[j];
-      double xi = ddiv(hsum, hscale);
-      #pragma unroll 1
-      for (int i = j + 2; i >= 2; --i) l[i] = l[i] * xi + l[i - 1];
-    }
-    #pragma unroll 1
-    for (int i = lane; i < n; i += 32)
-      #pragma unroll 1
-      for (int j = 2; j < q; ++j) (zb + (j) * n)[i] -= l[j] * (zb + (q) * n)[i];
-    __syncwarp();
+    share(ddiv(num, den));
+    tq[4] = quot[0];
+    gamrat = (nst > 0) ? quot[1] : 1.0;
+    if (next_order) tq[3] = fabs(quot[2]);
   }
   __device__ void adjust_order(int dq) {
     if (dq == 1)
-      increase_order();
+      hist_increase(zb, n, q, hscale, tau, l, lane);
     else if (dq == -1)
-      decrease_order();
+      hist_decrease(zb, n, q, hscale, tau, l, lane);
   }
   __device__ void adjust_params() {
     if (qprime != q) {
@@ -1745,7 +1821,7 @@ struct Cell {
   }
   // J reuse rule of the CVODE direct linear solver interface; returns 0, or
   // >0 for a recoverable failure
-  __device__ int lsetup(int convfail, const double* ypred) {
+  __device__ int lsetup(int convfail, const double* ypred, int flags) {
     double dgamma = fabs(ddiv(gamma, gammap) - 1.0);
     bool jbad = (nst == 0) || (nst > nstlj + MSBJ) ||
                 ((convfail == FAIL_BAD_J) && (dgamma < DGMAX_J)) || (convfail == FAIL_OTHER);
@@ -1764,9 +1840,9 @@ struct Cell {
         blk::call<LT>(cmd, *bx, blk::OP_JAC, ypred, nullptr, h > 0.0 ? h : h0);
         jr = 0;
       } else if constexpr (AERO) {
-        jr = dev_jac_aero<LT>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane);
+        jr = dev_jac_aero<LT>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
       } else {
-        jr = dev_jac<LT>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane);
+        jr = dev_jac<LT>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
       }
       if (jr) return 1;
     }
@@ -1775,7 +1851,8 @@ struct Cell {
                             : dev_form_factor<LT>(tb, J, gamma, LU, dinv, lane);
     return ok ? 0 : 1;
   }
-  __device__ int newton(bool projected) {
+  // viol: whether this lane's share of the converged y has a negative value
+  __device__ int newton(bool projected, bool* viol) {
     int mm = 0;
     double del, delp = 0.0;
     // the correction of a matrix whose gamma has moved since (1.0: not moved)
@@ -1801,9 +1878,11 @@ struct Cell {
       else if (lu_mode)
         dev_lsolve_seq<LT>(tb, LU, dinv, z, lane);
       else
-        dev_lsolve<LT>(tb, LU, dinv, z, lane);
+        dev_lsolve<LT>(LU, dinv, z, lane);
       nni++;
       double sum = 0.0;
+      int flags = 0;
+      *viol = false;
       #pragma unroll 1
       for (int i = lane; i < n; i += 32) {
         double v;
@@ -1817,9 +1896,12 @@ struct Cell {
         sum += t * t;
         const double a = acor[i] + d;
         acor[i] = a;
-        y[i] = (zb + (0) * n)[i] + a;
+        const double yn = (zb + (0) * n)[i] + a;
+        y[i] = yn;
+        flags |= yn >= 0.0 ? 0 : kOdd;
+        *viol |= yn < 0.0;
       }
-      del = rms(warp_sum(sum), (double)n, rn);
+      del = warp_rms(sum, n, rn);
       __syncwarp();
       if (mm > 0) crate = fmax(CRDOWN * crate, ddiv(del, delp));
       // del * min(1, crate) / tq[4] <= 1 (tq[4] > 0: the same without dividing)
@@ -1832,25 +1914,23 @@ struct Cell {
       if ((mm == MAXCOR) || ((mm >= 2) && (del > RDIV * delp)))
         return jcur ? NL_CONV_FAIL : NL_TRY_AGAIN;
       delp = del;
-      int r = f(y, ftemp);
+      int r = f(y, ftemp, flags);
       nfe++;
       if (r > 0) return jcur ? NL_RHS_RECVR : NL_TRY_AGAIN;
     }
   }
   // non-negativity of the converged iterate (CVODE's cvCheckConstraints
   // with constraint >= 0 on every component)
-  __device__ int check_constraints() {
-    bool viol = false;
+  __device__ int check_constraints(bool viol) {
+    if (!warp_any(viol)) return NL_OK;
     double s = 0.0;
     #pragma unroll 1
     for (int i = lane; i < n; i += 32)
       if (y[i] < 0.0) {
-        viol = true;
         double t = y[i] * ewt[i];
         s += t * t;
       }
-    if (!warp_any(viol)) return NL_OK;
-    double vnorm = rms(warp_sum(s), (double)n, rn);
+    double vnorm = warp_rms(s, n, rn);
     if (vnorm <= tq[4]) {
       #pragma unroll 1
       for (int i = lane; i < n; i += 32)
@@ -1873,30 +1953,19 @@ struct Cell {
     eta = e > 0.1 ? e : 0.1;
     return NL_CONSTR_RECVR;
   }
-  __device__ bool start_guess() {
-    bool proj = false;
-    #pragma unroll 1
-    for (int i = lane; i < n; i += 32) {
-      double a = (zb + (0) * n)[i] < 0.0 ? -(zb + (0) * n)[i] : 0.0;
-      proj |= a != 0.0;
-      acor[i] = a;
-      y[i] = (zb + (0) * n)[i] + a;
-    }
-    __syncwarp();
-    return warp_any(proj);
-  }
-  __device__ int nls(int nflag) {
+  // start: the flags of the first iterate, which the prediction has set
+  __device__ int nls(int nflag, int start) {
     int convfail = ((nflag == FIRST_CALL) || (nflag == PREV_ERR_FAIL)) ? NO_FAILURES : FAIL_OTHER;
     bool call_setup = (nflag == PREV_CONV_FAIL) || (nflag == PREV_ERR_FAIL) || (nst == 0) ||
                       (nst >= nstlp + MSBP) || (fabs(gamrat - 1.0) > DGMAX);
-    bool projected = start_guess();
     #pragma unroll 1
     for (;;) {
-      int r = f(y, ftemp);
+      const bool projected = warp_any((start & kProjected) != 0);
+      int r = f(y, ftemp, start & kOdd);
       nfe++;
       if (r > 0) return NL_RHS_RECVR;
       if (call_setup) {
-        int ier = lsetup(convfail, y);
+        int ier = lsetup(convfail, y, start & kOdd);
         nsetups++;
         call_setup = false;
         gamrat = crate = 1.0;
@@ -1904,12 +1973,13 @@ struct Cell {
         nstlp = nst;
         if (ier > 0) return NL_CONV_FAIL;
       }
-      int ier = newton(projected);
-      if (ier == NL_OK) return check_constraints();
+      bool viol;
+      int ier = newton(projected, &viol);
+      if (ier == NL_OK) return check_constraints(viol);
       if (ier != NL_TRY_AGAIN) return ier;
       call_setup = true;
       convfail = FAIL_BAD_J;
-      projected = start_guess();
+      start = vec_start(zb, acor, y, n, lane);
     }
   }
   __device__ int handle_nflag(int* nflag, double saved_t, int* ncf) {
@@ -1958,7 +2028,7 @@ struct Cell {
     #pragma unroll 1
     for (int i = lane; i < n; i += 32) y[i] = zb[i];
     __syncwarp();
-    int r = f(y, ftemp);
+    int r = f(y, ftemp, vec_odd(y, n, lane));
     nfe++;
     if (r > 0) return UNREC_RHSFUNC_ERR;
     #pragma unroll 1
@@ -1977,13 +2047,9 @@ struct Cell {
     #pragma unroll 1
     for (int i = lane; i < n; i += 32) {
       const double a = acor[i];
-      double v[LMAX];
-#pragma unroll
-      for (int j = 0; j < LMAX; ++j)
-        if (j <= q) v[j] = zb[j * n + i];
-#pragma unroll
-      for (int j = 0; j < LMAX; ++j)
-        if (j <= q) zb[j * n + i] = v[j] + l[j] * a;
+      double* z = zb + i;
+      #pragma unroll 1
+      for (int j = 0; j <= q; ++j, z += n) *z += l[j] * a;
       if (save) (zb + (QMAX) * n)[i] = a;
     }
     __syncwarp();
@@ -2070,9 +2136,9 @@ struct Cell {
     if ((nst > 0) && (hprime != h)) adjust_params();
     #pragma unroll 1
     for (;;) {
-      predict();
+      const int start = predict();
       set();
-      nflag = nls(nflag);
+      nflag = nls(nflag, start);
       int kflag = handle_nflag(&nflag, saved_t, &ncf);
       if (kflag == PREDICT_AGAIN) continue;
       if (kflag != DO_ERROR_TEST) return kflag;
@@ -2118,7 +2184,7 @@ struct Cell {
     __syncwarp();
     if (!set_ewt((zb + (0) * n))) return ILL_INPUT;
     next_h = 0.0;
-    if (f(y, ftemp)) return REPTD_RHSFUNC_ERR;
+    if (f(y, ftemp, vec_odd(y, n, lane))) return REPTD_RHSFUNC_ERR;
     nfe++;
     h = h0;
     // a zero initial step makes CVODE estimate one (cvHin), which refuses an
@@ -2177,6 +2243,7 @@ __device__ void bind_cell(Cell<LT, AERO>& c, const SolveArgs& a, const char* tab
   c.tau = ctl;
   c.tq = ctl + (LMAX + 2);
   c.l = ctl + (LMAX + 2) + 8;
+  c.quot = ctl + (LMAX + 2) + 8 + (LMAX + 1);
   c.ewt = (double*)(base + a.lay.ewt);
   c.acor = (double*)(base + a.lay.acor);
   c.y = (double*)(base + a.lay.y);
@@ -2380,6 +2447,7 @@ __global__ void __launch_bounds__(blk::kThreads, sizeof(LT) == 4 ? 2 : 1)
     c.tau = ctl;
     c.tq = ctl + (LMAX + 2);
     c.l = ctl + (LMAX + 2) + 8;
+    c.quot = ctl + (LMAX + 2) + 8 + (LMAX + 1);
     c.ewt = (double*)(smem + L.ewt);
     c.acor = (double*)(smem + L.acor);
     c.y = (double*)(smem + L.y);
@@ -2444,6 +2512,12 @@ __global__ void __launch_bounds__(blk::kThreads, sizeof(LT) == 4 ? 2 : 1)
   }
 }
 
+// CSC entry of every Jacobian slot
+__device__ __forceinline__ const uint16_t* csc_of(const char* tb) {
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  return (const uint16_t*)((const char*)o.self + o.j_csc);
+}
+
 struct EvalArgs {
   DevMech m;
   BlobOff off;
@@ -2482,22 +2556,28 @@ __global__ void eval_kernel(EvalArgs a) {
   set_unit(y, t.n, lane);
   compute_keff(m, st, a.env[2 * cell], a.env[2 * cell + 1],
                a.photo ? a.photo + (size_t)cell * m.n_photo : nullptr, keff, lane);
+  const int odd = vec_odd(y, t.n, lane);
   if (!a.do_jac) {
     double* out = (double*)(base + a.lay.ftemp);
     if (has_simpol(smem))
-      dev_f_aero<double>(smem, y, a.h, keff, rates, fscr, out, lane, a.rp + (size_t)cell * t.n,
+      dev_f_aero<double, true>(smem, y, a.h, keff, rates, fscr, out, lane, odd,
+                       a.rp + (size_t)cell * t.n,
                  a.rl + (size_t)cell * t.n);
     else
-      dev_f<double>(smem, y, a.h, keff, rates, fscr, out, lane, a.rp + (size_t)cell * t.n,
+      dev_f<double, true>(smem, y, a.h, keff, rates, fscr, out, lane, odd,
+                       a.rp + (size_t)cell * t.n,
             a.rl + (size_t)cell * t.n);
     #pragma unroll 1
     for (int i = lane; i < t.n; i += 32) a.f[(size_t)cell * t.n + i] = out[i];
   } else {
+    const uint16_t* csc = csc_of(smem);
     if (has_simpol(smem))
-      dev_jac_aero<double>(smem, y, a.h, keff, rates, a.jv + (size_t)cell * t.n_jac, lane,
+      dev_jac_aero<double, true>(smem, y, a.h, keff, rates, a.jv + (size_t)cell * t.n_jac, lane,
+                           odd, csc,
                            a.jp + (size_t)cell * t.n_jac, a.jl + (size_t)cell * t.n_jac);
     else
-      dev_jac<double>(smem, y, a.h, keff, rates, a.jv + (size_t)cell * t.n_jac, lane,
+      dev_jac<double, true>(smem, y, a.h, keff, rates, a.jv + (size_t)cell * t.n_jac, lane,
+                           odd, csc,
                       a.jp + (size_t)cell * t.n_jac, a.jl + (size_t)cell * t.n_jac);
   }
 }
@@ -2554,9 +2634,10 @@ __global__ void jac_check_kernel(CheckArgs c) {
   compute_keff(m, st, a.env[2 * cell], a.env[2 * cell + 1],
                a.photo ? a.photo + (size_t)cell * m.n_photo : nullptr, keff, lane);
   const bool aero = has_simpol(smem);
-  if (dev_f_aero<double>(smem, y, a.h, keff, rates, fscr, f0, lane, rp0, rl0) ||
-      (aero ? dev_jac_aero<double>(smem, y, a.h, keff, rates, J, lane)
-            : dev_jac<double>(smem, y, a.h, keff, rates, J, lane))) {
+  const int odd = vec_odd(y, t.n, lane);
+  if (dev_f_aero<double, true>(smem, y, a.h, keff, rates, fscr, f0, lane, odd, rp0, rl0) ||
+      (aero ? dev_jac_aero<double, true>(smem, y, a.h, keff, rates, J, lane, odd, csc_of(smem))
+            : dev_jac<double, true>(smem, y, a.h, keff, rates, J, lane, odd, csc_of(smem)))) {
     if (lane == 0) {
       c.nfail[cell] = -1;
       c.worst[cell] = -1.0;
@@ -2579,10 +2660,10 @@ __global__ void jac_check_kernel(CheckArgs c) {
       const double dx = x * scale;
       if (lane == 0) y[j] = x + dx;
       __syncwarp();
-      int r = dev_f_aero<double>(smem, y, a.h, keff, rates, fscr, f1, lane);
+      int r = dev_f_aero<double, true>(smem, y, a.h, keff, rates, fscr, f1, lane, vec_odd(y, t.n, lane));
       if (lane == 0) y[j] = x + 0.5 * dx;
       __syncwarp();
-      r |= dev_f_aero<double>(smem, y, a.h, keff, rates, fscr, f2, lane);
+      r |= dev_f_aero<double, true>(smem, y, a.h, keff, rates, fscr, f2, lane, vec_odd(y, t.n, lane));
       if (lane == 0) y[j] = x;
       __syncwarp();
       if (r) continue;
@@ -2679,8 +2760,9 @@ __global__ void precision_kernel(PrecArgs p) {
   set_unit(y, t.n, lane);
   compute_keff(m, st, a.env[2 * cell], a.env[2 * cell + 1],
                a.photo ? a.photo + (size_t)cell * m.n_photo : nullptr, keff, lane);
-  int r = has_simpol(smem) ? dev_jac_aero<LT>(smem, y, a.h, keff, rates, J, lane)
-                           : dev_jac<LT>(smem, y, a.h, keff, rates, J, lane);
+  const int odd = vec_odd(y, t.n, lane);
+  int r = has_simpol(smem) ? dev_jac_aero<LT>(smem, y, a.h, keff, rates, J, lane, odd)
+                           : dev_jac<LT>(smem, y, a.h, keff, rates, J, lane, odd);
   bool ok = r == 0 && dev_form_factor<LT>(smem, J, a.h, LU, dinv, lane);
   if (ok) {
     #pragma unroll 1
@@ -2690,7 +2772,7 @@ __global__ void precision_kernel(PrecArgs p) {
     }
     if (lane == 0) z[t.n] = (LT)0;
     __syncwarp();
-    dev_lsolve<LT>(smem, LU, dinv, z, lane);
+    dev_lsolve<LT>(LU, dinv, z, lane);
     #pragma unroll 1
     for (int i = lane; i < t.n; i += 32)
       p.x[(size_t)cell * t.n + i] = (double)z[t.lu_iperm[i]];
@@ -2993,8 +3075,8 @@ static Layout make_layout(const BlobOff& o, int lt_size, bool with_hist,
   // a spare slot: see clear_spare
   L.lu = take((size_t)lt_size * (o.n_lu + 1));
   L.dinv = take((size_t)lt_size * o.n);
-  // control block: tau[LMAX + 2], tq[8], l[LMAX + 1]
-  L.ctl = take(sizeof(double) * (LMAX + 2 + 8 + LMAX + 1));
+  // control block: tau[LMAX + 2], tq[8], l[LMAX + 1], quot[8]
+  L.ctl = take(sizeof(double) * (LMAX + 2 + 8 + LMAX + 1 + 8));
   L.bytes = (int)off;
   return L;
 }
@@ -3104,7 +3186,7 @@ static BlkLayout make_blk_layout(const BlockOff& o, int lt, bool zn_in_smem) {
   };
   const size_t n = (size_t)o.n;
   L.ctx = take(sizeof(blk::Ctx<double>));
-  L.ctl = take(sizeof(double) * (LMAX + 2 + 8 + LMAX + 1));
+  L.ctl = take(sizeof(double) * (LMAX + 2 + 8 + LMAX + 1 + 8));
   L.y = take(8 * n);
   L.ewt = take(8 * n);
   L.acor = take(8 * n);
