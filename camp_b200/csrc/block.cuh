@@ -259,12 +259,25 @@ __device__ __noinline__ bool op_factor(const Ctx<LT>& c, double gamma) {
   LT* LU = c.LU;
   const int tid = threadIdx.x;
   const int n = t.n, r0 = t.r0, m = n - r0;
+  // M = I - gamma*J, kForm positions per thread and turn: their table words,
+  // then their J values (both in global memory) in flight together
+  constexpr int kForm = 8;
   #pragma unroll 1
-  for (int p = tid; p < t.n_lu; p += kThreads) {
-    const int s = __ldg(t.lu_src + p);
-    double v = (s & 0x7FFF) ? -gamma * (double)c.J[(s & 0x7FFF) - 1] : 0.0;
-    if (s & 0x8000) v += 1.0;
-    LU[p] = (LT)v;
+  for (int p0 = tid; p0 < t.n_lu; p0 += kForm * kThreads) {
+    int s[kForm];
+    LT v[kForm];
+    #pragma unroll
+    for (int k = 0; k < kForm; ++k)
+      s[k] = p0 + k * kThreads < t.n_lu ? __ldg(t.lu_src + p0 + k * kThreads) : 0;
+    #pragma unroll
+    for (int k = 0; k < kForm; ++k) v[k] = (s[k] & 0x7FFF) ? c.J[(s[k] & 0x7FFF) - 1] : (LT)0;
+    #pragma unroll
+    for (int k = 0; k < kForm; ++k)
+      if (p0 + k * kThreads < t.n_lu) {
+        double d = (s[k] & 0x7FFF) ? -gamma * (double)v[k] : 0.0;
+        if (s[k] & 0x8000) d += 1.0;
+        LU[p0 + k * kThreads] = (LT)d;
+      }
   }
   #pragma unroll 1
   for (int e = tid; e < kXBuf; e += kThreads) c.xbuf[e] = (LT)0;
@@ -305,7 +318,7 @@ __device__ __noinline__ bool op_factor(const Ctx<LT>& c, double gamma) {
     const LT piv = LU[c.diag[k]];
     const bool pb = (piv == (LT)0) || !isfinite((double)piv);
     bad |= pb;
-    const LT dk = pb ? (LT)0 : (LT)(1.0 / (double)piv);
+    const LT dk = pb ? (LT)0 : (LT)__drcp_rn((double)piv);
     if (tid == 0) c.dinv[k] = dk;
     // the buffer two pivots on (last read before the previous barrier)
     LT* nb = c.xbuf + ((k + 1) % 3) * (2 * kMaxDense);
@@ -355,16 +368,21 @@ __device__ __noinline__ bool op_factor(const Ctx<LT>& c, double gamma) {
     for (int e = tid + kThreads; e < ne; e += kThreads) LU[__ldg(t.lk + e0 + e) & 0xFFFFu] *= dk;
     LT lv[kTile], uv[kTile];
     #pragma unroll
-    for (int s = 0; s < kTile; ++s) lv[s] = (p + 16 * s < m) ? lb[p + 16 * s] : (LT)0;
+    for (int s = 0; s < kTile; ++s) lv[s] = lb[p + 16 * s];  // zero past the block
     #pragma unroll
-    for (int u = 0; u < kTile; ++u) uv[u] = (q + 16 * u < m) ? ubf[q + 16 * u] : (LT)0;
+    for (int u = 0; u < kTile; ++u) uv[u] = ubf[q + 16 * u];
     #pragma unroll
     for (int s = 0; s < kTile; ++s)
     #pragma unroll
       for (int u = 0; u < kTile; ++u) a[s][u] -= lv[s] * uv[u];
   }
   // dense pivots: kk = 16 s0 + kq, held by the threads with q == kq
-  // (column), p == kq (row) and both (pivot)
+  // (column), p == kq (row) and both (pivot).  Tile rows and columns before s0
+  // are finished, those after it wholly trailing, so only row and column s0
+  // compare with the pivot; entries past the block are zero and stay zero.
+  // Bound by instruction fetch and issue (every thread runs all of it for every
+  // pivot): with a bound check on each of the 14 rows and columns and each of
+  // the 49 updates this was 560 instructions a pivot.
   #pragma unroll
   for (int s0 = 0; s0 < kTile; ++s0) {
     #pragma unroll 1
@@ -375,57 +393,49 @@ __device__ __noinline__ bool op_factor(const Ctx<LT>& c, double gamma) {
       LT* lb = c.xbuf + (k % 3) * (2 * kMaxDense);
       LT* ubf = lb + kMaxDense;
       if (q == kq) {
+        if (p > kq) lb[p + 16 * s0] = a[s0][s0];
         #pragma unroll
-        for (int s = 0; s < kTile; ++s) {
-          const int di = p + 16 * s;
-          if (di > kk && di < m) lb[di] = a[s][s0];
-        }
+        for (int s = s0 + 1; s < kTile; ++s) lb[p + 16 * s] = a[s][s0];
         if (p == kq) {
           // the pivot's owner publishes its reciprocal (0 for a zero or
           // non-finite pivot), so no other thread divides
           const LT pv = a[s0][s0];
           const bool pbad = (pv == (LT)0) || !isfinite((double)pv);
-          lb[kk] = pbad ? (LT)0 : (LT)(1.0 / (double)pv);
+          lb[kk] = pbad ? (LT)0 : (LT)__drcp_rn((double)pv);
         }
       }
       if (p == kq) {
+        if (q > kq) ubf[q + 16 * s0] = a[s0][s0];
         #pragma unroll
-        for (int u = 0; u < kTile; ++u) {
-          const int dj = q + 16 * u;
-          if (dj > kk && dj < m) ubf[dj] = a[s0][u];
-        }
+        for (int u = s0 + 1; u < kTile; ++u) ubf[q + 16 * u] = a[s0][u];
       }
       bsync();
       const LT dk = lb[kk];
       bad |= dk == (LT)0;
       if (tid == 0) c.dinv[k] = dk;
       LT lv[kTile], uv[kTile];
+      lv[s0] = p > kq ? lb[p + 16 * s0] * dk : (LT)0;
+      uv[s0] = q > kq ? ubf[q + 16 * s0] : (LT)0;
       #pragma unroll
-      for (int s = 0; s < kTile; ++s) {
-        const int di = p + 16 * s;
-        lv[s] = (di > kk && di < m) ? lb[di] * dk : (LT)0;
+      for (int s = s0 + 1; s < kTile; ++s) lv[s] = lb[p + 16 * s] * dk;
+      #pragma unroll
+      for (int u = s0 + 1; u < kTile; ++u) uv[u] = ubf[q + 16 * u];
+      // the pivot's column becomes its multipliers
+      if (q == kq) {
+        if (p > kq) a[s0][s0] = lv[s0];
+        #pragma unroll
+        for (int s = s0 + 1; s < kTile; ++s) a[s][s0] = lv[s];
       }
       #pragma unroll
-      for (int u = 0; u < kTile; ++u) {
-        const int dj = q + 16 * u;
-        uv[u] = (dj > kk && dj < m) ? ubf[dj] : (LT)0;
+      for (int s = s0 + 1; s < kTile; ++s) {
+        #pragma unroll
+        for (int u = s0 + 1; u < kTile; ++u) a[s][u] -= lv[s] * uv[u];
       }
-      // branch-free: lv / uv are zero outside the trailing rows / columns,
-      // so the update leaves row kk, column kk and the rest unchanged there
-      #pragma unroll
-      for (int s = 0; s < kTile; ++s) {
-        const bool sc = q == kq && p + 16 * s > kk;
-        a[s][s0] = sc ? a[s][s0] * dk : a[s][s0];
-      }
-      // tile rows / columns wholly at or before the pivot are finished:
-      // the branch is the same for the whole block
-      #pragma unroll
-      for (int s = 0; s < kTile; ++s) {
-        if (16 * s + 15 > kk) {
-          #pragma unroll
-          for (int u = 0; u < kTile; ++u)
-            if (16 * u + 15 > kk) a[s][u] -= lv[s] * uv[u];
-        }
+      if (kq < 15) {  // row and column s0 are finished after their last pivot
+        #pragma unroll
+        for (int u = s0; u < kTile; ++u) a[s0][u] -= lv[s0] * uv[u];
+        #pragma unroll
+        for (int s = s0 + 1; s < kTile; ++s) a[s][s0] -= lv[s] * uv[s0];
       }
     }
   }
