@@ -59,10 +59,14 @@ struct GatherItem {
     if (c == 1) o.insert(o.end(), neg.begin(), neg.end());
     return o;
   }
-  int longest() const {
-    size_t m = 0;
-    for (int c = 0; c < 4; ++c) m = std::max(m, chain(c).size());
-    return (int)m;
+  int longest = 0, padded = 0;  // longest chain; entries in multiples of four
+  void measure() {
+    const int len[4] = {(int)(loss.size() + 1) / 2, (int)(loss.size() / 2 + neg.size()),
+                        (int)(lead.size() + (prod.size() + 1) / 2), (int)prod.size() / 2};
+    for (int v : len) {
+      longest = std::max(longest, v);
+      padded += (v + 3) / 4 * 4;
+    }
   }
 };
 
@@ -74,97 +78,115 @@ struct GatherTables {
 // with a lane per item (blob.hpp).  A chain round costs its longest chain (11
 // instructions an entry, 45 for the reduction), an item round its longest
 // lists (9 a word, 30 besides) and their padded words; with the longest chains
-// first, the number of chain rounds with the least sum is taken,
-// `bytes_per_inst` table bytes counting as one instruction.
+// first, the number of chain rounds and the order of the rest with the least
+// sum are taken, `bytes_per_inst` table bytes counting as one instruction.
 void pack_gather(std::vector<GatherItem> items, uint32_t zero, int bytes_per_inst,
                  GatherTables* o) {
-  std::stable_sort(items.begin(), items.end(), [](const GatherItem& a, const GatherItem& b) {
-    return !a.neg.empty() != !b.neg.empty() ? !a.neg.empty() : a.longest() > b.longest();
-  });
   auto half = [](size_t n) { return (int)(n + 1) / 2; };
   auto up = [](int n, int m) { return (n + m - 1) / m * m; };
-  // the items from `first` on in rounds of 32, similar lists together
-  auto rest = [&](size_t first) {
-    std::vector<const GatherItem*> r;
-    for (size_t k = first; k < items.size(); ++k) r.push_back(&items[k]);
-    std::stable_sort(r.begin(), r.end(), [&](const GatherItem* a, const GatherItem* b) {
-      auto w = [&](const GatherItem* x) {
-        return up(half(x->loss.size()), 2) + up((int)x->prod.size(), 2) + (int)x->lead.size();
-      };
-      return w(a) > w(b);
-    });
-    return r;
-  };
+  for (GatherItem& x : items) x.measure();
+  std::stable_sort(items.begin(), items.end(), [](const GatherItem& a, const GatherItem& b) {
+    return !a.neg.empty() != !b.neg.empty() ? !a.neg.empty() : a.longest > b.longest;
+  });
+  const int n = (int)items.size();
   struct Steps {
     int u = 0, l = 0, p = 0;
   };
-  auto steps = [&](const std::vector<const GatherItem*>& r, size_t k0) {
+  std::vector<Steps> sh(n);
+  for (int k = 0; k < n; ++k)
+    sh[k] = {(int)items[k].lead.size(), half(items[k].loss.size()), (int)items[k].prod.size()};
+  // orders that put similar lists together: by words, products, losses
+  std::vector<std::vector<int>> orders(3, std::vector<int>(n));
+  for (int w = 0; w < 3; ++w) {
+    std::iota(orders[w].begin(), orders[w].end(), 0);
+    std::stable_sort(orders[w].begin(), orders[w].end(), [&](int a, int b) {
+      const Steps &x = sh[a], &y = sh[b];
+      if (w == 1 && x.p != y.p) return x.p > y.p;
+      if (w == 2 && x.l != y.l) return x.l > y.l;
+      return x.u + x.l + x.p > y.u + y.l + y.p;
+    });
+  }
+  // the items from `first` on, in order w, as rounds of 32
+  auto rounds = [&](int first, int w) {
+    std::vector<std::vector<int>> r;
+    for (int k : orders[w]) {
+      if (k < first) continue;
+      if (r.empty() || r.back().size() == kLanes) r.emplace_back();
+      r.back().push_back(k);
+    }
+    return r;
+  };
+  auto steps = [&](const std::vector<int>& r) {
     Steps s;
-    for (size_t k = k0; k < std::min(r.size(), k0 + kLanes); ++k) {
-      s.u = std::max(s.u, (int)r[k]->lead.size());
-      s.l = std::max(s.l, half(r[k]->loss.size()));
-      s.p = std::max(s.p, (int)r[k]->prod.size());
+    for (int k : r) {
+      s.u = std::max(s.u, sh[k].u);
+      s.l = std::max(s.l, sh[k].l);
+      s.p = std::max(s.p, sh[k].p);
     }
     s.l = s.l > 1 ? up(s.l, 2) : s.l;
     s.p = s.p > 1 ? up(s.p, 2) : s.p;
     return s;
   };
-  size_t n_neg = 0;
-  while (n_neg < items.size() && !items[n_neg].neg.empty()) ++n_neg;
-  const size_t r_min = (n_neg + 7) / 8;
-  size_t best_r = r_min;
+  int n_neg = 0;
+  while (n_neg < n && !items[n_neg].neg.empty()) ++n_neg;
+  const int r_min = (n_neg + 7) / 8;
+  int best_r = r_min, best_w = 0;
   long best = -1, chains = 0;
-  for (size_t ra = 0; ra * 8 < items.size() + 8; ++ra) {
-    if (ra > 0 && (ra - 1) * 8 < items.size()) {
+  // past the long lists the cost only rises: a few rounds beyond the best end
+  // the search
+  for (int ra = 0; 8 * ra < n + 8 && (best < 0 || ra < best_r + 6); ++ra) {
+    if (ra > 0) {
       long len = 0, bytes = 32 * 8;
-      for (size_t k = 8 * (ra - 1); k < std::min(items.size(), 8 * ra); ++k) {
-        len = std::max(len, (long)up(items[k].longest(), 4));
-        for (int c = 0; c < 4; ++c) bytes += 4 * up((int)items[k].chain(c).size(), 4);
+      for (int k = 8 * (ra - 1); k < std::min(n, 8 * ra); ++k) {
+        len = std::max(len, (long)up(items[k].longest, 4));
+        bytes += 4 * items[k].padded;
       }
       chains += 45 + 11 * len + bytes / bytes_per_inst;
     }
     if (ra < r_min) continue;
-    const auto r = rest(8 * ra);
-    long cost = chains;
-    for (size_t k = 0; k < r.size(); k += kLanes) {
-      const Steps s = steps(r, k);
-      cost += 30 + 9 * (s.u + s.l + s.p) + 128L * (1 + s.u + s.l + s.p) / bytes_per_inst;
-    }
-    if (best < 0 || cost < best) {
-      best = cost;
-      best_r = ra;
+    for (int w = 0; w < 3; ++w) {
+      long cost = chains;
+      for (const auto& r : rounds(8 * ra, w)) {
+        const Steps s = steps(r);
+        cost += 30 + 9 * (s.u + s.l + s.p) + 128L * (1 + s.u + s.l + s.p) / bytes_per_inst;
+      }
+      if (best < 0 || cost < best) {
+        best = cost;
+        best_r = ra;
+        best_w = w;
+      }
     }
   }
-  for (size_t k = 0; k < 8 * best_r; ++k) {
+  for (int k = 0; k < 8 * best_r; ++k) {
     for (int c = 0; c < 4; ++c) {
       std::vector<uint32_t> e;
-      if (k < items.size()) e = items[k].chain(c);
+      if (k < n) e = items[k].chain(c);
       e.resize(up((int)e.size(), 4), zero);
       o->a_rec.push_back((uint32_t)o->a_ent.size() | ((uint32_t)e.size() << 16));
-      o->a_rec.push_back(k < items.size()
-                             ? (uint32_t)items[k].id | ((uint32_t)items[k].tag << 16)
-                             : 0xFFFFu);
+      o->a_rec.push_back(
+          k < n ? (uint32_t)items[k].id | ((uint32_t)items[k].tag << 16) : 0xFFFFu);
       o->a_ent.insert(o->a_ent.end(), e.begin(), e.end());
     }
   }
-  const auto r = rest(8 * best_r);
-  for (size_t k0 = 0; k0 < r.size(); k0 += kLanes) {
-    const Steps s = steps(r, k0);
+  for (const auto& r : rounds(8 * best_r, best_w)) {
+    const Steps s = steps(r);
     o->b_hdr.push_back((uint32_t)s.l | ((uint32_t)s.p << 16));
     o->b_hdr.push_back((uint32_t)s.u);
-    auto at = [&](const std::vector<uint32_t> GatherItem::*list, size_t k, size_t j) {
-      return k < r.size() && j < (r[k]->*list).size() ? (r[k]->*list)[j] : zero;
+    auto at = [&](const std::vector<uint32_t> GatherItem::*list, int k, size_t j) {
+      return k < (int)r.size() && j < (items[r[k]].*list).size() ? (items[r[k]].*list)[j] : zero;
     };
-    for (size_t k = k0; k < k0 + kLanes; ++k)
-      o->b_id.push_back(k < r.size() ? (uint32_t)r[k]->id | ((uint32_t)r[k]->tag << 16) : 0xFFFFu);
+    for (int k = 0; k < kLanes; ++k)
+      o->b_id.push_back(k < (int)r.size() ? (uint32_t)items[r[k]].id |
+                                                ((uint32_t)items[r[k]].tag << 16)
+                                          : 0xFFFFu);
     for (int j = 0; j < s.u; ++j)
-      for (size_t k = k0; k < k0 + kLanes; ++k) o->b_ent.push_back(at(&GatherItem::lead, k, j));
+      for (int k = 0; k < kLanes; ++k) o->b_ent.push_back(at(&GatherItem::lead, k, j));
     for (int j = 0; j < s.l; ++j)
-      for (size_t k = k0; k < k0 + kLanes; ++k)
+      for (int k = 0; k < kLanes; ++k)
         o->b_ent.push_back((at(&GatherItem::loss, k, 2 * j) & 0xFFFFu) |
                            (at(&GatherItem::loss, k, 2 * j + 1) << 16));
     for (int j = 0; j < s.p; ++j)
-      for (size_t k = k0; k < k0 + kLanes; ++k) o->b_ent.push_back(at(&GatherItem::prod, k, j));
+      for (int k = 0; k < kLanes; ++k) o->b_ent.push_back(at(&GatherItem::prod, k, j));
   }
   o->a_ent.resize(o->a_ent.size() + 4, zero);  // read ahead, never used
   o->b_ent.resize(o->b_ent.size() + 2 * kLanes, zero);
@@ -370,8 +392,8 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     jg_lupos[e] = (uint16_t)t.jg_lupos[e];
     jg_row[e] = (uint16_t)t.jg_row[e];
   }
-  // per LU position: the solver-J slot that fills it (+1, 0 = none) and, in
-  // bit 15, whether it is a diagonal (M = I - gamma*J in one pass)
+  // per 32 LU positions: those that a solver-J slot fills, the diagonals, and
+  // the slots before them (M = I - gamma*J in one pass)
   if (t.n_jac >= 32767) {
     *err = "too many Jacobian elements for the table encoding";
     return false;
@@ -383,9 +405,11 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     for (int q = 0, k = 0; q < t.n_lu; ++q)
       if (at[q]) jslot[at[q] - 1] = k++;
   }
-  std::vector<uint16_t> lu_src(t.n_lu, 0);
-  for (int e = 0; e < t.n_jac; ++e) lu_src[t.jg_lupos[e]] = (uint16_t)(jslot[e] + 1);
-  for (int i = 0; i < n; ++i) lu_src[t.lu_diag[i]] |= 0x8000u;
+  std::vector<uint32_t> lu_src(3 * ((t.n_lu + 127) / 128 * 4), 0);
+  for (int e = 0; e < t.n_jac; ++e) lu_src[3 * (t.jg_lupos[e] / 32)] |= 1u << (t.jg_lupos[e] % 32);
+  for (int i = 0; i < n; ++i) lu_src[3 * (t.lu_diag[i] / 32) + 1] |= 1u << (t.lu_diag[i] % 32);
+  for (size_t c = 1; c < lu_src.size() / 3; ++c)
+    lu_src[3 * c + 2] = lu_src[3 * c - 1] + (uint32_t)__builtin_popcount(lu_src[3 * c - 3]);
   std::vector<int> jcsc(t.n_jac);
   for (int e = 0; e < t.n_jac; ++e) jcsc[jslot[e]] = e;
   std::vector<long> jw(t.n_jac);
@@ -443,8 +467,10 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   };
   // Grouped phases as rounds of 32 targets, longest first within a level, so
   // that a round's targets have similar lengths and its padding stays small.
-  // Per round its pair count, 32 records (first pair, target, pivot or finish
-  // mark) and its further pairs.
+  // Targets of four pairs or more take two lanes, one for each of their
+  // alternating sums, 16 to a round.  Per round its pair count per lane | two
+  // lanes<<15, 32 records (first pair, target, pivot or finish mark) and its
+  // further pairs.
   struct Rounds {
     std::vector<uint32_t> pair0, target, recip, ext;
     std::vector<int> cnt, level;
@@ -458,23 +484,29 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
       std::stable_sort(us.begin(), us.end(), [&](int a, int b) {
         return g.unit_count[a] > g.unit_count[b];
       });
-      for (size_t k0 = 0; k0 < us.size(); k0 += kLanes) {
-        auto pair = [&](size_t k, int j) {
-          if (k >= us.size() || j >= g.unit_count[us[k]]) return no_pair;
-          const int p = g.unit_begin[us[k]] + j;
+      for (size_t k0 = 0; k0 < us.size();) {
+        const bool two = g.unit_count[us[k0]] >= 4;
+        auto pair = [&](size_t lane, int j) {
+          const size_t k = k0 + (two ? lane / 2 : lane);
+          const int at = two ? 2 * j + (int)(lane & 1) : j;
+          if (k >= us.size() || at >= g.unit_count[us[k]]) return no_pair;
+          const int p = g.unit_begin[us[k]] + at;
           return (uint32_t)g.pair_a[p] | ((uint32_t)g.pair_b[p] << 16);
         };
-        const int cnt = std::max(1, g.unit_count[us[k0]]);
-        o->cnt.push_back(cnt);
+        const int most = std::max(1, g.unit_count[us[k0]]);
+        const int cnt = two ? (most + 1) / 2 : most;
+        o->cnt.push_back(cnt | (two ? 0x8000 : 0));
         o->level.push_back(l);
-        for (size_t k = k0; k < k0 + kLanes; ++k) {
-          const bool real = k < us.size();
-          o->pair0.push_back(pair(k, 0));
+        for (size_t lane = 0; lane < kLanes; ++lane) {
+          const size_t k = k0 + (two ? lane / 2 : lane);
+          const bool real = k < us.size() && !(two && (lane & 1));
+          o->pair0.push_back(pair(lane, 0));
           o->target.push_back(real ? (uint32_t)g.unit_target[us[k]] : (uint32_t)spare);
           o->recip.push_back(real ? (uint32_t)g.unit_recip[us[k]] : 0u);
         }
         for (int j = 1; j < cnt; ++j)
-          for (size_t k = k0; k < k0 + kLanes; ++k) o->ext.push_back(pair(k, j));
+          for (size_t lane = 0; lane < kLanes; ++lane) o->ext.push_back(pair(lane, j));
+        k0 += two ? kLanes / 2 : kLanes;
       }
     }
   };
@@ -516,19 +548,15 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
       if (t.fb.unit_recip[u] && !has[t.fb.unit_recip[u] - 1])
         e.push_back({t.n_lu, t.fb.unit_recip[u] - 1});
     std::vector<char> stored(n, 0);
-    for (size_t k = 0; k < (e.size() + kLanes - 1) / kLanes * kLanes; ++k) {
-      if (k >= e.size()) {
-        fs_rec.push_back((uint32_t)t.n_lu);
-        fs_rec.push_back(0x7FFFu);
-        continue;
-      }
-      const int piv = e[k].second;
-      fs_rec.push_back((uint32_t)e[k].first | ((uint32_t)t.lu_diag[piv] << 16));
-      fs_rec.push_back((uint32_t)piv | (stored[piv] ? 0u : 0x8000u));
-      stored[piv] = 1;
+    for (const auto& x : e) {
+      fs_rec.push_back((uint32_t)x.first | ((uint32_t)t.lu_diag[x.second] << 16));
+      fs_rec.push_back((uint32_t)x.second | (stored[x.second] ? 0u : 0x8000u));
+      stored[x.second] = 1;
     }
-    fl_hdr[2 * l] = (uint16_t)((e.size() + kLanes - 1) / kLanes);
+    fl_hdr[2 * l] = (uint16_t)(fs_rec.size() / 2);
   }
+  svr.ext.resize(svr.ext.size() + kLanes, sv_none);  // read ahead, never used
+  fbr.ext.resize(fbr.ext.size() + kLanes, lu_none);
   for (size_t k = 0; k < svr.pair0.size(); ++k) {
     sv_rec.push_back(svr.pair0[k]);
     sv_rec.push_back(svr.target[k] | (svr.recip[k] ? 0x8000u : 0u) |
@@ -651,6 +679,90 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     std::vector<int> cv_state;
     for (const SubProgram& g : t.cv) cv_state.push_back(g.state);
     o.sm_state = w.put(u16(cv_state));
+    // parallel parts of the programs (blob.hpp)
+    std::vector<uint32_t> item[5], scr, pel, pst;
+    uint32_t slots = 0;
+    for (size_t c = 0; c < t.cv.size(); ++c) {
+      const std::vector<int>& I = t.cv[c].ints;
+      const uint32_t i0 = rec[2 * c], f0 = rec[2 * c + 1], cc = (uint32_t)c << 8;
+      const uint32_t s0 = slots;
+      if (I[0] == 1) {
+        int ii = 3, fi = 0;
+        for (int x = 0; x < I[2]; ++x) {
+          const int type = I[ii++];
+          if (type == 1) {
+            for (uint32_t v : {1u | cc, i0 + (uint32_t)ii, f0 + (uint32_t)fi, slots})
+              item[1].push_back(v);
+            slots += 7;
+            fi += 3 + I[ii + 2];
+            ii += 6;
+          } else if (type == 2) {
+            fi += 2 + I[ii];
+            ii += 2 + 2 * I[ii];
+          }
+        }
+        for (uint32_t v : {s0, 0u, 0u, 0u}) scr.push_back(v);
+        continue;
+      }
+      const int npair = I[2], x = I[3], ninter = I[4];
+      const int* pr = I.data() + 6;
+      const int* it = pr + 5 * npair;
+      int fi = 2 * npair;
+      for (int k = 0; k < ninter; ++k) {
+        for (uint32_t v : {3u | cc, i0 + 6u + 5u * npair + 2u * k, f0 + (uint32_t)fi, slots})
+          item[3].push_back(v);
+        slots += 3;
+        fi += 2 + it[2 * k + 1];
+      }
+      const uint32_t p0 = slots;
+      for (int j = 0; j < npair; ++j) {
+        for (uint32_t v : {4u | cc, i0 + 6u + 5u * j, f0 + 2u * j, slots}) item[4].push_back(v);
+        slots += 2;
+      }
+      for (uint32_t v : {s0, (uint32_t)ninter, p0, slots}) scr.push_back(v);
+      slots += 2;
+      // every partial of this coefficient with its terms in the order of the
+      // interactions: the direct ones, then those through omega
+      std::vector<int> ids{I[5]};
+      for (int j = 0; j < npair; ++j)
+        for (int a : {pr[5 * j + 3], pr[5 * j + 4]})
+          if (std::find(ids.begin(), ids.end(), a) == ids.end()) ids.push_back(a);
+      for (int id : ids) {
+        pel.push_back((uint32_t)id | ((uint32_t)c << 16));
+        pel.push_back((uint32_t)pst.size() / 2);
+        auto step = [&](uint32_t kind, int k, int j, int q) {
+          pst.push_back(kind | ((uint32_t)k << 4));
+          pst.push_back((uint32_t)j | ((uint32_t)q << 16));
+        };
+        for (int k = 0; k < ninter; ++k) {
+          const int j = it[2 * k];
+          if (j == x) {
+            if (id == I[5]) step(0, k, j, 0);
+            continue;
+          }
+          if (id == pr[5 * j + 3]) step(2, k, j, 0);
+          if (id == pr[5 * j + 4]) step(3, k, j, 0);
+          if (id == I[5]) step(1, k, j, 0);
+          for (int q = 0; q < npair; ++q) {
+            if (q == x) continue;
+            if (id == pr[5 * q + 3]) step(4, k, j, q);
+            if (id == pr[5 * q + 4]) step(5, k, j, q);
+          }
+        }
+      }
+    }
+    o.n_smp = (int)pel.size() / 2;
+    pel.push_back(0);
+    pel.push_back((uint32_t)pst.size() / 2);
+    std::vector<uint32_t> items;
+    for (int kind : {1, 3, 4}) items.insert(items.end(), item[kind].begin(), item[kind].end());
+    o.n_smi = (int)items.size() / 4;
+    o.sm_item = w.put(items);
+    o.sm_scr = w.put(scr);
+    o.sm_pel = w.put(pel);
+    o.sm_pst = w.put(pst);
+    o.n_sms = (int)slots;
+    for (int k = 0; k < 2; ++k) o.scr0[k] = o.g[k].zero + 1 + o.g[k].n_neg;
     o.sm_int = w.put(ints);
     o.sm_flt = w.put(flts);
     o.n_virt = t.n_virt;

@@ -80,8 +80,10 @@ struct SolveArgs {
 // ---------------------------------------------------------------------------
 // Warp helpers
 // ---------------------------------------------------------------------------
+// (one shuffle in a loop: a shuffle of a double is some 25 instructions of
+// code, and the kernel is short of instruction cache)
 __device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
+#pragma unroll 1
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULLMASK, v, o);
   return v;
 }
@@ -149,6 +151,9 @@ __device__ __noinline__ double dpow(double x, double y) { return pow(x, y); }
 __device__ __noinline__ double ddiv(double a, double b) { return a / b; }
 __device__ __noinline__ double dsqrt(double a) { return sqrt(a); }
 
+// step size ratio 1 / (x^(1/k) + ADDON)
+__device__ __noinline__ double step_ratio(double x, int k);
+
 // sqrt(sum of s over the lanes / n) with n a small whole number and rn = 1 / n
 // rounded to nearest: one residual step makes sum * rn the correctly rounded
 // quotient (Markstein, IBM J. Res. Dev. 34, 1990) at a fifth of a division's
@@ -171,6 +176,9 @@ __constant__ double kAlpha0[6] = {
     -1.0, -1.0, -1.0 - 1.0 / 2.0, -1.0 - 1.0 / 2.0 - 1.0 / 3.0,
     -1.0 - 1.0 / 2.0 - 1.0 / 3.0 - 1.0 / 4.0,
     -1.0 - 1.0 / 2.0 - 1.0 / 3.0 - 1.0 / 4.0 - 1.0 / 5.0};
+__device__ __noinline__ double step_ratio(double x, int k) {
+  return ddiv(1.0, dpow(x, kInvInt[k]) + ADDON);
+}
 // above kNoGrowth[k], x^(1/k) + ADDON is certainly above 1 / THRESH, so a step
 // size ratio 1 / (x^(1/k) + ADDON) is below THRESH and leaves the step as it is
 // (0.66667^k; 1 / THRESH - ADDON = 0.6666657)
@@ -320,14 +328,56 @@ __device__ __forceinline__ bool rates_of(const Tab& t, const double* y, const do
 // ---------------------------------------------------------------------------
 // Sub-models: the species they compute, before every f and J
 // ---------------------------------------------------------------------------
+// The programs (SubProgram in model.hpp) are evaluated in turns over the lanes:
+// first every Jacobson pair of ZSR and every interaction and pair of PD-FiTE
+// (their exponentials, polynomials and moles), then the sums, one lane per
+// computed species, then PD-FiTE's partials, one lane per element.  Each sum
+// keeps its terms' order.  With one lane per computed species alone, ZSR and
+// PD-FiTE ran one after the other, 5 of 32 lanes at work (f of the shipped
+// mod37 configuration: 14 600 of its 25 700 cycles; its Jacobian: 38 100 of
+// 70 200).
+//
 // ZSR aerosol water of one phase instance
-// (src/sub_models/sub_model_ZSR_aerosol_water.c:225-305, Jacobian :318-437)
-// from its program (SubProgram in model.hpp); P, when given, receives the
-// partials of the water against the gas-phase water and the ions.  Ion
-// concentrations use the program's reciprocal factors (the reference divides
-// by count, MW and 1000 in turn: equal to rounding).
-__device__ double zsr_water(const int* I, const double* F, const double* y, double ppm,
-                            double* P) {
+// (src/sub_models/sub_model_ZSR_aerosol_water.c:225-305, Jacobian :318-437).
+// Ion concentrations use the program's reciprocal factors (the reference
+// divides by count, MW and 1000 in turn: equal to rounding).
+template <bool PJ>
+__device__ __forceinline__ void zsr_pair(const int* I, const double* F, const double* y,
+                                         double a_w, double ppm, double* s) {
+  // Jacobson et al. (1996)
+  const int ny = I[2];
+  const double low = F[0], fc = F[1], fa = F[2];
+  const double* Y = F + 3;
+  const bool above = a_w > low;
+  const double j_aw = above ? a_w : low;
+  // Y_0 + Y_1 a + ... and its derivative in a, by Horner's rule
+  double mol = 0.0, dm = 0.0;
+  #pragma unroll 1
+  for (int k = ny - 1; k >= 0; --k) {
+    if (PJ) dm = dm * j_aw + mol;
+    mol = mol * j_aw + Y[k];
+  }
+  const double cat = state_of(y[I[0]]) * fc, an = state_of(y[I[1]]) * fa;
+  // smooth minimum of the ion concentrations (smoothing factor -100)
+  const double ec = exp(-100.0 * cat), ea = exp(-100.0 * an);
+  const double inv_e = __drcp_rn(ec + ea);
+  const double conc = (cat * ec + an * ea) * inv_e;
+  const double inv_m2 = __drcp_rn(mol * mol);
+  s[0] = conc * inv_m2;
+  if constexpr (PJ) {
+    const double dcc = (ec * ec + ec * ea * (1.0 + 100.0 * an - 100.0 * cat)) * inv_e * inv_e;
+    const double dca = (ea * ea + ec * ea * (1.0 + 100.0 * cat - 100.0 * an)) * inv_e * inv_e;
+    s[1] = -2.0 * conc * inv_m2 * ddiv(1000.0, mol);
+    s[2] = above ? dm * ppm : 0.0;
+    s[3] = inv_m2 * 1000.0 * dca;
+    s[4] = fa;
+    s[5] = inv_m2 * 1000.0 * dcc;
+    s[6] = fc;
+  }
+}
+template <bool PJ>
+__device__ __forceinline__ double zsr_water(const int* I, const double* F, const double* y,
+                                            double ppm, const double* s, double* P) {
   const double a_w = ppm * state_of(y[I[1]]);
   const int npair = I[2];
   double W = 1.0e-30;  // MINIMUM_WATER_MASS_
@@ -335,36 +385,16 @@ __device__ double zsr_water(const int* I, const double* F, const double* y, doub
   #pragma unroll 1
   for (int x = 0; x < npair; ++x) {
     const int type = I[ii++];
-    if (type == 1) {  // Jacobson et al. (1996)
-      const int ci = I[ii], ai = I[ii + 1], ny = I[ii + 2];
-      const int pg = I[ii + 3], pc = I[ii + 4], pa = I[ii + 5];
+    if (type == 1) {
+      W += s[0] * 1000.0;
+      if constexpr (PJ) {
+        P[I[ii + 3]] += s[1] * s[2];
+        P[I[ii + 5]] += s[3] * s[4];
+        P[I[ii + 4]] += s[5] * s[6];
+      }
+      s += 7;
+      fi += 3 + I[ii + 2];
       ii += 6;
-      const double low = F[fi], fc = F[fi + 1], fa = F[fi + 2];
-      const double* Y = F + fi + 3;
-      fi += 3 + ny;
-      const bool above = a_w > low;
-      const double j_aw = above ? a_w : low;
-      // Y_0 + Y_1 a + ... and its derivative in a, by Horner's rule
-      double mol = 0.0, dm = 0.0;
-      #pragma unroll 1
-      for (int k = ny - 1; k >= 0; --k) {
-        dm = dm * j_aw + mol;
-        mol = mol * j_aw + Y[k];
-      }
-      const double cat = state_of(y[ci]) * fc, an = state_of(y[ai]) * fa;
-      // smooth minimum of the ion concentrations (smoothing factor -100)
-      const double ec = exp(-100.0 * cat), ea = exp(-100.0 * an);
-      const double inv_e = ddiv(1.0, ec + ea);
-      const double conc = (cat * ec + an * ea) * inv_e;
-      const double inv_m2 = ddiv(1.0, mol * mol);
-      W += conc * inv_m2 * 1000.0;
-      if (P) {
-        const double dcc = (ec * ec + ec * ea * (1.0 + 100.0 * an - 100.0 * cat)) * inv_e * inv_e;
-        const double dca = (ea * ea + ec * ea * (1.0 + 100.0 * cat - 100.0 * an)) * inv_e * inv_e;
-        P[pg] += -2.0 * conc * inv_m2 * ddiv(1000.0, mol) * (above ? dm * ppm : 0.0);
-        P[pa] += inv_m2 * 1000.0 * dca * fa;
-        P[pc] += inv_m2 * 1000.0 * dcc * fc;
-      }
     } else if (type == 2) {  // EQSAM (Metzger et al., 2002)
       const int nion = I[ii], pg = I[ii + 1];
       ii += 2;
@@ -372,11 +402,11 @@ __device__ double zsr_water(const int* I, const double* F, const double* y, doub
       fi += 2;
       double e_aw = a_w > 0.99 ? 0.99 : a_w;
       e_aw = e_aw < 0.001 ? 0.001 : e_aw;
-      const double base = pre * (ddiv(1.0, e_aw) - 1.0);
+      const double base = pre * (__drcp_rn(e_aw) - 1.0);
       const double mol = dpow(base, zw);
-      const double inv_mol = ddiv(1.0, mol);
+      const double inv_mol = __drcp_rn(mol);
       double dmol = 0.0;
-      if (P) {
+      if constexpr (PJ) {
         const double de = (a_w > 0.99 || a_w < 0.001) ? 0.0 : ppm;
         dmol = zw * dpow(base, zw - 1.0) * ddiv(-pre, e_aw * e_aw) * de;
       }
@@ -388,7 +418,7 @@ __device__ double zsr_water(const int* I, const double* F, const double* y, doub
         double c = state_of(y[ion]);
         c = c > 0.0 ? c : 0.0;
         W += c * inv_mw * inv_mol;
-        if (P) {
+        if constexpr (PJ) {
           P[pg] += -c * inv_mw * inv_mol * inv_mol * dmol;
           P[pid] += (c > 0.0 ? 1.0 : 0.0) * inv_mw * inv_mol;
         }
@@ -400,104 +430,139 @@ __device__ double zsr_water(const int* I, const double* F, const double* y, doub
 
 // PD-FiTE activity coefficient of one ion pair in one phase instance
 // (src/sub_models/sub_model_PDFiTE.c:167-259, Jacobian :273-432; Topping et
-// al. 2009, eq. 15) from its program; P, when given, receives its partials
-// against the gas-phase water and every ion.  Moles per concentration and
-// the partials' factors are the program's reciprocals; 1 / omega is taken
-// once.
-__device__ double pdfite_gamma(const int* I, const double* F, const double* y, double ppm,
-                               double* P) {
-  double a_w = ppm * state_of(y[I[1]]);
-  a_w = a_w < 0.0 ? 0.0 : (a_w > 1.0 ? 1.0 : a_w);
-  const int npair = I[2], x = I[3], ninter = I[4], pw = I[5];
-  const int* pr = I + 6;              // per pair: cation, anion, stoichiometry, 2 param ids
-  const int* it = pr + 5 * npair;     // per interaction: pair, B count
-  const double* fb = F + 2 * npair;   // per interaction: min RH, max RH, B...
-  auto cn = [&](int j) { return state_of(y[pr[5 * j]]) * F[2 * j]; };
-  auto an = [&](int j) { return state_of(y[pr[5 * j + 1]]) * F[2 * j + 1]; };
+// al. 2009, eq. 15).  Moles per concentration and the partials' factors are the
+// program's reciprocals; 1 / omega is taken once.  si: the interactions' slots,
+// sp: the pairs', sg: gamma and 1 / omega (0: no omega).
+__device__ __forceinline__ double pdfite_gamma(const int* I, const double* si, const double* sp,
+                                               double* sg) {
+  const int npair = I[2], x = I[3], ninter = I[4];
+  const int* pr = I + 6;           // per pair: cation, anion, stoichiometry, 2 param ids
+  const int* it = pr + 5 * npair;  // per interaction: pair, B count
   double omega = 0.0;
   #pragma unroll 1
   for (int j = 0; j < npair; ++j)
-    if (j != x) omega += 2.0 * pr[5 * j + 2] * cn(j) * an(j);
-  const double inv_omega = omega > 0.0 ? ddiv(1.0, omega) : 0.0;
-  auto in_range = [&](double lo, double hi) {
-    return !((a_w <= lo || a_w > hi) && !(a_w <= 0.0 && lo <= 0.0));
-  };
+    if (j != x) omega += 2.0 * pr[5 * j + 2] * sp[2 * j] * sp[2 * j + 1];
+  const double inv_omega = omega > 0.0 ? __drcp_rn(omega) : 0.0;
   double lng = 0.0;
-  int fi = 0;
   #pragma unroll 1
   for (int k = 0; k < ninter; ++k) {
-    const int j = it[2 * k], nb = it[2 * k + 1];
-    const double lo = fb[fi], hi = fb[fi + 1];
-    const double* B = fb + fi + 2;
-    fi += 2 + nb;
-    if (!in_range(lo, hi)) continue;
-    double li = 0.0;
-    #pragma unroll 1
-    for (int z = nb - 1; z >= 0; --z) li = li * a_w + B[z];
+    const int j = it[2 * k];
+    const double li = si[3 * k];
+    if (si[3 * k + 2] == 0.0) continue;
     if (j == x)
       lng += li;
     else if (omega > 0.0)
-      lng += li * cn(j) * an(j) * inv_omega;
+      lng += li * sp[2 * j] * sp[2 * j + 1] * inv_omega;
   }
   const double g = exp(lng);
-  if (P) {
-    fi = 0;
-    #pragma unroll 1
-    for (int k = 0; k < ninter; ++k) {
-      const int j = it[2 * k], nb = it[2 * k + 1];
-      const double lo = fb[fi], hi = fb[fi + 1];
-      const double* B = fb + fi + 2;
-      fi += 2 + nb;
-      if (!in_range(lo, hi)) continue;
-      double li = 0.0, dli = 0.0;
-      #pragma unroll 1
-      for (int z = nb - 1; z >= 0; --z) {
-        dli = dli * a_w + li;
-        li = li * a_w + B[z];
-      }
-      dli *= ppm;
-      if (j == x) {
-        P[pw] += g * dli;
-      } else if (omega > 0.0) {
-        const double cj = cn(j), aj = an(j);
-        P[pr[5 * j + 3]] += g * li * aj * F[2 * j] * inv_omega;
-        P[pr[5 * j + 4]] += g * li * cj * F[2 * j + 1] * inv_omega;
-        P[pw] += g * cj * aj * inv_omega * dli;
-        const double s = -g * li * cj * aj * inv_omega * inv_omega * 2.0;
-        #pragma unroll 1
-        for (int q = 0; q < npair; ++q) {
-          if (q == x) continue;
-          const double sq = s * pr[5 * q + 2];
-          P[pr[5 * q + 3]] += sq * an(q) * F[2 * q];
-          P[pr[5 * q + 4]] += sq * cn(q) * F[2 * q + 1];
-        }
-      }
-    }
-  }
+  sg[0] = g;
+  sg[1] = omega > 0.0 ? inv_omega : -1.0;
   return g;
 }
 
-// Every computed species, one lane each, into cv; with P, also the
-// parameter Jacobian (P zeroed first; element ids index it)
-__device__ __noinline__ void sub_model_eval(const char* tb, const double* y, const double* keff,
-                                            double* cv, double* P, int lane) {
+// Every computed species into cv, with scr the programs' scratch; PJ: also the
+// parameter Jacobian P (zeroed first; element ids index it)
+template <bool PJ>
+__device__ __noinline__ void sub_model_eval(const double* y, const double* keff, double* cv,
+                                            double* P, double* scr, int lane) {
+  y = sh(y);
+  keff = sh(keff);
+  cv = sh(cv);
+  scr = sh(scr);
+  const char* const tb = g_smem;
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
-  if (P) {
+  if constexpr (PJ) {
+    P = sh(P);
     #pragma unroll 1
     for (int i = lane; i < o.n_pj; i += 32) P[i] = 0.0;
-    __syncwarp();
   }
   const uint32_t* rec = (const uint32_t*)(tb + o.sm_rec);
   const int* I0 = (const int*)(tb + o.sm_int);
   const double* F0 = (const double*)(tb + o.sm_flt);
   const double ppm = keff[o.sm_keff];
+  const uint4* item = (const uint4*)(tb + o.sm_item);
+  #pragma unroll 1
+  for (int e = lane; e < o.n_smi; e += 32) {
+    const uint4 w = item[e];
+    const int* I = I0 + w.y;
+    const double* F = F0 + w.z;
+    double* s = scr + w.w;
+    const int kind = w.x & 0xFFu;
+    if (kind == 4) {
+      s[0] = state_of(y[I[0]]) * F[0];
+      s[1] = state_of(y[I[1]]) * F[1];
+      continue;
+    }
+    double a_w = ppm * state_of(y[I0[rec[2 * (w.x >> 8)] + 1]]);
+    if (kind == 1) {
+      zsr_pair<PJ>(I, F, y, a_w, ppm, s);
+      continue;
+    }
+    a_w = a_w < 0.0 ? 0.0 : (a_w > 1.0 ? 1.0 : a_w);
+    const double lo = F[0], hi = F[1];
+    const bool in = !((a_w <= lo || a_w > hi) && !(a_w <= 0.0 && lo <= 0.0));
+    double li = 0.0, dli = 0.0;
+    #pragma unroll 1
+    for (int z = I[1] - 1; z >= 0; --z) {
+      if (PJ) dli = dli * a_w + li;
+      li = li * a_w + F[2 + z];
+    }
+    s[0] = li;
+    if (PJ) s[1] = dli * ppm;
+    s[2] = in ? 1.0 : 0.0;
+  }
+  __syncwarp();
+  const uint4* sc = (const uint4*)(tb + o.sm_scr);
   #pragma unroll 1
   for (int c = lane; c < o.n_cv; c += 32) {
     const int* I = I0 + rec[2 * c];
-    const double* F = F0 + rec[2 * c + 1];
-    cv[c] = I[0] == 1 ? zsr_water(I, F, y, ppm, P) : pdfite_gamma(I, F, y, ppm, P);
+    const uint4 q = sc[c];
+    cv[c] = I[0] == 1 ? zsr_water<PJ>(I, F0 + rec[2 * c + 1], y, ppm, scr + q.x, P)
+                      : pdfite_gamma(I, scr + q.x, scr + q.z, scr + q.w);
   }
   __syncwarp();
+  if constexpr (PJ) {
+    const uint2* pel = (const uint2*)(tb + o.sm_pel);
+    const uint2* pst = (const uint2*)(tb + o.sm_pst);
+    #pragma unroll 1
+    for (int e = lane; e < o.n_smp; e += 32) {
+      const uint2 w = pel[e];
+      const int c = w.x >> 16, end = pel[e + 1].y;
+      const uint4 q = sc[c];
+      const int* pr = I0 + rec[2 * c] + 6;
+      const double* F = F0 + rec[2 * c + 1];
+      const double *si = scr + q.x, *sp = scr + q.z;
+      const double g = scr[q.w], io = scr[q.w + 1];
+      double v = 0.0;
+      #pragma unroll 1
+      for (int n = w.y; n < end; ++n) {
+        const uint2 st = pst[n];
+        const int kind = st.x & 0xFu, k = st.x >> 4;
+        if (si[3 * k + 2] == 0.0) continue;
+        const double li = si[3 * k], dli = si[3 * k + 1];
+        if (kind == 0) {
+          v += g * dli;
+          continue;
+        }
+        if (io < 0.0) continue;  // no omega
+        const int j = st.y & 0xFFFFu, r = st.y >> 16;
+        const double cj = sp[2 * j], aj = sp[2 * j + 1];
+        if (kind == 1) {
+          v += g * cj * aj * io * dli;
+        } else if (kind == 2) {
+          v += g * li * aj * F[2 * j] * io;
+        } else if (kind == 3) {
+          v += g * li * cj * F[2 * j + 1] * io;
+        } else {
+          const double s = -g * li * cj * aj * io * io * 2.0;
+          const double sq = s * pr[5 * r + 2];
+          v += sq * sp[2 * r + (kind == 4 ? 1 : 0)] * F[2 * r + (kind == 4 ? 0 : 1)];
+        }
+      }
+      P[w.x & 0xFFFFu] += v;
+    }
+    __syncwarp();
+  }
 }
 
 // SIMPOL phase transfer, one lane per instance
@@ -544,7 +609,11 @@ __device__ __forceinline__ SimpolState simpol_state(const Tab& t, int k, const d
 // negative
 __device__ __noinline__ bool simpol_rates(const char* tb, const double* y, const double* keff,
                                           const double* cv, double* rates, int lane) {
-  const Tab t = make_tab(tb);
+  y = sh(y);
+  keff = sh(keff);
+  cv = sh(cv);
+  rates = sh(rates);
+  const Tab t = make_tab(g_smem);
   bool neg = false;
   #pragma unroll 1
   for (int k = lane; k < t.n_simpol; k += 32) {
@@ -566,7 +635,11 @@ __device__ __noinline__ bool simpol_rates(const char* tb, const double* y, const
 // rows against that water (src/rxns/rxn_HL_phase_transfer.c:383-404)
 __device__ __noinline__ void simpol_partials(const char* tb, const double* y, const double* keff,
                                              const double* cv, double* part, int lane) {
-  const Tab t = make_tab(tb);
+  y = sh(y);
+  keff = sh(keff);
+  cv = sh(cv);
+  part = sh(part);
+  const Tab t = make_tab(g_smem);
   #pragma unroll 1
   for (int k = lane; k < t.n_simpol; k += 32) {
     const uint16_t* rec = t.si_rec + 8 * k;
@@ -586,7 +659,7 @@ __device__ __noinline__ void simpol_partials(const char* tb, const double* y, co
     // d evap / d mass = -evap / m, d evap / d MW = evap / MW = evap mol / m
     const double dedm = -ddiv(s.evap, s.m);
     const double dedw = dedm * -s.mol;
-    const double inv_mol2 = ddiv(1.0, s.mol * s.mol);
+    const double inv_mol2 = __drcp_rn(s.mol * s.mol);
     const int e0 = rec[3], nd = rec[2];
     #pragma unroll 1
     for (int j = 0; j < nd; ++j) {
@@ -658,7 +731,11 @@ __device__ __forceinline__ void aq_fr(const Tab& t, const uint16_t* rec, const d
 // whether any is negative
 __device__ __noinline__ bool aq_rates(const char* tb, const double* y, const double* keff,
                                       const double* cv, double* rates, int lane) {
-  const Tab t = make_tab(tb);
+  y = sh(y);
+  keff = sh(keff);
+  cv = sh(cv);
+  rates = sh(rates);
+  const Tab t = make_tab(g_smem);
   bool neg = false;
   #pragma unroll 1
   for (int q = lane; q < t.n_aq; q += 32) {
@@ -686,7 +763,11 @@ __device__ __noinline__ bool aq_rates(const char* tb, const double* y, const dou
 // (src/rxns/rxn_aqueous_equilibrium.c:486-537).
 __device__ __noinline__ void aq_partials(const char* tb, const double* y, const double* keff,
                                          const double* cv, double* part, int lane) {
-  const Tab t = make_tab(tb);
+  y = sh(y);
+  keff = sh(keff);
+  cv = sh(cv);
+  part = sh(part);
+  const Tab t = make_tab(g_smem);
   #pragma unroll 1
   for (int q = lane; q < t.n_aq; q += 32) {
     const uint16_t* rec = t.aq_rec + 12 * q;
@@ -922,8 +1003,12 @@ __device__ __noinline__ void gather(int k, const double* src, double* out, doubl
         s += v3;
       }
       __syncwarp();
-      s += __shfl_xor_sync(FULLMASK, s, 1);  // L0 + L1, P0 + P1
-      const double P = __shfl_xor_sync(FULLMASK, s, 2);
+      double P = 0.0;
+      #pragma unroll 1
+      for (int m = 1; m < 4; m <<= 1) {  // L0 + L1 and P0 + P1, then P beside L
+        P = __shfl_xor_sync(FULLMASK, s, m);
+        s += m == 1 ? P : 0.0;
+      }
       const int id = w.y & 0xFFFFu;
       if (id != 0xFFFF && (lane & 3) == 0) put(id, w.y >> 16, P, s);
     }
@@ -1217,7 +1302,7 @@ __device__ __noinline__ int dev_f_aero(const char* tb, const double* y, double h
                                        double* rl = nullptr) {
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
   double* cv = rates + o.n_rates;
-  if (o.n_cv > 0) sub_model_eval(tb, y, keff, cv, nullptr, lane);
+  if (o.n_cv > 0) sub_model_eval<false>(y, keff, cv, nullptr, rates + o.scr0[0], lane);
   const bool neg = aero_rates(tb, y, keff, cv, rates, lane);
   return dev_f<LT, EV>(tb, y, h, keff, rates, fscr, out, lane, flags | (neg ? kNegRate : 0), rp,
                        rl);
@@ -1231,7 +1316,7 @@ __device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double
   double* cv = part + o.n_part_all;
   double* P = cv + o.n_cv;
   double* V = P + o.n_pj;
-  if (o.n_cv > 0) sub_model_eval(tb, y, keff, cv, P, lane);
+  if (o.n_cv > 0) sub_model_eval<true>(y, keff, cv, P, part + o.scr0[1], lane);
   aero_partials(tb, y, keff, cv, part, lane);
   const int r = dev_jac<JT, EV>(tb, y, h, keff, part, Jout, lane, flags, csc, jp, jl);
   if (r != 0 || o.n_chain == 0) return r;
@@ -1254,7 +1339,8 @@ __device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double
     double s = (double)Jout[at], sp = 0.0, sl = 0.0;
     #pragma unroll 1
     for (int e = cptr[g]; e < cptr[g + 1]; ++e) {
-      const double v = V[ent[e] & 0xFFFFu] * P[ent[e] >> 16];
+      // rounded by itself: it also goes to the split parts
+      const double v = __dmul_rn(V[ent[e] & 0xFFFFu], P[ent[e] >> 16]);
       s += v;
       sp += v > 0.0 ? v : 0.0;
       sl += v < 0.0 ? -v : 0.0;
@@ -1276,6 +1362,38 @@ __device__ __forceinline__ bool has_simpol(const char* tb) {
 // ---------------------------------------------------------------------------
 // LU of M = I - gamma*J on the fixed order, and the triangular solves
 // ---------------------------------------------------------------------------
+// The further pairs of a round's target (count c, as in its record): two lanes
+// with one of the alternating sums each (the even lane ends with the target, the
+// odd one with the spare slot's zero), or up to two more pairs in one lane.
+template <typename LT>
+__device__ __forceinline__ LT more_pairs(LT s, uint32_t c, const LT* LU, const LT* x,
+                                         const uint32_t** ext, int lane) {
+  const uint32_t* e = *ext;
+  if (c & 0x8000u) {
+    uint32_t q = *e;
+    #pragma unroll 1
+    for (int k = c & 0x7FFFu; k > 1; --k) {
+      e += 32;
+      const LT a = LU[q & 0xFFFFu], b = x[q >> 16];
+      q = *e;
+      s -= a * b;
+    }
+    s += __shfl_xor_sync(FULLMASK, s, 1);
+    if (lane & 1) s = (LT)0;
+  } else {
+    LT s1 = (LT)0;
+    s1 -= LU[e[0] & 0xFFFFu] * x[e[0] >> 16];
+    if (c > 2) {
+      s -= LU[e[32] & 0xFFFFu] * x[e[32] >> 16];
+      e += 32;
+    }
+    e += 32;
+    s += s1;
+  }
+  *ext = e;
+  return s;
+}
+
 __device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
 __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
 
@@ -1298,71 +1416,62 @@ __device__ __noinline__ bool dev_form_factor(const char* tb, const LT* J, double
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
   const int n_lu = o.n_lu;
   {
-    const uint16_t* lu_src = (const uint16_t*)(tb + o.lu_src);
+    const uint32_t* m = (const uint32_t*)(tb + o.lu_src);
+    const uint32_t below = (1u << lane) - 1u;
     #pragma unroll 1
-    for (int q = lane; q < n_lu; q += 128) {
-      uint32_t src[4];
+    for (int q = lane; q < n_lu; q += 128, m += 12) {
       LT v[4];
+      uint32_t has[4], at[4];
       #pragma unroll
-      for (int k = 0; k < 4; ++k) src[k] = q + 32 * k < n_lu ? lu_src[q + 32 * k] : 0u;
+      for (int k = 0; k < 4; ++k) {
+        has[k] = q + 32 * k < n_lu ? m[3 * k] : 0u;
+        at[k] = (has[k] >> lane & 1u) ? m[3 * k + 2] + __popc(has[k] & below) : 0u;
+      }
       #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = (src[k] & 0x7FFFu) ? J[(src[k] & 0x7FFFu) - 1] : (LT)0;
+      for (int k = 0; k < 4; ++k) v[k] = J[at[k]];
       #pragma unroll
       for (int k = 0; k < 4; ++k)
         if (q + 32 * k < n_lu) {
-          LT m = (src[k] & 0x7FFFu) ? (LT)(-gamma * (double)v[k]) : (LT)0;
-          if (src[k] & 0x8000u) m += (LT)1;
-          LU[q + 32 * k] = m;
+          LT e = (has[k] >> lane & 1u) ? (LT)(-gamma * (double)v[k]) : (LT)0;
+          if (m[3 * k + 1] >> lane & 1u) e += (LT)1;
+          LU[q + 32 * k] = e;
         }
     }
   }
   const ushort2* hdr = (const ushort2*)(tb + o.fl_hdr);
-  const uint2* fs = (const uint2*)(tb + o.fs_rec) + lane;
+  const uint2* fs = (const uint2*)(tb + o.fs_rec);
   const uint2* rec = (const uint2*)(tb + o.fb_rec) + lane;
   const uint32_t* ext = (const uint32_t*)(tb + o.fb_ext) + lane;
   uint2 w = rec[0], wn = rec[32];
   rec += 64;
   bool bad = false;
+  int f0 = 0;
   __syncwarp();
   #pragma unroll 1
   for (int lv = o.n_plev; lv > 0; --lv) {
     const ushort2 hd = *hdr++;
     #pragma unroll 1
-    for (int c = hd.x; c > 0; --c, fs += 32) {
-      const uint2 f = *fs;
-      const int piv = f.y & 0x7FFFu, pos = f.x & 0xFFFFu;
-      if (piv != 0x7FFF) {
-        const LT p = LU[f.x >> 16], v = LU[pos];
-        const bool pbad = p == (LT)0 || !isfinite(p);
-        bad |= pbad;
-        const LT d = pbad ? (LT)0 : rcp_rn(p);
-        if (pos != n_lu) LU[pos] = v * d;
-        if (f.y & 0x8000u) dinv[piv] = d;
-      }
+    for (int e = f0 + lane; e < hd.x; e += 32) {
+      const uint2 f = fs[e];
+      const int pos = f.x & 0xFFFFu;
+      const LT p = LU[f.x >> 16], v = LU[pos];
+      const bool pbad = p == (LT)0 || !isfinite(p);
+      bad |= pbad;
+      const LT d = pbad ? (LT)0 : rcp_rn(p);
+      if (pos != n_lu) LU[pos] = v * d;
+      if (f.y & 0x8000u) dinv[f.y & 0x7FFFu] = d;
     }
+    f0 = hd.x;
     __syncwarp();
     #pragma unroll 1
     for (int r = hd.y; r > 0; --r) {
       const int tgt = w.y & 0xFFFFu;
       LT s = LU[tgt] - LU[w.x & 0xFFFFu] * LU[w.x >> 16];
-      int c = w.y >> 16;
+      const uint32_t c = w.y >> 16;
       w = wn;
       wn = *rec;
       rec += 32;
-      if (c > 1) {
-        LT s1 = (LT)0;
-        #pragma unroll 1
-        for (; c > 2; c -= 2, ext += 64) {
-          const uint32_t q0 = ext[0], q1 = ext[32];
-          s1 -= LU[q0 & 0xFFFFu] * LU[q0 >> 16];
-          s -= LU[q1 & 0xFFFFu] * LU[q1 >> 16];
-        }
-        if (c > 1) {
-          s1 -= LU[ext[0] & 0xFFFFu] * LU[ext[0] >> 16];
-          ext += 32;
-        }
-        s += s1;
-      }
+      if (c > 1) s = more_pairs(s, c, LU, LU, &ext, lane);
       LU[tgt] = s;
     }
     __syncwarp();
@@ -1405,22 +1514,8 @@ __device__ __noinline__ void dev_lsolve(const LT* LU, const LT* dinv, LT* z, int
     const int tgt = w.y & 0x7FFFu;
     LT s = z[tgt] - a * z[w.x >> 16];
     a = LU[wn.x & 0xFFFFu];
-    int c = w.y >> 16;
-    if (c > 1) {
-      // further pairs into alternating sums
-      LT s1 = (LT)0;
-      #pragma unroll 1
-      for (; c > 2; c -= 2, ext += 64) {
-        const uint32_t q0 = ext[0], q1 = ext[32];
-        s1 -= LU[q0 & 0xFFFFu] * z[q0 >> 16];
-        s -= LU[q1 & 0xFFFFu] * z[q1 >> 16];
-      }
-      if (c > 1) {
-        s1 -= LU[ext[0] & 0xFFFFu] * z[ext[0] >> 16];
-        ext += 32;
-      }
-      s += s1;
-    }
+    const uint32_t c = w.y >> 16;
+    if (c > 1) s = more_pairs(s, c, LU, z, &ext, lane);
     z[tgt] = s * d;
     d = (wn.y & 0x8000u) ? dinv[wn.y & 0x7FFFu] : (LT)1;
     __syncwarp();
@@ -1542,11 +1637,8 @@ __device__ __noinline__ double vec_wrms(const double* v, const double* ewt, int 
 }
 // zn <- zn * Pascal(q) (sign +1) or its inverse (sign -1), one element's
 // q+1 history values at a time in registers: for k = 1..q, j = q..k,
-// zn[j-1] += sign * zn[j].  With acor (a prediction) also the first Newton
-// iterate, see vec_start.
-__device__ __noinline__ int hist_pascal(double* zb, int n, int q, double sign, double* acor,
-                                        double* y, int lane) {
-  int flags = 0;
+// zn[j-1] += sign * zn[j]
+__device__ __noinline__ void hist_pascal(double* zb, int n, int q, double sign, int lane) {
   #pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     double v[LMAX];
@@ -1560,15 +1652,8 @@ __device__ __noinline__ int hist_pascal(double* zb, int n, int q, double sign, d
 #pragma unroll
     for (int j = 0; j < QMAX; ++j)
       if (j < q) zb[j * n + i] = v[j];
-    if (acor) {
-      const double a = v[0] < 0.0 ? -v[0] : 0.0, s = v[0] + a;
-      sh(acor)[i] = a;
-      sh(y)[i] = s;
-      flags |= (a != 0.0 ? kProjected : 0) | (s >= 0.0 ? 0 : kOdd);
-    }
   }
   __syncwarp();
-  return flags;
 }
 // zn[j] *= eta^j, j = 1..q
 __device__ __noinline__ void hist_rescale(double* zb, int n, int q, double eta, int lane) {
@@ -1725,11 +1810,12 @@ struct Cell {
   }
   __device__ int predict() {
     tn += h;
-    return hist_pascal(zb, n, q, 1.0, acor, y, lane);
+    hist_pascal(zb, n, q, 1.0, lane);
+    return vec_start(zb, acor, y, n, lane);
   }
   __device__ void restore(double saved_t) {
     tn = saved_t;
-    hist_pascal(zb, n, q, -1.0, nullptr, nullptr, lane);
+    hist_pascal(zb, n, q, -1.0, lane);
   }
   // one value per lane (the first eight) into quot, for every lane to read
   __device__ void share(double v) {
@@ -2005,7 +2091,7 @@ struct Cell {
     if (*nef == maxnef) return ERR_FAILURE;
     etamax = 1.0;
     if (*nef <= MXNEF1) {
-      eta = ddiv(1.0, dpow(BIAS2 * *dsm, kInvInt[L]) + ADDON);
+      eta = step_ratio(BIAS2 * *dsm, L);
       eta = fmax(ETAMIN, eta);
       if (*nef >= SMALL_NEF) eta = fmin(eta, ETAMXF);
       rescale();
@@ -2080,8 +2166,7 @@ struct Cell {
     const bool no_q = BIAS2 * dsm > kNoGrowth[L];
     if (qwait != 0) {
       qprime = q;
-      eta = no_q ? 1.0
-                 : ddiv(1.0, dpow(BIAS2 * dsm, kInvInt[L]) + ADDON);
+      eta = no_q ? 1.0 : step_ratio(BIAS2 * dsm, L);
       set_eta();
       return;
     }
@@ -2107,10 +2192,10 @@ struct Cell {
       set_eta();
       return;
     }
-    const double etaq = ddiv(1.0, dpow(BIAS2 * dsm, kInvInt[L]) + ADDON);
+    const double etaq = step_ratio(BIAS2 * dsm, L);
     double etaqm1 = 0.0, etaqp1 = 0.0;
-    if (q > 1) etaqm1 = ddiv(1.0, dpow(BIAS1 * ddn, kInvInt[q]) + ADDON);
-    if (up) etaqp1 = ddiv(1.0, dpow(BIAS3 * dup, kInvInt[L + 1]) + ADDON);
+    if (q > 1) etaqm1 = step_ratio(BIAS1 * ddn, q);
+    if (up) etaqp1 = step_ratio(BIAS3 * dup, L + 1);
     double etam = fmax(etaqm1, fmax(etaq, etaqp1));
     if (etam < THRESH) {
       eta = 1.0;
@@ -2319,7 +2404,7 @@ __global__ void __launch_bounds__(32 * (AERO ? kMaxCellsAero : kMaxCellsPerBlock
         if (o.n_cv > 0) {
           __syncwarp();
           double* cv = c.rates + o.n_rates;
-          sub_model_eval(smem, c.y, c.keff, cv, nullptr, lane);
+          sub_model_eval<false>(c.y, c.keff, cv, nullptr, c.rates + o.scr0[0], lane);
           const uint16_t* cs = (const uint16_t*)(smem + o.sm_state);
           #pragma unroll 1
           for (int k = lane; k < o.n_cv; k += 32) st[cs[k]] = cv[k];
@@ -3067,11 +3152,15 @@ static Layout make_layout(const BlobOff& o, int lt_size, bool with_hist,
   L.tempv = with_tempv ? take(vec) : -1;
   // the f scratch (pseudo-rates, then the computed species, a zero and the guarded terms) and
   // the J scratch (partials, computed species, parameter partials, virtual
-  // slots, a zero and the guarded terms); the solves' vector lies over them
-  const int n_scr = std::max(o.g[0].zero + 1 + o.g[0].n_neg, o.g[1].zero + 1 + o.g[1].n_neg);
+  // slots, a zero and the guarded terms), each followed by the sub-models'
+  // scratch; the solves' vector lies over them
+  const int n_scr = std::max(o.scr0[0], o.scr0[1]) + o.n_sms;
   L.rates = L.z = take(std::max(sizeof(double) * n_scr, (size_t)lt_size * (o.n + 1)));
   L.keff = take(sizeof(double) * o.n_keff);
-  L.fscr = take(sizeof(double) * 2 * std::max(1, o.n_fscratch));
+  // the split species' parts lie behind f's terms, over J's where those leave room
+  const int f_end = o.scr0[0] + o.n_sms, n_fscr = 2 * std::max(1, o.n_fscratch);
+  L.fscr = f_end + n_fscr <= n_scr ? L.rates + (int)sizeof(double) * f_end
+                                   : take(sizeof(double) * n_fscr);
   // a spare slot: see clear_spare
   L.lu = take((size_t)lt_size * (o.n_lu + 1));
   L.dinv = take((size_t)lt_size * o.n);
