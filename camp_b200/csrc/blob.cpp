@@ -80,7 +80,7 @@ struct GatherTables {
 // lists (9 a word, 30 besides) and their padded words; with the longest chains
 // first, the number of chain rounds and the order of the rest with the least
 // sum are taken, `bytes_per_inst` table bytes counting as one instruction.
-void pack_gather(std::vector<GatherItem> items, uint32_t zero, int bytes_per_inst,
+void pack_gather(std::vector<GatherItem>& items, uint32_t zero, int bytes_per_inst,
                  GatherTables* o) {
   auto half = [](size_t n) { return (int)(n + 1) / 2; };
   auto up = [](int n, int m) { return (n + m - 1) / m * m; };
@@ -146,10 +146,23 @@ void pack_gather(std::vector<GatherItem> items, uint32_t zero, int bytes_per_ins
     if (ra < r_min) continue;
     for (int w = 0; w < 3; ++w) {
       long cost = chains;
-      for (const auto& r : rounds(8 * ra, w)) {
-        const Steps s = steps(r);
+      Steps s;
+      int in_round = 0;
+      auto close = [&]() {
+        s.l = s.l > 1 ? up(s.l, 2) : s.l;
+        s.p = s.p > 1 ? up(s.p, 2) : s.p;
         cost += 30 + 9 * (s.u + s.l + s.p) + 128L * (1 + s.u + s.l + s.p) / bytes_per_inst;
+        s = Steps{};
+        in_round = 0;
+      };
+      for (int k : orders[w]) {
+        if (k < 8 * ra) continue;
+        s.u = std::max(s.u, sh[k].u);
+        s.l = std::max(s.l, sh[k].l);
+        s.p = std::max(s.p, sh[k].p);
+        if (++in_round == kLanes) close();
       }
+      if (in_round) close();
       if (best < 0 || cost < best) {
         best = cost;
         best_r = ra;
@@ -325,7 +338,7 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
         fgt.neg.push_back((uint32_t)x.sp);
         it.neg.push_back((uint32_t)(f_zero + (int)fgt.neg.size() / 2) | one);
       }
-      items.push_back(it);
+      items.push_back(std::move(it));
     }
     pack_gather(items, (uint32_t)f_zero, 16, &fgt);
   }
@@ -434,6 +447,7 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   GatherTables jgt;
   {
     std::vector<GatherItem> items;
+    items.reserve(t.n_jac);
     for (int e = 0; e < t.n_jac; ++e) {
       GatherItem it;
       it.id = jslot[e];
@@ -450,7 +464,7 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
         jgt.neg.push_back((uint32_t)(jg_w1[g] - 1) | ((uint32_t)t.jg_row[e] << 16));
         it.prod.push_back((uint32_t)(j_zero + (int)jgt.neg.size() / 2) | one);
       }
-      items.push_back(it);
+      items.push_back(std::move(it));
     }
     pack_gather(items, (uint32_t)j_zero, 8, &jgt);
   }
