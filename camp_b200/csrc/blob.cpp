@@ -44,19 +44,29 @@ std::vector<std::vector<int>> lpt(const std::vector<long>& weight) {
 }
 
 // One item of the f or J gather: index | coef<<16 entries of its sums (a loss
-// or an unguarded product carries the coefficient 1)
+// or an unguarded product carries the coefficient 1), which lie one after the
+// other in a vector shared by all items: a vector per list made up half of the
+// time that packing takes
+struct GatherList {
+  const uint32_t* p = nullptr;
+  size_t n = 0;
+  size_t size() const { return n; }
+  bool empty() const { return n == 0; }
+  uint32_t operator[](size_t k) const { return p[k]; }
+};
+
 struct GatherItem {
   int id = 0, tag = 0xFFFF;
-  std::vector<uint32_t> lead, loss, prod;
-  std::vector<uint32_t> neg;  // f: guarded losses, after the others into L1
+  GatherList lead, loss, prod;
+  GatherList neg;  // f: guarded losses, after the others into L1
   // the four chains: losses alternate between L0 and L1, products between P0,
   // which starts with the unguarded ones, and P1
   std::vector<uint32_t> chain(int c) const {
     std::vector<uint32_t> o;
-    const std::vector<uint32_t>& v = c < 2 ? loss : prod;
-    if (c == 2) o = lead;
+    const GatherList& v = c < 2 ? loss : prod;
+    if (c == 2) o.assign(lead.p, lead.p + lead.n);
     for (size_t k = c & 1; k < v.size(); k += 2) o.push_back(v[k]);
-    if (c == 1) o.insert(o.end(), neg.begin(), neg.end());
+    if (c == 1) o.insert(o.end(), neg.p, neg.p + neg.n);
     return o;
   }
   int longest = 0, padded = 0;  // longest chain; entries in multiples of four
@@ -127,6 +137,15 @@ void pack_gather(std::vector<GatherItem>& items, uint32_t zero, int bytes_per_in
     s.p = s.p > 1 ? up(s.p, 2) : s.p;
     return s;
   };
+  // the same orders with the lengths beside the items, for the search
+  struct Shape {
+    int item, u, l, p;
+  };
+  std::vector<Shape> shapes[3];
+  for (int w = 0; w < 3; ++w) {
+    shapes[w].reserve(n);
+    for (int k : orders[w]) shapes[w].push_back({k, sh[k].u, sh[k].l, sh[k].p});
+  }
   int n_neg = 0;
   while (n_neg < n && !items[n_neg].neg.empty()) ++n_neg;
   const int r_min = (n_neg + 7) / 8;
@@ -155,12 +174,14 @@ void pack_gather(std::vector<GatherItem>& items, uint32_t zero, int bytes_per_in
         s = Steps{};
         in_round = 0;
       };
-      for (int k : orders[w]) {
-        if (k < 8 * ra) continue;
-        s.u = std::max(s.u, sh[k].u);
-        s.l = std::max(s.l, sh[k].l);
-        s.p = std::max(s.p, sh[k].p);
-        if (++in_round == kLanes) close();
+      for (const Shape& x : shapes[w]) {
+        if (x.item < 8 * ra) continue;
+        s.u = std::max(s.u, x.u);
+        s.l = std::max(s.l, x.l);
+        s.p = std::max(s.p, x.p);
+        if (++in_round < kLanes) continue;
+        close();
+        if (best >= 0 && cost >= best) break;
       }
       if (in_round) close();
       if (best < 0 || cost < best) {
@@ -185,7 +206,7 @@ void pack_gather(std::vector<GatherItem>& items, uint32_t zero, int bytes_per_in
     const Steps s = steps(r);
     o->b_hdr.push_back((uint32_t)s.l | ((uint32_t)s.p << 16));
     o->b_hdr.push_back((uint32_t)s.u);
-    auto at = [&](const std::vector<uint32_t> GatherItem::*list, int k, size_t j) {
+    auto at = [&](const GatherList GatherItem::*list, int k, size_t j) {
       return k < (int)r.size() && j < (items[r[k]].*list).size() ? (items[r[k]].*list)[j] : zero;
     };
     for (int k = 0; k < kLanes; ++k)
@@ -324,21 +345,31 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   const int f_zero = t.n_rates + t.n_cv;
   GatherTables fgt;
   {
+    std::vector<uint32_t> ent;  // the items' lists: never more than reserved
+    ent.reserve(fg_ent.size());
+    auto list = [&](size_t from) { return GatherList{ent.data() + from, ent.size() - from}; };
     std::vector<GatherItem> items;
+    items.reserve(units.size());
     for (const Unit& x : units) {
       const int m1 = clampi(grp_end[2 * x.sp], x.b, x.e);
       const int m2 = clampi(grp_end[2 * x.sp + 1], x.b, x.e);
       GatherItem it;
       it.id = x.sp;
       it.tag = x.slot;
-      for (int k = x.b; k < m1; ++k) it.loss.push_back((fg_ent[k] & 0xFFFFu) | one);
-      for (int k = m1; k < m2; ++k) it.prod.push_back(fg_ent[k] & 0x7FFFFFFFu);
+      size_t at = ent.size();
+      for (int k = x.b; k < m1; ++k) ent.push_back((fg_ent[k] & 0xFFFFu) | one);
+      it.loss = list(at);
+      at = ent.size();
+      for (int k = m1; k < m2; ++k) ent.push_back(fg_ent[k] & 0x7FFFFFFFu);
+      it.prod = list(at);
+      at = ent.size();
       for (int k = m2; k < x.e; ++k) {
         fgt.neg.push_back(fg_ent[k] & 0x7FFFFFFFu);
         fgt.neg.push_back((uint32_t)x.sp);
-        it.neg.push_back((uint32_t)(f_zero + (int)fgt.neg.size() / 2) | one);
+        ent.push_back((uint32_t)(f_zero + (int)fgt.neg.size() / 2) | one);
       }
-      items.push_back(std::move(it));
+      it.neg = list(at);
+      items.push_back(it);
     }
     pack_gather(items, (uint32_t)f_zero, 16, &fgt);
   }
@@ -446,25 +477,32 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   const int j_zero = t.n_part_all + t.n_cv + t.n_pj + t.n_virt;
   GatherTables jgt;
   {
+    std::vector<uint32_t> ent;
+    ent.reserve(jg_w0.size());
+    auto list = [&](size_t from) { return GatherList{ent.data() + from, ent.size() - from}; };
     std::vector<GatherItem> items;
     items.reserve(t.n_jac);
     for (int e = 0; e < t.n_jac; ++e) {
       GatherItem it;
       it.id = jslot[e];
-      for (int g = t.jg_ptr[e]; g < jg_umid[e]; ++g)
-        it.lead.push_back((jg_w0[g] & 0xFFFFu) | one);
-      for (int g = jg_umid[e]; g < jg_mid[e]; ++g)
-        it.loss.push_back((jg_w0[g] & 0xFFFFu) | one);
+      size_t at = ent.size();
+      for (int g = t.jg_ptr[e]; g < jg_umid[e]; ++g) ent.push_back((jg_w0[g] & 0xFFFFu) | one);
+      it.lead = list(at);
+      at = ent.size();
+      for (int g = jg_umid[e]; g < jg_mid[e]; ++g) ent.push_back((jg_w0[g] & 0xFFFFu) | one);
+      it.loss = list(at);
+      at = ent.size();
       for (int g = jg_mid[e]; g < t.jg_ptr[e + 1]; ++g) {
         if (coef[jg_w0[g] >> 16] >= 0.0) {
-          it.prod.push_back(jg_w0[g]);
+          ent.push_back(jg_w0[g]);
           continue;
         }
         jgt.neg.push_back(jg_w0[g]);
         jgt.neg.push_back((uint32_t)(jg_w1[g] - 1) | ((uint32_t)t.jg_row[e] << 16));
-        it.prod.push_back((uint32_t)(j_zero + (int)jgt.neg.size() / 2) | one);
+        ent.push_back((uint32_t)(j_zero + (int)jgt.neg.size() / 2) | one);
       }
-      items.push_back(std::move(it));
+      it.prod = list(at);
+      items.push_back(it);
     }
     pack_gather(items, (uint32_t)j_zero, 8, &jgt);
   }
@@ -593,11 +631,8 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   o.n_jac = t.n_jac;
   o.n_lu = t.n_lu;
   o.n_coef = (int)coef.size();
-  o.n_funits = (int)units.size();
   o.n_fsplit = (int)split.size() / 3;
   o.n_fscratch = n_slots;
-  o.n_flev = t.n_flev;
-  o.n_blev = t.n_blev;
   o.rx_word = w.put(rx_word);
   o.coef = w.put(coef);
   o.fg_split = w.put(split);

@@ -16,8 +16,7 @@ struct BlobOff {
   int stage_bytes;  // prefix the level-scheduled mode stages
   int seq_bytes;    // prefix the one-lane LU mode stages (its LU tables too)
   // counts
-  int n, n_rxn, n_part, n_jac, n_lu, n_coef, n_funits, n_fsplit, n_fscratch;
-  int n_plev, n_flev, n_blev;
+  int n, n_rxn, n_part, n_jac, n_lu, n_coef, n_fsplit, n_fscratch, n_plev;
   // reactions: variable reactants packed (nv<<30 | d2<<20 | d1<<10 | d0; d0
   // and d1 default to n, where y holds 1), partial base
   int rx_word, rx_vptr;
@@ -62,15 +61,17 @@ struct BlobOff {
   // lu_src (uint32 x 3): those that a J slot fills (slots are numbered by LU
   // position), the diagonals, and the number of slots before them.
   int lu_iperm, lu_diag, lu_src;
-  // factorization by pivot level (n_plev): fl_hdr (uint16 x 2 per level):
-  // rounds of scaled L entries, rounds of updates.  A scaling round gives every lane fs_rec (uint32 L position |
-  // diagonal position<<16, uint32 pivot | store its reciprocal<<15; pivot
-  // 0x7FFF idle lane, L position n_lu nothing to scale).  An update round gives
-  // every lane one target LU[tgt] -= sum LU[a] LU[b]: record uint32 a | b<<16,
-  // uint32 tgt | cnt<<16 (fb_rec), the first pair in the record, cnt - 1 more
-  // per lane in fb_ext (uint32 a | b<<16, 32 per step).  cnt is the round's
-  // largest, the same in every lane: shorter targets and idle lanes are padded
-  // with the spare slot LU[n_lu] = 0.
+  // factorization by pivot level (n_plev): fl_hdr (uint16 x 2 per level): end
+  // of the level's scaling records, rounds of updates.  A scaling record fs_rec
+  // is an L entry (uint32 L position | diagonal position<<16, uint32 pivot |
+  // store its reciprocal<<15; L position n_lu: nothing to scale).  An update
+  // round gives every lane one target LU[tgt] -= sum LU[a] LU[b]: record uint32
+  // a | b<<16, uint32 tgt | cnt<<16 (fb_rec), the first pair in the record,
+  // cnt - 1 more per lane in fb_ext (uint32 a | b<<16, 32 per step).  cnt is the
+  // round's largest, the same in every lane: shorter targets and idle lanes are
+  // padded with the spare slot LU[n_lu] = 0.  Bit 15 of cnt: a round of targets
+  // of four pairs or more on two neighbouring lanes each, one of the two
+  // alternating sums per lane.
   int fl_hdr, fs_rec, fb_rec, fb_ext;
   // triangular solves: n_fwd rounds forward, then n_bwd backward.  A round
   // gives every lane one target z[tgt] -= sum LU[a] z[x] (backward: then times

@@ -11,7 +11,7 @@
 namespace campb {
 
 struct DevMech {
-  int n, n_state, n_rxn, n_part, n_jac, n_lu, n_photo, n_flev, n_blev;
+  int n, n_state, n_rxn, n_part, n_jac, n_lu, n_photo;
   int n_const;
   const int *rx_type, *rx_nreact, *rx_fpar, *rx_photo;
   const double* fpar;

@@ -2971,8 +2971,6 @@ bool Engine::init(const Model& model, const std::vector<double>& atol_dep, int c
   m.n_jac = t.n_jac;
   m.n_lu = t.n_lu;
   m.n_photo = t.n_photo;
-  m.n_flev = t.n_flev;
-  m.n_blev = t.n_blev;
   std::vector<int> cst;
   for (int i = 0; i < t.n_state; ++i)
     if (model.var_type()[i] == VAR_CONSTANT) cst.push_back(i);
