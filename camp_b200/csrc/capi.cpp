@@ -875,6 +875,22 @@ int camp_b200_get_jac_map(void* solver_data, int* triplets) {
   std::copy(m.jac_map().begin(), m.jac_map().end(), triplets);
   return 0;
 }
+long camp_b200_get_warp_tables(void* solver_data, void* out, long capacity) {
+  const Model& m = *S(solver_data)->model;
+  if (!m.built()) {
+    set_error("camp_b200_get_warp_tables: sparsity not built");
+    return -1;
+  }
+  std::vector<uint8_t> blob;
+  campb::BlobOff off{};
+  std::string err;
+  if (!campb::build_blob(m.tables(), std::vector<double>(m.tables().n, 0.0), &blob, &off, &err)) {
+    set_error("camp_b200_get_warp_tables: " + err);
+    return -1;
+  }
+  if (out && capacity >= (long)blob.size()) memcpy(out, blob.data(), blob.size());
+  return (long)blob.size();
+}
 long camp_b200_get_block_tables(void* solver_data, void* out, long capacity) {
   const Model& m = *S(solver_data)->model;
   if (!m.built()) {

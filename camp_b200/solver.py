@@ -328,15 +328,23 @@ class Solver:
     def n_lu(self) -> int:
         return int(self.lib.camp_b200_n_lu_elem(self._h))
 
-    def block_tables(self) -> bytes:
-        """The block-per-cell kernel's tables as built on the host (the
-        BlockOff header, then its sections)."""
-        n = int(self.lib.camp_b200_get_block_tables(self._h, None, 0))
+    def _tables(self, get) -> bytes:
+        n = int(get(self._h, None, 0))
         if n < 0:
             raise SolverError(_lib.last_error())
         buf = (C.c_uint8 * n)()
-        self.lib.camp_b200_get_block_tables(self._h, buf, n)
+        get(self._h, buf, n)
         return bytes(buf)
+
+    def block_tables(self) -> bytes:
+        """The block-per-cell kernel's tables as built on the host (the
+        BlockOff header, then its sections)."""
+        return self._tables(self.lib.camp_b200_get_block_tables)
+
+    def warp_tables(self) -> bytes:
+        """The warp-per-cell kernel's tables as built on the host (the
+        BlobOff header, then its sections)."""
+        return self._tables(self.lib.camp_b200_get_warp_tables)
 
     def check_jac(self, state, env, h: float, rel_tol: float = 1e-4, abs_tol: float = 1e-9):
         """Finite-difference audit of the device Jacobian at these states;

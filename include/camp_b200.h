@@ -309,6 +309,9 @@ int camp_b200_get_lu_order(void *solver_data, int *perm);
  * capacity allows; -1 (with camp_b200_last_error) when the mechanism has no
  * such tables. */
 long camp_b200_get_block_tables(void *solver_data, void *out, long capacity);
+/* The same of the warp-per-cell kernel's tables (the BlobOff header of
+ * blob.hpp, then its sections). */
+long camp_b200_get_warp_tables(void *solver_data, void *out, long capacity);
 /* The solver-Jacobian fold J_solver[s] += J_rxn[r] * J_params[p] as (s, r,
  * p) triplets in the reference's order (src/camp_solver.c:1649-1681; p = 0
  * is the unit parameter, the others the sub-model parameter Jacobian's

@@ -1,0 +1,105 @@
+"""The warp kernel on mechanisms whose LU, lists or yields lie at the edges of
+its tables (tests/test_warp_tables.py asserts which rounds each one has).
+
+An LU without L entries has no forward round, so the first round of the
+triangular solves already scales by reciprocal pivots; a solve that left the
+scaling out still converges where gamma * k < 1 and so shows as many more
+steps, as step limits on stiff losses and as a total that is not conserved.
+"""
+import numpy as np
+import pytest
+
+import small_mechs
+from conftest import gpu_available
+
+pytestmark = [pytest.mark.gpu,
+              pytest.mark.skipif(not gpu_available(), reason="no CUDA device")]
+
+RTOL, ATOL = 1e-4, 1e-8
+
+
+def _run(mech, y, rates, t, precision, max_steps=10000):
+    """(state, stats) of the library and (state, status, steps) of the oracle."""
+    from camp_b200.solver import Solver
+    from oracle.oracle import OracleModel
+
+    n = y.shape[0]
+    env = np.tile(np.array([298.0, 1.0e5]), (n, 1))
+    atol = np.full(mech.n_state_var, ATOL)
+    s = Solver(mech, n)
+    s.initialize(abs_tol=atol, rel_tol=RTOL, max_steps=max_steps)
+    s.set_precision(precision)
+    assert s.kernel() == 0
+    if rates.shape[1]:
+        s.set_photo_rates(rates)
+    x = y.copy()
+    s.solve(x, env, 0.0, t)
+    _, status, stats, o = OracleModel(mech).solve(y.copy(), env, rates, 0.0, t, RTOL, atol,
+                                                  max_steps=max_steps)
+    return x, s.cell_stats(), o, status, np.array([v.nst for v in stats])
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("t", [60.0, 900.0])
+@pytest.mark.parametrize("n_species", [1, 2, 32, 33, 65])
+def test_emission_and_first_order_loss(tmp_path, n_species, t, precision):
+    """dy/dt = e - k y with k from 0.1 to 1e3 s-1 over the cells: the oracle's
+    outcome, its step count to 20 %, and y = e/k + (y0 - e/k) exp(-k t) to ten
+    error weights (the problem is contracting, so an error of each step's
+    size, about a weight, is all that remains of the earlier ones)."""
+    names = small_mechs.names_of(n_species)
+    mech = small_mechs.mechanism(tmp_path, names, [
+        {"type": kind, "species": x} for x in names for kind in ("EMISSION", "FIRST_ORDER_LOSS")])
+    k = np.array([0.1, 1.0, 10.0, 100.0, 1000.0])[:, None] * np.linspace(0.5, 1.0, n_species)
+    eq = np.linspace(0.2, 1.5, n_species)[None, :]
+    rates = np.stack([k * eq, k], axis=2).reshape(len(k), -1)
+    y = np.ones((len(k), n_species))
+    x, st, o, status, nst = _run(mech, y, rates, t, precision)
+    assert (status == 0).all() and (st["status"] == 0).all()
+    assert (np.abs(st["nst"] - nst) <= 0.2 * nst).all(), (st["nst"], nst)
+    expect = eq + (y - eq) * np.exp(-k * t)
+    assert (np.abs(x - expect) <= 10.0 * (RTOL * expect + ATOL)).all()
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("n_species", [3, 40])
+def test_chain_conserves_its_total(tmp_path, n_species, reverse):
+    """X0 -> X1 -> ... in either state order, FP64: the columns of I - gamma*J
+    add up to one, so a solve conserves the total to its own rounding: at
+    most 1e-15 of the concentrations per species, iteration and pass."""
+    mech = small_mechs.chain(tmp_path, n_species, reverse)
+    y = np.random.default_rng(5).uniform(0.5, 1.0, (6, n_species))
+    x, st, o, status, nst = _run(mech, y, np.zeros((6, 0)), 10.0, 0)
+    assert (status == 0).all() and (st["status"] == 0).all()
+    assert (np.abs(st["nst"] - nst) <= 0.2 * nst).all(), (st["nst"], nst)
+    total = y.sum(axis=1)
+    assert (np.abs(x.sum(axis=1) - total) <= 1e-15 * n_species * st["nni"] * total).all()
+
+
+@pytest.mark.parametrize("negative", [False, True])
+@pytest.mark.parametrize("n_species", [10, 41, 90])
+def test_hub_f_and_jacobian(tmp_path, n_species, negative):
+    """Long lists and guarded terms: f and J against the oracle's to 1e-12 of
+    production plus loss, as on the packed mechanisms.  Half of the cells
+    hold species at 1e-9 ppm, where the guard drops terms."""
+    from camp_b200.solver import Solver
+    from oracle.oracle import OracleModel
+
+    mech = small_mechs.hub(tmp_path, n_species, negative)
+    n = 6
+    rng = np.random.default_rng(8)
+    y = rng.uniform(0.1, 1.0, (n, n_species))
+    y[: n // 2] = np.where(rng.random((n // 2, n_species)) < 0.3, 1e-9, y[: n // 2])
+    env = np.tile(np.array([298.0, 1.0e5]), (n, 1))
+    s = Solver(mech, n)
+    s.initialize(abs_tol=np.full(n_species, ATOL), rel_tol=RTOL)
+    om = OracleModel(mech)
+    for h in (0.01, 60.0):
+        f, p, l = s.eval_deriv(y, env, h)
+        j, jp, jl = s.eval_jac(y, env, h)
+        for c in range(n):
+            row = om.rxn_env_row(env[c], np.zeros(0))
+            of, _, _ = om.deriv(y[c], row, h)
+            oj = om.jac(y[c], row, h)
+            assert np.all(np.abs(f[c] - of) <= 1e-12 * (p[c] + l[c]))
+            assert np.all(np.abs(j[c] - oj) <= 1e-12 * (np.abs(jp[c]) + np.abs(jl[c])))
