@@ -6,6 +6,7 @@
 #include <map>
 #include <numeric>
 
+#include "bdf_consts.hpp"
 #include "model.hpp"
 
 namespace campb {
@@ -14,6 +15,7 @@ namespace {
 
 constexpr int kLanes = 32;
 constexpr uint16_t kNoSlot = 0xFFFF;
+constexpr int kEnoughCells = 8;  // cells per block beyond which more gain little
 
 struct Writer {
   std::vector<uint8_t> buf;
@@ -23,6 +25,16 @@ struct Writer {
     buf.resize(off + std::max<size_t>(v.size(), 1) * sizeof(T), 0);
     if (!v.empty()) memcpy(buf.data() + off, v.data(), v.size() * sizeof(T));
     return (int)off;
+  }
+};
+
+// where a Writer would be after the same puts
+struct Sizer {
+  size_t at;
+  template <typename T>
+  int put(const std::vector<T>& v) {
+    at = ((at + 15) & ~size_t(15)) + std::max<size_t>(v.size(), 1) * sizeof(T);
+    return 0;
   }
 };
 
@@ -228,8 +240,43 @@ void pack_gather(std::vector<GatherItem>& items, uint32_t zero, int bytes_per_in
 
 }  // namespace
 
-bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vector<uint8_t>* blob,
-                BlobOff* off, std::string* err) {
+Layout make_layout(const BlobOff& o, int lt_size, bool with_hist, bool with_tempv) {
+  Layout L{};
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    size_t r = off;
+    off = (off + bytes + 15) & ~size_t(15);
+    return (int)r;
+  };
+  const size_t vec = sizeof(double) * o.n;
+  L.zn = with_hist ? take(vec * bdf::LMAX) : -1;
+  L.ewt = take(vec);
+  L.acor = take(vec);
+  L.y = take(vec + sizeof(double));  // y[n]: see set_unit
+  L.ftemp = take(vec);
+  L.tempv = with_tempv ? take(vec) : -1;
+  // the f scratch (pseudo-rates, then the computed species, a zero and the guarded terms) and
+  // the J scratch (partials, computed species, parameter partials, virtual
+  // slots, a zero and the guarded terms), each followed by the sub-models'
+  // scratch; the solves' vector lies over them
+  const int n_scr = std::max(o.scr0[0], o.scr0[1]) + o.n_sms;
+  L.rates = L.z = take(std::max(sizeof(double) * n_scr, (size_t)lt_size * (o.n + 1)));
+  L.keff = take(sizeof(double) * o.n_keff);
+  // the split species' parts lie behind f's terms, over J's where those leave room
+  const int f_end = o.scr0[0] + o.n_sms, n_fscr = 2 * std::max(1, o.n_fscratch);
+  L.fscr = f_end + n_fscr <= n_scr ? L.rates + (int)sizeof(double) * f_end
+                                   : take(sizeof(double) * n_fscr);
+  // a spare slot: see clear_spare
+  L.lu = take((size_t)lt_size * (o.n_lu + 1));
+  L.dinv = take((size_t)lt_size * o.n);
+  // control block: tau[LMAX + 2], tq[8], l[LMAX + 1], quot[8]
+  L.ctl = take(sizeof(double) * (2 * bdf::LMAX + 19));
+  L.bytes = (int)off;
+  return L;
+}
+
+bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_smem,
+                std::vector<uint8_t>* blob, BlobOff* off, std::string* err) {
   const int n = t.n;
   if (n > 1023) {
     *err = "more than 1023 dependent variables";
@@ -506,11 +553,6 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     }
     pack_gather(items, (uint32_t)j_zero, 8, &jgt);
   }
-  if (fgt.a_ent.size() > 65535 || jgt.a_ent.size() > 65535 ||
-      f_zero + fgt.neg.size() / 2 > 65535 || j_zero + jgt.neg.size() / 2 > 65535) {
-    *err = "mechanism exceeds the 16-bit table encodings";
-    return false;
-  }
   // LU
   auto u16 = [](const std::vector<int>& v) {
     std::vector<uint16_t> o(v.size());
@@ -637,21 +679,6 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   o.coef = w.put(coef);
   o.fg_split = w.put(split);
   o.rx_vptr = w.put(rx_vptr);
-  for (int k = 0; k < 2; ++k) {
-    GatherTables& x = k == 0 ? fgt : jgt;
-    BlobOff::Gather& g = o.g[k];
-    g.n_a = (int)x.a_rec.size() / (2 * kLanes);
-    g.n_b = (int)x.b_hdr.size() / 2;
-    g.n_neg = (int)x.neg.size() / 2;
-    g.zero = k == 0 ? f_zero : j_zero;
-    g.a_rec = w.put(x.a_rec);
-    g.a_ent = w.put(x.a_ent);
-    g.b_hdr = w.put(x.b_hdr);
-    g.b_id = k == 0 ? w.put(x.b_id)
-                    : w.put(std::vector<uint16_t>(x.b_id.begin(), x.b_id.end()));
-    g.b_ent = w.put(x.b_ent);
-    g.neg = w.put(x.neg);
-  }
   o.has_ug = has_ug ? 1 : 0;
   o.n_simpol = t.n_simpol;
   o.n_keff = t.n_keff;
@@ -811,7 +838,6 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
     o.sm_pel = w.put(pel);
     o.sm_pst = w.put(pst);
     o.n_sms = (int)slots;
-    for (int k = 0; k < 2; ++k) o.scr0[k] = o.g[k].zero + 1 + o.g[k].n_neg;
     o.sm_int = w.put(ints);
     o.sm_flt = w.put(flts);
     o.n_virt = t.n_virt;
@@ -845,9 +871,72 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   o.sv_ext = w.put(svr.ext);
   o.dep_state = w.put(u16(t.dep_state));
   o.atol = w.put(atol_dep);
+  auto put_known = [&](auto& v, BlobOff* q) {
+    for (int k = 0; k < 2; ++k) {
+      GatherTables& x = k == 0 ? fgt : jgt;
+      BlobOff::Gather& g = q->g[k];
+      g.n_a = (int)x.a_rec.size() / (2 * kLanes);
+      g.n_b = (int)x.b_hdr.size() / 2;
+      g.n_neg = (int)x.neg.size() / 2;
+      g.a_rec = v.put(x.a_rec);
+      g.a_ent = v.put(x.a_ent);
+      g.b_hdr = v.put(x.b_hdr);
+      g.b_id = k == 0 ? v.put(x.b_id)
+                      : v.put(std::vector<uint16_t>(x.b_id.begin(), x.b_id.end()));
+      g.b_ent = v.put(x.b_ent);
+      g.neg = v.put(x.neg);
+    }
+  };
+  auto put_any = [&](auto& v, BlobOff* q) {
+    q->fg_ent = v.put(fg_ent);
+    q->fg_unit = v.put(fg_unit);
+    q->fg_lane = v.put(fg_lane);
+    q->j_csc = v.put(u16(jcsc));
+    q->jg_slot = v.put(u16(jslot));
+    q->jg_w0 = v.put(jg_w0);
+    q->jg_w1 = v.put(jg_w1);
+    q->jg_ptr = v.put(jg_ptr);
+    q->jg_mid = v.put(jg_mid);
+    q->jg_row = v.put(jg_row);
+    q->jg_lane = v.put(jg_lane);
+    q->jg_slots = v.put(jg_slots);
+    q->jg_umid = v.put(jg_umid);
+  };
+  for (int k = 0; k < 2; ++k) o.g[k].zero = k == 0 ? f_zero : j_zero;
+  // cells per block (FP64, all in shared memory) with the given gathers staged
+  auto cells = [&](bool any) {
+    BlobOff q = o;
+    Sizer v{w.buf.size()};
+    any ? put_any(v, &q) : put_known(v, &q);
+    for (int k = 0; k < 2; ++k) q.scr0[k] = q.g[k].zero + 1 + q.g[k].n_neg;
+    const int room = max_smem - (int)((v.at + 127) & ~size_t(127));
+    return std::max(0, room / make_layout(q, 8, true, false).bytes);
+  };
+  // A guarded term takes eight bytes of every cell's slab beside its table
+  // entry, so a mechanism with many of them holds fewer cells, or none at all,
+  // with the known-sign gathers staged; it keeps the gathers for any signs
+  // where those hold a third more cells (1 500 cells of random mechanisms,
+  // FP64, cells and ms of known / any signs: 20 species x 300 reactions, all
+  // yields negative, 3 / 12 cells 111 / 37 ms; 15 x 600 1 / 7, 372 / 72;
+  // 40 x 100, half negative, 3 / 4, 131 / 110; 15 x 300 6 / 16, 51 / 47; with
+  // as many cells known signs are 0.99 to 1.8 times as fast (cb05 1.11, mod37
+  // gas 1.18), and beyond eight cells a block gains little: instruction fetch
+  // bounds it).
+  const bool fits = fgt.a_ent.size() <= 65535 && jgt.a_ent.size() <= 65535 &&
+                    f_zero + fgt.neg.size() / 2 <= 65535 && j_zero + jgt.neg.size() / 2 <= 65535;
+  const bool guards = !fgt.neg.empty() || !jgt.neg.empty();
+  if (!fits) {
+    o.any_sign = 1;
+  } else if (guards) {
+    const int known = cells(false);
+    const int any = known < kEnoughCells ? std::min(cells(true), kEnoughCells) : 0;
+    o.any_sign = any > 0 && 4 * known <= 3 * any;
+  }
+  o.any_sign ? put_any(w, &o) : put_known(w, &o);
+  for (int k = 0; k < 2; ++k) o.scr0[k] = o.g[k].zero + 1 + o.g[k].n_neg;
   // the level-scheduled mode stages only the bytes up to here into shared
-  // memory, the one-lane LU mode its LU tables too; the f gather for any
-  // signs and the J gather come last and stay in global memory
+  // memory, the one-lane LU mode its LU tables too; the gathers for any signs,
+  // where they are the exception, come last and stay in global memory
   w.buf.resize((w.buf.size() + 15) & ~size_t(15), 0);
   o.stage_bytes = (int)w.buf.size();
   {
@@ -863,19 +952,7 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, std::vecto
   }
   w.buf.resize((w.buf.size() + 15) & ~size_t(15), 0);
   o.seq_bytes = (int)w.buf.size();
-  o.fg_ent = w.put(fg_ent);
-  o.fg_unit = w.put(fg_unit);
-  o.fg_lane = w.put(fg_lane);
-  o.j_csc = w.put(u16(jcsc));
-  o.jg_slot = w.put(u16(jslot));
-  o.jg_w0 = w.put(jg_w0);
-  o.jg_w1 = w.put(jg_w1);
-  o.jg_ptr = w.put(jg_ptr);
-  o.jg_mid = w.put(jg_mid);
-  o.jg_row = w.put(jg_row);
-  o.jg_lane = w.put(jg_lane);
-  o.jg_slots = w.put(jg_slots);
-  o.jg_umid = w.put(jg_umid);
+  if (!o.any_sign) put_any(w, &o);
   w.buf.resize((w.buf.size() + 15) & ~size_t(15), 0);
   o.bytes = (int)w.buf.size();
   memcpy(w.buf.data(), &o, sizeof(o));

@@ -17,6 +17,7 @@ struct BlobOff {
   int seq_bytes;    // prefix the one-lane LU mode stages (its LU tables too)
   // counts
   int n, n_rxn, n_part, n_jac, n_lu, n_coef, n_fsplit, n_fscratch, n_plev;
+  int any_sign;  // the gathers for any signs are staged and used throughout
   // reactions: variable reactants packed (nv<<30 | d2<<20 | d1<<10 | d0; d0
   // and d1 default to n, where y holds 1), partial base
   int rx_word, rx_vptr;
@@ -25,11 +26,11 @@ struct BlobOff {
   // f gather for any signs: entries (rxn | coef<<16 | prod<<31), units
   // (species, begin, end of losses, end of non-negative-yield products, end,
   // slot) as 8 x uint16, lane pointers (33 x uint16); read from the blob in
-  // global memory (self).  Split species (species, first slot, count) as 3 x
+  // global memory (self) where they are the exception.  Split species (species, first slot, count) as 3 x
   // uint16
   int fg_ent, fg_unit, fg_lane, fg_split;
   // f (g[0]) and J (g[1]) gathers where no rate (partial), concentration or
-  // step is negative; every item is a unit of the f gather or a slot of the
+  // step is negative (empty with any_sign); every item is a unit of the f gather or a slot of the
   // solver Jacobian, its sums L0, L1, P0 and P1 four chains of entries (uint32
   // index | coef<<16).  Long items come first, as n_a rounds of eight items
   // with one lane per chain: per lane a_rec (uint32 first entry | entries<<16,
@@ -52,7 +53,7 @@ struct BlobOff {
   unsigned long long self;  // the blob's own address in global memory
   // J gather for any signs: w0 = part | coef<<16, w1 = independent species + 1
   // (0 = loss entry); per slot: entry pointer, LU position, row; lane slot
-  // lists.  Read from the blob in global memory (self).
+  // lists.  Read as those of f.
   int jg_w0, jg_w1, jg_ptr, jg_mid, jg_lupos, jg_row, jg_lane, jg_slots;
   // device J slots are numbered by LU position; CSC entry of each slot and
   // slot of each CSC entry (uint16; self)
@@ -133,14 +134,24 @@ struct BlobOff {
 };
 
 constexpr int kBlobHeader = 512;
+constexpr int kBlockSmem = 232448;  // the most shared memory of a block on sm_100a
 
 struct Tables;
 
 // Builds the blob; false (with a message) if the mechanism exceeds the
 // encodings (more than 3 variable reactants in a reaction, more than 1023
 // dependent variables, or index spaces beyond 16 bits).
-bool build_blob(const Tables& t, const std::vector<double>& atol_dep,
+// max_smem: the most shared memory of a block, for the choice of the gathers.
+bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_smem,
                 std::vector<uint8_t>* blob, BlobOff* off, std::string* err);
+
+// A cell's shared-memory slice (byte offsets; -1 = not in it).  Without the
+// Nordsieck history it leaves room for more resident cells; tempv is for the
+// evaluation hooks.
+struct Layout {
+  int zn, ewt, acor, y, ftemp, tempv, rates, keff, fscr, lu, z, dinv, ctl, bytes;
+};
+Layout make_layout(const BlobOff& o, int lt_size, bool with_hist, bool with_tempv);
 
 }  // namespace campb
 

@@ -884,7 +884,8 @@ long camp_b200_get_warp_tables(void* solver_data, void* out, long capacity) {
   std::vector<uint8_t> blob;
   campb::BlobOff off{};
   std::string err;
-  if (!campb::build_blob(m.tables(), std::vector<double>(m.tables().n, 0.0), &blob, &off, &err)) {
+  if (!campb::build_blob(m.tables(), std::vector<double>(m.tables().n, 0.0), campb::kBlockSmem,
+                         &blob, &off, &err)) {
     set_error("camp_b200_get_warp_tables: " + err);
     return -1;
   }

@@ -49,10 +49,6 @@ constexpr int DO_ERROR_TEST = 100, PREDICT_AGAIN = 101, TRY_AGAIN = 102;
 constexpr int kMaxCellsPerBlock = 12;
 constexpr int kMaxCellsAero = 8;  // cells per block of the aerosol form
 
-struct Layout {  // per-warp shared-memory slice (byte offsets; -1 = not in it)
-  int zn, ewt, acor, y, ftemp, tempv, rates, keff, fscr, lu, z, dinv, ctl, bytes;
-};
-
 struct SolveArgs {
   DevMech m;
   BlobOff off;
@@ -208,9 +204,12 @@ struct Tab {
   int n, n_rxn, n_jac, n_lu, n_fsplit, n_simpol, has_ug, n_aq;
 };
 
+// STAGED: the gathers for any signs too are in shared memory (any_sign); the
+// whole blob is in global memory in any case
+template <bool STAGED = false>
 __device__ __forceinline__ Tab make_tab(const char* b) {
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(b);
-  const char* g = (const char*)o.self;  // the tables that are not staged
+  const char* g = STAGED ? b : (const char*)o.self;
   Tab t;
   t.rx_word = (const uint32_t*)(b + o.rx_word);
   t.rx_vptr = (const uint16_t*)(b + o.rx_vptr);
@@ -856,11 +855,16 @@ __device__ __forceinline__ void f_combine(const char* tb, const double* fscr, do
 }
 
 // f with any signs; see dev_f
-__device__ __noinline__ int dev_f_any(const char* tb, const double* y, double h,
-                                      const double* keff, double* rates, double* fscr,
-                                      double* out, int lane, double* rp, double* rl,
-                                      bool neg_extra) {
-  const Tab t = make_tab(tb);
+template <bool STAGED>
+__device__ __noinline__ int dev_f_any(const double* y, double h, const double* keff,
+                                      double* rates, double* fscr, double* out, int lane,
+                                      double* rp, double* rl, bool neg_extra) {
+  y = sh(y);
+  keff = sh(keff);
+  rates = sh(rates);
+  fscr = sh(fscr);
+  out = sh(out);
+  const Tab t = make_tab<STAGED>(g_smem);
   bool bad = false;
   #pragma unroll 1
   for (int i = lane; i < t.n; i += 32) bad |= y[i] < -kSmall;
@@ -941,7 +945,7 @@ __device__ __noinline__ int dev_f_any(const char* tb, const double* y, double h,
     }
   }
   __syncwarp();
-  f_combine<true>(tb, fscr, out, lane, rp, rl);
+  f_combine<true>(g_smem, fscr, out, lane, rp, rl);
   return 0;
 }
 
@@ -1093,6 +1097,10 @@ __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
   keff = sh(keff);
   rates = sh(rates);
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  const bool neg_rate = (flags & kNegRate) != 0;
+  if (o.any_sign)
+    return dev_f_any<true>(y, h, keff, rates, fscr, out, lane, EV ? rp : nullptr,
+                           EV ? rl : nullptr, neg_rate);
   bool odd = flags != 0 || !(h >= 0.0);
   const int n_rxn = o.n_rxn;
   const uint32_t* rx_word = (const uint32_t*)(tb + o.rx_word);
@@ -1107,8 +1115,8 @@ __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
     odd |= !(rate >= 0.0);
   }
   if (warp_any(odd))
-    return dev_f_any(tb, y, h, keff, rates, fscr, out, lane, EV ? rp : nullptr,
-                     EV ? rl : nullptr, (flags & kNegRate) != 0);
+    return dev_f_any<false>(y, h, keff, rates, fscr, out, lane, EV ? rp : nullptr,
+                            EV ? rl : nullptr, neg_rate);
   const BlobOff::Gather& g = o.g[0];
   if (lane == 0) rates[g.zero] = 0.0;
   __syncwarp();
@@ -1143,11 +1151,14 @@ __device__ __forceinline__ double jac_prod(const Tab& t, const double* part, con
 
 // the Jacobian with any signs (each lane writes the slots of its balanced
 // list); see dev_jac
-template <typename JT>
-__device__ __noinline__ int dev_jac_any(const char* tb, const double* y, double h,
-                                        const double* keff, double* part, JT* Jout, int lane,
-                                        const uint16_t* csc, double* jp, double* jl) {
-  const Tab t = make_tab(tb);
+template <typename JT, bool STAGED>
+__device__ __noinline__ int dev_jac_any(const double* y, double h, const double* keff,
+                                        double* part, JT* Jout, int lane, const uint16_t* csc,
+                                        double* jp, double* jl) {
+  y = sh(y);
+  keff = sh(keff);
+  part = sh(part);
+  const Tab t = make_tab<STAGED>(g_smem);
   bool bad = false;
   #pragma unroll 1
   for (int i = lane; i < t.n; i += 32) bad |= y[i] < -kSmall;
@@ -1229,6 +1240,9 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
   keff = sh(keff);
   part = sh(part);
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  if (o.any_sign)
+    return dev_jac_any<JT, true>(y, h, keff, part, Jout, lane, EV ? csc : nullptr,
+                                 EV ? jp : nullptr, EV ? jl : nullptr);
   bool odd = flags != 0 || !(h >= 0.0);
   const int n_rxn = o.n_rxn;
   // d rate / d y_k for every variable reactant occurrence k
@@ -1258,8 +1272,8 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
     }
   }
   if (warp_any(odd))
-    return dev_jac_any<JT>(tb, y, h, keff, part, Jout, lane, EV ? csc : nullptr,
-                           EV ? jp : nullptr, EV ? jl : nullptr);
+    return dev_jac_any<JT, false>(y, h, keff, part, Jout, lane, EV ? csc : nullptr,
+                                  EV ? jp : nullptr, EV ? jl : nullptr);
   const BlobOff::Gather& g = o.g[1];
   if (lane == 0) part[g.zero] = 0.0;
   __syncwarp();
@@ -3089,7 +3103,7 @@ bool Engine::init(const Model& model, const std::vector<double>& atol_dep, int c
   if (I->d_blob) cudaFree(I->d_blob);
   I->d_blob = nullptr;
   I->warp_why.clear();
-  I->warp_ok = build_blob(t, atol_dep, &blob, &I->off, &I->warp_why);
+  I->warp_ok = build_blob(t, atol_dep, I->max_smem, &blob, &I->off, &I->warp_why);
   if (I->warp_ok) {
     CK(cudaMalloc(&I->d_blob, blob.size()));
     I->off.self = (unsigned long long)(uintptr_t)I->d_blob;
@@ -3128,45 +3142,6 @@ bool Engine::init(const Model& model, const std::vector<double>& atol_dep, int c
     CK(cudaEventCreate(&I->ev1));
   }
   return true;
-}
-
-// per-warp shared-memory slice; the solve kernel keeps the Nordsieck history
-// and the rate constants in global memory (with_hist = false), which leaves
-// room for more resident cells
-static Layout make_layout(const BlobOff& o, int lt_size, bool with_hist,
-                          bool with_tempv) {
-  Layout L{};
-  size_t off = 0;
-  auto take = [&](size_t bytes) {
-    size_t r = off;
-    off = (off + bytes + 15) & ~size_t(15);
-    return (int)r;
-  };
-  const size_t vec = sizeof(double) * o.n;
-  L.zn = with_hist ? take(vec * LMAX) : -1;
-  L.ewt = take(vec);
-  L.acor = take(vec);
-  L.y = take(vec + sizeof(double));  // y[n]: see set_unit
-  L.ftemp = take(vec);
-  L.tempv = with_tempv ? take(vec) : -1;
-  // the f scratch (pseudo-rates, then the computed species, a zero and the guarded terms) and
-  // the J scratch (partials, computed species, parameter partials, virtual
-  // slots, a zero and the guarded terms), each followed by the sub-models'
-  // scratch; the solves' vector lies over them
-  const int n_scr = std::max(o.scr0[0], o.scr0[1]) + o.n_sms;
-  L.rates = L.z = take(std::max(sizeof(double) * n_scr, (size_t)lt_size * (o.n + 1)));
-  L.keff = take(sizeof(double) * o.n_keff);
-  // the split species' parts lie behind f's terms, over J's where those leave room
-  const int f_end = o.scr0[0] + o.n_sms, n_fscr = 2 * std::max(1, o.n_fscratch);
-  L.fscr = f_end + n_fscr <= n_scr ? L.rates + (int)sizeof(double) * f_end
-                                   : take(sizeof(double) * n_fscr);
-  // a spare slot: see clear_spare
-  L.lu = take((size_t)lt_size * (o.n_lu + 1));
-  L.dinv = take((size_t)lt_size * o.n);
-  // control block: tau[LMAX + 2], tq[8], l[LMAX + 1], quot[8]
-  L.ctl = take(sizeof(double) * (LMAX + 2 + 8 + LMAX + 1 + 8));
-  L.bytes = (int)off;
-  return L;
 }
 
 // shared-memory bytes of the staged tables: the one-lane LU mode also needs

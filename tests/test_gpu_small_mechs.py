@@ -103,3 +103,42 @@ def test_hub_f_and_jacobian(tmp_path, n_species, negative):
             oj = om.jac(y[c], row, h)
             assert np.all(np.abs(f[c] - of) <= 1e-12 * (p[c] + l[c]))
             assert np.all(np.abs(j[c] - oj) <= 1e-12 * (np.abs(jp[c]) + np.abs(jl[c])))
+
+
+@pytest.mark.parametrize("n_species,n_rxn", [(15, 600), (30, 300), (10, 1000)])
+def test_guarded_terms_f_and_jacobian(tmp_path, n_species, n_rxn):
+    """Every product guarded: the gathers for any signs, staged; to the same
+    bound as above.  Half of the cells hold a species below zero (above the
+    smallest refused value) or at 1e-12 ppm."""
+    from camp_b200.solver import Solver
+    from oracle.oracle import OracleModel
+
+    mech = small_mechs.dense_negative(tmp_path, n_species, n_rxn, 5)
+    n = 6
+    y = np.random.default_rng(9).uniform(0.1, 1.0, (n, n_species))
+    y[0, 3], y[1, 1], y[2, :5] = -1e-31, 0.0, 1e-12
+    env = np.tile(np.array([298.0, 1.0e5]), (n, 1))
+    s = Solver(mech, n)
+    s.initialize(abs_tol=np.full(n_species, ATOL), rel_tol=RTOL)
+    om = OracleModel(mech)
+    for h in (1e-5, 1.0):
+        f, p, l = s.eval_deriv(y, env, h)
+        j, jp, jl = s.eval_jac(y, env, h)
+        for c in range(n):
+            row = om.rxn_env_row(env[c], np.zeros(0))
+            of, _, _ = om.deriv(y[c], row, h)
+            oj = om.jac(y[c], row, h)
+            assert np.all(np.abs(f[c] - of) <= 1e-12 * (p[c] + l[c]))
+            assert np.all(np.abs(j[c] - oj) <= 1e-12 * (np.abs(jp[c]) + np.abs(jl[c])))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_guarded_terms_solve(tmp_path, precision):
+    """10 species, 1 000 reactions of guarded products: the oracle's outcomes
+    and no concentration below zero (the guards make f jump, so the distance
+    of two runs says nothing)."""
+    mech = small_mechs.dense_negative(tmp_path, 10, 1000, 5)
+    y = np.random.default_rng(9).uniform(0.1, 1.0, (6, 10))
+    x, st, _, status, _ = _run(mech, y, np.zeros((6, 0)), 0.01, precision)
+    assert (status == 0).all() and (st["status"] == 0).all()
+    assert (x >= 0.0).all() and (x <= y + ATOL).all()

@@ -34,7 +34,7 @@ class BlobOff(C.Structure):
     _fields_ = (
         [(f, C.c_int) for f in (
             "bytes stage_bytes seq_bytes n n_rxn n_part n_jac n_lu n_coef n_fsplit n_fscratch "
-            "n_plev rx_word rx_vptr coef fg_ent fg_unit fg_lane fg_split").split()]
+            "n_plev any_sign rx_word rx_vptr coef fg_ent fg_unit fg_lane fg_split").split()]
         + [("g", Gather * 2), ("self", C.c_ulonglong)]
         + [(f, C.c_int) for f in (
             "jg_w0 jg_w1 jg_ptr jg_mid jg_lupos jg_row jg_lane jg_slots j_csc jg_slot lu_iperm "
@@ -142,6 +142,7 @@ def sums(t, k, src):
     assert len(src) == g.zero + 1 + g.n_neg
     neg = t.arr(g.neg, np.uint32, 2 * g.n_neg)[0::2]
     src[g.zero + 1:] = src[neg & 0xFFFF] * t.coef[neg >> 16] * (-1.0 if k == 0 else 1.0)
+    assert not o.any_sign
     P, L = {}, {}
 
     def add(word, p, l):
@@ -289,3 +290,18 @@ def test_synthetic(n_species, n_rxn):
     t = Tables(mech)
     check_factor_and_solve(t, 11)
     check_gathers(t, 12)
+
+
+@pytest.mark.parametrize("n_species,n_rxn,any_sign", [(15, 600, 1), (30, 300, 1), (10, 1000, 1),
+                                                       (20, 20, 0)])
+def test_guarded_terms_take_no_cells(tmp_path, n_species, n_rxn, any_sign):
+    """A guarded term would take a slot of every cell's slab: where that costs
+    cells, the gathers for any signs are staged and the others empty."""
+    t = Tables(small_mechs.dense_negative(tmp_path, n_species, n_rxn, 5))
+    o = t.o
+    assert o.any_sign == any_sign
+    for k in range(2):
+        assert (o.g[k].n_neg == 0 and o.g[k].n_a + o.g[k].n_b == 0) == bool(any_sign)
+    for at in (o.fg_ent, o.fg_unit, o.fg_lane, o.jg_slot, o.jg_w0, o.jg_w1, o.jg_ptr, o.jg_umid):
+        assert (at < o.stage_bytes) == bool(any_sign)
+    check_factor_and_solve(t, 13)
