@@ -616,6 +616,13 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
   // without pairs drop out (the schedule's phase g holds level g - 1's updates)
   rounds_of(t.fb, &fbr, lu_none, t.n_lu, false);
   rounds_of(t.fwd, &svr, sv_none, n, true);
+  if (svr.cnt.empty()) {
+    // L has no entries: an empty round, as the solve starts with a forward one
+    svr.cnt.push_back(1);
+    svr.pair0.resize(kLanes, sv_none);
+    svr.target.resize(kLanes, (uint32_t)n);
+    svr.recip.resize(kLanes, 0u);
+  }
   const int n_fwd = (int)svr.cnt.size();
   rounds_of(t.bwd, &svr, sv_none, n, true);
   std::vector<uint32_t> fb_rec, sv_rec, fs_rec;

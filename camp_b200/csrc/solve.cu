@@ -1521,8 +1521,7 @@ __device__ __noinline__ void dev_lsolve(const LT* LU, const LT* dinv, LT* z, int
   const uint2* rec = (const uint2*)(g_smem + o.sv_rec) + lane;
   const uint32_t* ext = (const uint32_t*)(g_smem + o.sv_ext) + lane;
   uint2 w = rec[0], wn = rec[32];
-  // the first round is a backward one where L has no entries
-  LT a = LU[w.x & 0xFFFFu], d = (w.y & 0x8000u) ? dinv[w.y & 0x7FFFu] : (LT)1;
+  LT a = LU[w.x & 0xFFFFu], d = (LT)1;  // the first round is a forward one
   rec += 64;
   #pragma unroll 1
   for (int r = o.n_fwd + o.n_bwd; r > 0; --r) {
