@@ -854,6 +854,11 @@ __device__ __forceinline__ void f_combine(const char* tb, const double* fscr, do
   __syncwarp();
 }
 
+// which gathers of f and J are staged (BlobOff::any_sign); the solve kernel is
+// compiled for each, the evaluation hooks for either (the branch and the other
+// gathers' code cost the solve kernel 3 to 5 % on cb05: instruction fetch)
+constexpr int kKnownSigns = 0, kAnySigns = 1, kEither = 2;
+
 // f with any signs; see dev_f
 template <bool STAGED>
 __device__ __noinline__ int dev_f_any(const double* y, double h, const double* keff,
@@ -1087,7 +1092,7 @@ __device__ __noinline__ void gather(int k, const double* src, double* out, doubl
 // aerosol pseudo-rate is negative (kNegRate).  Everything else (also a NaN) takes
 // dev_f_any, which classifies and guards term by term; the sums' order is the
 // same.
-template <typename LT, bool EV = false>
+template <typename LT, bool EV = false, int FORM = kEither>
 __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
                                   const double* keff, double* rates, double* fscr,
                                   double* out, int lane, int flags, double* rp = nullptr,
@@ -1097,10 +1102,9 @@ __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
   keff = sh(keff);
   rates = sh(rates);
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
-  const bool neg_rate = (flags & kNegRate) != 0;
-  if (o.any_sign)
+  if (FORM == kAnySigns || (FORM == kEither && o.any_sign))
     return dev_f_any<true>(y, h, keff, rates, fscr, out, lane, EV ? rp : nullptr,
-                           EV ? rl : nullptr, neg_rate);
+                           EV ? rl : nullptr, (flags & kNegRate) != 0);
   bool odd = flags != 0 || !(h >= 0.0);
   const int n_rxn = o.n_rxn;
   const uint32_t* rx_word = (const uint32_t*)(tb + o.rx_word);
@@ -1116,7 +1120,7 @@ __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
   }
   if (warp_any(odd))
     return dev_f_any<false>(y, h, keff, rates, fscr, out, lane, EV ? rp : nullptr,
-                            EV ? rl : nullptr, neg_rate);
+                            EV ? rl : nullptr, (flags & kNegRate) != 0);
   const BlobOff::Gather& g = o.g[0];
   if (lane == 0) rates[g.zero] = 0.0;
   __syncwarp();
@@ -1230,7 +1234,7 @@ __device__ __noinline__ int dev_jac_any(const double* y, double h, const double*
 // concentration or step: then a product with a non-negative yield always
 // passes its guard; anything else takes dev_jac_any, with the sums in the same
 // order.
-template <typename JT, bool EV = false>
+template <typename JT, bool EV = false, int FORM = kEither>
 __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
                                     const double* keff, double* part, JT* Jout, int lane, int flags,
                                     const uint16_t* csc = nullptr, double* jp = nullptr,
@@ -1240,7 +1244,7 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
   keff = sh(keff);
   part = sh(part);
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
-  if (o.any_sign)
+  if (FORM == kAnySigns || (FORM == kEither && o.any_sign))
     return dev_jac_any<JT, true>(y, h, keff, part, Jout, lane, EV ? csc : nullptr,
                                  EV ? jp : nullptr, EV ? jl : nullptr);
   bool odd = flags != 0 || !(h >= 0.0);
@@ -1309,7 +1313,7 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
 // J[row][j] += V[row][c] * P[c][j] (src/camp_solver.c:1063-1106).  Where
 // the production / loss split jp / jl is asked for, each chained term adds to
 // the production part when positive and to the loss part when negative.
-template <typename LT, bool EV = false>
+template <typename LT, bool EV = false, int FORM = kEither>
 __device__ __noinline__ int dev_f_aero(const char* tb, const double* y, double h,
                                        const double* keff, double* rates, double* fscr,
                                        double* out, int lane, int flags, double* rp = nullptr,
@@ -1318,10 +1322,10 @@ __device__ __noinline__ int dev_f_aero(const char* tb, const double* y, double h
   double* cv = rates + o.n_rates;
   if (o.n_cv > 0) sub_model_eval<false>(y, keff, cv, nullptr, rates + o.scr0[0], lane);
   const bool neg = aero_rates(tb, y, keff, cv, rates, lane);
-  return dev_f<LT, EV>(tb, y, h, keff, rates, fscr, out, lane, flags | (neg ? kNegRate : 0), rp,
+  return dev_f<LT, EV, FORM>(tb, y, h, keff, rates, fscr, out, lane, flags | (neg ? kNegRate : 0), rp,
                        rl);
 }
-template <typename JT, bool EV = false>
+template <typename JT, bool EV = false, int FORM = kEither>
 __device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double h,
                                          const double* keff, double* part, JT* Jout, int lane, int flags,
                                          const uint16_t* csc = nullptr, double* jp = nullptr,
@@ -1332,7 +1336,7 @@ __device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double
   double* V = P + o.n_pj;
   if (o.n_cv > 0) sub_model_eval<true>(y, keff, cv, P, part + o.scr0[1], lane);
   aero_partials(tb, y, keff, cv, part, lane);
-  const int r = dev_jac<JT, EV>(tb, y, h, keff, part, Jout, lane, flags, csc, jp, jl);
+  const int r = dev_jac<JT, EV, FORM>(tb, y, h, keff, part, Jout, lane, flags, csc, jp, jl);
   if (r != 0 || o.n_chain == 0) return r;
   const uint16_t* vptr = (const uint16_t*)(tb + o.jv_ptr);
   const uint16_t* vpart = (const uint16_t*)(tb + o.jv_part);
@@ -1751,7 +1755,7 @@ __device__ __noinline__ int vec_start(const double* zb, double* acor, double* y,
 // loops, warp reductions).  BLK: the CTA-per-cell form, whose heavy
 // operations (f, J, factorization, solves) run on the whole block through
 // blk::call (block.cuh) while this warp keeps the control.
-template <typename LT, bool AERO, bool BLK = false>
+template <typename LT, bool AERO, int FORM, bool BLK = false>
 struct Cell {
   const char* tb;     // shared-memory tables
   const uint16_t* iperm;  // dependent index -> pivot row
@@ -1786,9 +1790,9 @@ struct Cell {
       blk::call<LT>(cmd, *bx, blk::OP_F, yy, out, h > 0.0 ? h : h0);
       return 0;
     } else if constexpr (AERO)
-      return dev_f_aero<LT>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
+      return dev_f_aero<LT, false, FORM>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
     else
-      return dev_f<LT>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
+      return dev_f<LT, false, FORM>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
   }
   __device__ bool set_ewt(const double* yy) {
     bool bad = false;
@@ -1940,9 +1944,9 @@ struct Cell {
         blk::call<LT>(cmd, *bx, blk::OP_JAC, ypred, nullptr, h > 0.0 ? h : h0);
         jr = 0;
       } else if constexpr (AERO) {
-        jr = dev_jac_aero<LT>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
+        jr = dev_jac_aero<LT, false, FORM>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
       } else {
-        jr = dev_jac<LT>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
+        jr = dev_jac<LT, false, FORM>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
       }
       if (jr) return 1;
     }
@@ -2326,8 +2330,8 @@ struct Cell {
 // ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
-template <typename LT, bool AERO>
-__device__ void bind_cell(Cell<LT, AERO>& c, const SolveArgs& a, const char* tab, char* base,
+template <typename LT, bool AERO, int FORM>
+__device__ void bind_cell(Cell<LT, AERO, FORM>& c, const SolveArgs& a, const char* tab, char* base,
                           int gwarp, int lane) {
   c.tb = tab;
   c.atol = make_tab(tab).atol;
@@ -2365,7 +2369,7 @@ __device__ void bind_cell(Cell<LT, AERO>& c, const SolveArgs& a, const char* tab
 // AERO: the mechanism has SIMPOL, HL, aqueous equilibrium or sub-models,
 // whose out-of-line evaluations take registers that the gas-phase form keeps
 // for itself; that form runs fewer cells per block.
-template <typename LT, bool AERO>
+template <typename LT, bool AERO, int FORM>
 __global__ void __launch_bounds__(32 * (AERO ? kMaxCellsAero : kMaxCellsPerBlock), 1)
     solve_kernel(SolveArgs a) {
   char* const smem = g_smem;
@@ -2375,8 +2379,8 @@ __global__ void __launch_bounds__(32 * (AERO ? kMaxCellsAero : kMaxCellsPerBlock
   const int wib = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * (blockDim.x >> 5) + wib;
   char* base = smem + a.tab_bytes + (size_t)wib * a.lay.bytes;
-  Cell<LT, AERO> c;
-  bind_cell<LT, AERO>(c, a, smem, base, gwarp, lane);
+  Cell<LT, AERO, FORM> c;
+  bind_cell<LT, AERO, FORM>(c, a, smem, base, gwarp, lane);
   clear_spare<LT>(smem, c.LU, lane);
   set_unit(c.y, c.n, lane);
   const DevMech& m = a.m;
@@ -2532,7 +2536,7 @@ __global__ void __launch_bounds__(blk::kThreads, sizeof(LT) == 4 ? 2 : 1)
       blk::serve<LT>(&cmd, *cx);
       continue;
     }
-    Cell<LT, false, true> c;
+    Cell<LT, false, kKnownSigns, true> c;
     c.tb = nullptr;
     c.iperm = nullptr;
     c.cmd = &cmd;
@@ -3160,10 +3164,17 @@ static bool aero_form(const BlobOff& o) { return o.n_simpol > 0 || o.n_aq > 0 ||
 static int max_cells_of(const BlobOff& o) {
   return aero_form(o) ? kMaxCellsAero : kMaxCellsPerBlock;
 }
+template <bool AERO, int FORM>
+static void* solve_kernel_of(int precision) {
+  return precision == 1 ? (void*)solve_kernel<float, AERO, FORM>
+                        : (void*)solve_kernel<double, AERO, FORM>;
+}
 static void* solve_kernel_fn(const BlobOff& o, int precision) {
   if (aero_form(o))
-    return precision == 1 ? (void*)solve_kernel<float, true> : (void*)solve_kernel<double, true>;
-  return precision == 1 ? (void*)solve_kernel<float, false> : (void*)solve_kernel<double, false>;
+    return o.any_sign ? solve_kernel_of<true, kAnySigns>(precision)
+                      : solve_kernel_of<true, kKnownSigns>(precision);
+  return o.any_sign ? solve_kernel_of<false, kAnySigns>(precision)
+                    : solve_kernel_of<false, kKnownSigns>(precision);
 }
 
 struct WarpLaunch {
