@@ -255,15 +255,15 @@ Layout make_layout(const BlobOff& o, int lt_size, bool with_hist, bool with_temp
   L.y = take(vec + sizeof(double));  // y[n]: see set_unit
   L.ftemp = take(vec);
   L.tempv = with_tempv ? take(vec) : -1;
-  // the f scratch (pseudo-rates, then the computed species, a zero and the guarded terms) and
-  // the J scratch (partials, computed species, parameter partials, virtual
-  // slots, a zero and the guarded terms), each followed by the sub-models'
-  // scratch; the solves' vector lies over them
-  const int n_scr = std::max(o.scr0[0], o.scr0[1]) + o.n_sms;
+  // the f scratch (pseudo-rates, then the computed species, a zero and the
+  // guarded terms) and the J scratch (partials, computed species, parameter
+  // partials, virtual slots, a zero and the guarded terms), with the
+  // sub-models' scratch over or behind them; the solves' vector lies over all
+  const int n_scr = std::max(o.scr_end[0], o.scr_end[1]);
   L.rates = L.z = take(std::max(sizeof(double) * n_scr, (size_t)lt_size * (o.n + 1)));
   L.keff = take(sizeof(double) * o.n_keff);
   // the split species' parts lie behind f's terms, over J's where those leave room
-  const int f_end = o.scr0[0] + o.n_sms, n_fscr = 2 * std::max(1, o.n_fscratch);
+  const int f_end = o.scr_end[0], n_fscr = 2 * std::max(1, o.n_fscratch);
   L.fscr = f_end + n_fscr <= n_scr ? L.rates + (int)sizeof(double) * f_end
                                    : take(sizeof(double) * n_fscr);
   // a spare slot: see clear_spare
@@ -745,6 +745,9 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
   o.aq_cp = w.put(aq_cp);
   o.aq_cpm = w.put(aq_cpm);
   // sub-model programs, virtual slots and the chain
+  std::vector<uint32_t> sm_item, sm_scr, sm_pel;
+  std::vector<uint16_t> sm_pq;
+  int sm_slots = 0;
   {
     std::vector<uint32_t> rec;
     std::vector<int32_t> ints;
@@ -763,20 +766,24 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
     for (const SubProgram& g : t.cv) cv_state.push_back(g.state);
     o.sm_state = w.put(u16(cv_state));
     // parallel parts of the programs (blob.hpp)
-    std::vector<uint32_t> item[5], scr, pel, pst;
+    std::vector<uint32_t> item[5];  // by kind
     uint32_t slots = 0;
+    // slots of the pairs' moles, by their ions and factors
+    std::map<std::vector<double>, uint32_t> moles;
     for (size_t c = 0; c < t.cv.size(); ++c) {
       const std::vector<int>& I = t.cv[c].ints;
       const uint32_t i0 = rec[2 * c], f0 = rec[2 * c + 1], cc = (uint32_t)c << 8;
+      auto add = [&](uint32_t kind, uint32_t i, uint32_t f, int n) {
+        for (uint32_t v : {kind | cc, i0 + i, f0 + f, slots}) item[kind].push_back(v);
+        slots += n;
+      };
       const uint32_t s0 = slots;
       if (I[0] == 1) {
         int ii = 3, fi = 0;
         for (int x = 0; x < I[2]; ++x) {
           const int type = I[ii++];
           if (type == 1) {
-            for (uint32_t v : {1u | cc, i0 + (uint32_t)ii, f0 + (uint32_t)fi, slots})
-              item[1].push_back(v);
-            slots += 7;
+            add(1, ii, fi, 7);
             fi += 3 + I[ii + 2];
             ii += 6;
           } else if (type == 2) {
@@ -784,7 +791,7 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
             ii += 2 + 2 * I[ii];
           }
         }
-        for (uint32_t v : {s0, 0u, 0u, 0u}) scr.push_back(v);
+        for (uint32_t v : {s0, 0u, 0u, 0u}) sm_scr.push_back(v);
         continue;
       }
       const int npair = I[2], x = I[3], ninter = I[4];
@@ -792,59 +799,38 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
       const int* it = pr + 5 * npair;
       int fi = 2 * npair;
       for (int k = 0; k < ninter; ++k) {
-        for (uint32_t v : {3u | cc, i0 + 6u + 5u * npair + 2u * k, f0 + (uint32_t)fi, slots})
-          item[3].push_back(v);
-        slots += 3;
+        add(3, 6 + 5 * npair + 2 * k, fi, 3);
         fi += 2 + it[2 * k + 1];
       }
-      const uint32_t p0 = slots;
-      for (int j = 0; j < npair; ++j) {
-        for (uint32_t v : {4u | cc, i0 + 6u + 5u * j, f0 + 2u * j, slots}) item[4].push_back(v);
-        slots += 2;
-      }
-      for (uint32_t v : {s0, (uint32_t)ninter, p0, slots}) scr.push_back(v);
+      std::vector<double> key;
+      for (int j = 0; j < npair; ++j)
+        for (double v : {(double)pr[5 * j], (double)pr[5 * j + 1], t.cv[c].flts[2 * j],
+                         t.cv[c].flts[2 * j + 1]})
+          key.push_back(v);
+      const auto at = moles.insert({key, slots});
+      if (at.second)
+        for (int j = 0; j < npair; ++j) add(4, 6 + 5 * j, 2 * j, 2);
+      for (uint32_t v : {s0, (uint32_t)ninter, at.first->second, slots}) sm_scr.push_back(v);
       slots += 2;
-      // every partial of this coefficient with its terms in the order of the
-      // interactions: the direct ones, then those through omega
+      // every partial of this coefficient, with the other pairs whose cation or
+      // anion it is against
       std::vector<int> ids{I[5]};
       for (int j = 0; j < npair; ++j)
         for (int a : {pr[5 * j + 3], pr[5 * j + 4]})
           if (std::find(ids.begin(), ids.end(), a) == ids.end()) ids.push_back(a);
       for (int id : ids) {
-        pel.push_back((uint32_t)id | ((uint32_t)c << 16));
-        pel.push_back((uint32_t)pst.size() / 2);
-        auto step = [&](uint32_t kind, int k, int j, int q) {
-          pst.push_back(kind | ((uint32_t)k << 4));
-          pst.push_back((uint32_t)j | ((uint32_t)q << 16));
-        };
-        for (int k = 0; k < ninter; ++k) {
-          const int j = it[2 * k];
-          if (j == x) {
-            if (id == I[5]) step(0, k, j, 0);
-            continue;
-          }
-          if (id == pr[5 * j + 3]) step(2, k, j, 0);
-          if (id == pr[5 * j + 4]) step(3, k, j, 0);
-          if (id == I[5]) step(1, k, j, 0);
-          for (int q = 0; q < npair; ++q) {
-            if (q == x) continue;
-            if (id == pr[5 * q + 3]) step(4, k, j, q);
-            if (id == pr[5 * q + 4]) step(5, k, j, q);
-          }
+        const size_t q0 = sm_pq.size();
+        for (int q = 0; q < npair; ++q) {
+          if (q == x) continue;
+          if (id == pr[5 * q + 3]) sm_pq.push_back((uint16_t)q);
+          if (id == pr[5 * q + 4]) sm_pq.push_back((uint16_t)(q | 0x8000));
         }
+        sm_pel.push_back((uint32_t)id | ((uint32_t)c << 16));
+        sm_pel.push_back((uint32_t)q0 | ((uint32_t)(sm_pq.size() - q0) << 16));
       }
     }
-    o.n_smp = (int)pel.size() / 2;
-    pel.push_back(0);
-    pel.push_back((uint32_t)pst.size() / 2);
-    std::vector<uint32_t> items;
-    for (int kind : {1, 3, 4}) items.insert(items.end(), item[kind].begin(), item[kind].end());
-    o.n_smi = (int)items.size() / 4;
-    o.sm_item = w.put(items);
-    o.sm_scr = w.put(scr);
-    o.sm_pel = w.put(pel);
-    o.sm_pst = w.put(pst);
-    o.n_sms = (int)slots;
+    for (int kind : {1, 3, 4}) sm_item.insert(sm_item.end(), item[kind].begin(), item[kind].end());
+    sm_slots = (int)slots;
     o.sm_int = w.put(ints);
     o.sm_flt = w.put(flts);
     o.n_virt = t.n_virt;
@@ -909,16 +895,48 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
     q->jg_slots = v.put(jg_slots);
     q->jg_umid = v.put(jg_umid);
   };
+  auto put_parts = [&](auto& v, BlobOff* q) {
+    q->n_smi = (int)sm_item.size() / 4;
+    q->n_smp = (int)sm_pel.size() / 2;
+    q->n_sms = sm_slots;
+    q->sm_item = v.put(sm_item);
+    q->sm_scr = v.put(sm_scr);
+    q->sm_pel = v.put(sm_pel);
+    q->sm_pq = v.put(sm_pq);
+  };
   for (int k = 0; k < 2; ++k) o.g[k].zero = k == 0 ? f_zero : j_zero;
-  // cells per block (FP64, all in shared memory) with the given gathers staged
-  auto cells = [&](bool any) {
+  // The sub-models' scratch lies over the pseudo-rates (f) and partials (J),
+  // which are computed after them, or, where it does not fit there, behind the
+  // rest.
+  auto place_scratch = [&](BlobOff* q) {
+    const bool over = q->n_sms <= std::min(t.n_rates, t.n_part_all);
+    for (int k = 0; k < 2; ++k) {
+      const int end = q->g[k].zero + 1 + q->g[k].n_neg;
+      q->scr0[k] = over ? 0 : end;
+      q->scr_end[k] = over ? end : end + q->n_sms;
+    }
+  };
+  // cells per block (FP64, all in shared memory) with the given tables staged
+  auto cells = [&](bool any, bool parts) {
     BlobOff q = o;
     Sizer v{w.buf.size()};
+    if (parts) put_parts(v, &q);
     any ? put_any(v, &q) : put_known(v, &q);
-    for (int k = 0; k < 2; ++k) q.scr0[k] = q.g[k].zero + 1 + q.g[k].n_neg;
+    place_scratch(&q);
     const int room = max_smem - (int)((v.at + 127) & ~size_t(127));
     return std::max(0, room / make_layout(q, 8, true, false).bytes);
   };
+  // The parts of the sub-models' programs over the lanes, unless their tables and
+  // scratch cost a quarter of the cells (4 000 cells of one phase in
+  // several modes, FP64, cells and ms of the parts / a lane per program: 4 ion
+  // pairs x 16 modes 3 / 4, 7.6 / 6.0; 9 x 4 5 / 8, 3.9 / 3.5; 9 x 8 1 / 2,
+  // 26.8 / 12.8; 20 x 1 6 / 14, 2.52 / 2.59; 9 x 2 12 / 20, 2.00 / 2.20; the
+  // shipped mod37 configuration 5 / 5, 214 / 241).
+  if (sm_pq.size() <= 65535 && !t.cv.empty()) {
+    const int parts = cells(false, true);
+    if (parts >= kEnoughCells || 4 * parts > 3 * std::min(cells(false, false), kEnoughCells))
+      put_parts(w, &o);
+  }
   // A guarded term takes eight bytes of every cell's slab beside its table
   // entry, so a mechanism with many of them holds fewer cells, or none at all,
   // with the known-sign gathers staged; it keeps the gathers for any signs
@@ -935,12 +953,12 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
   if (!fits) {
     o.any_sign = 1;
   } else if (guards) {
-    const int known = cells(false);
-    const int any = known < kEnoughCells ? std::min(cells(true), kEnoughCells) : 0;
+    const int known = cells(false, false);
+    const int any = known < kEnoughCells ? std::min(cells(true, false), kEnoughCells) : 0;
     o.any_sign = any > 0 && 4 * known <= 3 * any;
   }
   o.any_sign ? put_any(w, &o) : put_known(w, &o);
-  for (int k = 0; k < 2; ++k) o.scr0[k] = o.g[k].zero + 1 + o.g[k].n_neg;
+  place_scratch(&o);
   // the level-scheduled mode stages only the bytes up to here into shared
   // memory, the one-lane LU mode its LU tables too; the gathers for any signs,
   // where they are the exception, come last and stay in global memory

@@ -114,18 +114,19 @@ struct BlobOff {
   // parameter partials and the virtual slots after the values.
   int n_cv, n_pj, sm_keff, sm_rec, sm_int, sm_flt;
   int sm_state;  // state index of each computed species (uint16)
-  // their parallel parts: n_smi items (sm_item, uint32 x 4: kind | computed
-  // species<<8, first int, first float, scratch slot), kind 1 a Jacobson pair
-  // of ZSR (7 slots: the water's factor, then factor and multiplier of its
-  // three partials), kind 3 a PD-FiTE interaction (slots li, dli, in range),
-  // kind 4 a PD-FiTE pair (slots its cation's and anion's moles); per computed
-  // species sm_scr (uint32 x 4: first slot; PD-FiTE: interactions, slot of the
-  // first pair, slot of gamma and 1 / omega).  PD-FiTE's partials: n_smp
-  // elements, sm_pel (uint32 x 2: parameter id | computed species<<16, first
-  // step; one more at the end) and their steps in order, sm_pst (uint32 x 2:
-  // kind | interaction<<4, interaction's pair | pair<<16).  The scratch of
-  // n_sms slots lies at scr0[0] (f) or scr0[1] (J) of the f / J scratch.
-  int n_smi, sm_item, sm_scr, n_smp, sm_pel, sm_pst, n_sms, scr0[2];
+  // their parallel parts (n_smi 0: none, a lane per computed species): n_smi
+  // items (sm_item, uint32 x 4: kind | computed species<<8, first int, first
+  // float, scratch slot), kind 1 a Jacobson pair of ZSR (7 slots: the water's
+  // factor, then factor and multiplier of its three partials), kind 3 a PD-FiTE
+  // interaction (slots li, dli, in range), kind 4 a PD-FiTE pair (slots its
+  // cation's and anion's moles; shared by the coefficients of a phase); per
+  // computed species sm_scr (uint32 x 4: first slot; PD-FiTE: interactions, slot
+  // of the first pair, slot of gamma and 1 / omega).  PD-FiTE's partials: n_smp
+  // elements, sm_pel (uint32 x 2: parameter id | computed species<<16, first |
+  // count<<16 of the other pairs, in order, whose cation or anion it is
+  // against), sm_pq (uint16: pair | anion<<15).  The scratch of n_sms slots lies
+  // at scr0[0] (f) or scr0[1] (J) of the f / J scratch, which end at scr_end.
+  int n_smi, sm_item, sm_scr, n_smp, sm_pel, sm_pq, n_sms, scr0[2], scr_end[2];
   // virtual Jacobian slots: partial lists (uint16 pointers, n_virt + 1, and
   // uint16 partial indices); the chain by target slot: target (uint16),
   // entry pointers (uint16, n_chain + 1), entries (uint32: virtual slot |

@@ -51,7 +51,6 @@ constexpr int kMaxCellsAero = 8;  // cells per block of the aerosol form
 
 struct SolveArgs {
   DevMech m;
-  BlobOff off;
   const void* blob;  // table blob in global memory (copied to shared)
   int tab_bytes;     // shared-memory bytes reserved for the tables
   int stage_bytes;   // blob bytes staged into them
@@ -71,6 +70,9 @@ struct SolveArgs {
   double t0, t1, rtol;
   int max_steps, maxncf, maxnef;
   int lu_mode;
+  // last, as its size would shift the other arguments by 8 bytes, which decides
+  // how the compiler loads them (cb05, 100 000 cells mixed: 122.1 or 124.3 ms)
+  BlobOff off;
 };
 
 // ---------------------------------------------------------------------------
@@ -331,10 +333,8 @@ __device__ __forceinline__ bool rates_of(const Tab& t, const double* y, const do
 // first every Jacobson pair of ZSR and every interaction and pair of PD-FiTE
 // (their exponentials, polynomials and moles), then the sums, one lane per
 // computed species, then PD-FiTE's partials, one lane per element.  Each sum
-// keeps its terms' order.  With one lane per computed species alone, ZSR and
-// PD-FiTE ran one after the other, 5 of 32 lanes at work (f of the shipped
-// mod37 configuration: 14 600 of its 25 700 cycles; its Jacobian: 38 100 of
-// 70 200).
+// keeps its terms' order.  A lane per computed species alone leaves 27 of the
+// shipped mod37 configuration's 32 lanes idle through chains of exponentials.
 //
 // ZSR aerosol water of one phase instance
 // (src/sub_models/sub_model_ZSR_aerosol_water.c:225-305, Jacobian :318-437).
@@ -374,7 +374,8 @@ __device__ __forceinline__ void zsr_pair(const int* I, const double* F, const do
     s[6] = fc;
   }
 }
-template <bool PJ>
+// PAR: with the pairs' slots s filled before
+template <bool PJ, bool PAR>
 __device__ __forceinline__ double zsr_water(const int* I, const double* F, const double* y,
                                             double ppm, const double* s, double* P) {
   const double a_w = ppm * state_of(y[I[1]]);
@@ -385,13 +386,18 @@ __device__ __forceinline__ double zsr_water(const int* I, const double* F, const
   for (int x = 0; x < npair; ++x) {
     const int type = I[ii++];
     if (type == 1) {
+      double own[7];
+      if constexpr (!PAR) {
+        zsr_pair<PJ>(I + ii, F + fi, y, a_w, ppm, own);
+        s = own;
+      }
       W += s[0] * 1000.0;
       if constexpr (PJ) {
         P[I[ii + 3]] += s[1] * s[2];
         P[I[ii + 5]] += s[3] * s[4];
         P[I[ii + 4]] += s[5] * s[6];
       }
-      s += 7;
+      if constexpr (PAR) s += 7;
       fi += 3 + I[ii + 2];
       ii += 6;
     } else if (type == 2) {  // EQSAM (Metzger et al., 2002)
@@ -427,6 +433,23 @@ __device__ __forceinline__ double zsr_water(const int* I, const double* F, const
   return W;
 }
 
+// PD-FiTE's polynomial of one interaction (it: pair, B count; F: min RH, max
+// RH, B...) and its derivative in the gas water; whether the RH is in range
+template <bool PJ>
+__device__ __forceinline__ bool pdfite_inter(const int* it, const double* F, double a_w,
+                                             double ppm, double* li, double* dli) {
+  const double lo = F[0], hi = F[1];
+  double l = 0.0, d = 0.0;
+  #pragma unroll 1
+  for (int z = it[1] - 1; z >= 0; --z) {
+    if (PJ) d = d * a_w + l;
+    l = l * a_w + F[2 + z];
+  }
+  *li = l;
+  if (PJ) *dli = d * ppm;
+  return !((a_w <= lo || a_w > hi) && !(a_w <= 0.0 && lo <= 0.0));
+}
+
 // PD-FiTE activity coefficient of one ion pair in one phase instance
 // (src/sub_models/sub_model_PDFiTE.c:167-259, Jacobian :273-432; Topping et
 // al. 2009, eq. 15).  Moles per concentration and the partials' factors are the
@@ -459,8 +482,67 @@ __device__ __forceinline__ double pdfite_gamma(const int* I, const double* si, c
   return g;
 }
 
-// Every computed species into cv, with scr the programs' scratch; PJ: also the
-// parameter Jacobian P (zeroed first; element ids index it)
+// The same by one lane from the program alone, with P its partials
+template <bool PJ>
+__device__ __forceinline__ double pdfite_serial(const int* I, const double* F, const double* y,
+                                                double ppm, double* P) {
+  double a_w = ppm * state_of(y[I[1]]);
+  a_w = a_w < 0.0 ? 0.0 : (a_w > 1.0 ? 1.0 : a_w);
+  const int npair = I[2], x = I[3], ninter = I[4], pw = I[5];
+  const int* pr = I + 6;
+  const int* it = pr + 5 * npair;
+  const double* fb = F + 2 * npair;
+  auto cn = [&](int j) { return state_of(y[pr[5 * j]]) * F[2 * j]; };
+  auto an = [&](int j) { return state_of(y[pr[5 * j + 1]]) * F[2 * j + 1]; };
+  double omega = 0.0;
+  #pragma unroll 1
+  for (int j = 0; j < npair; ++j)
+    if (j != x) omega += 2.0 * pr[5 * j + 2] * cn(j) * an(j);
+  const double inv_omega = omega > 0.0 ? __drcp_rn(omega) : 0.0;
+  double lng = 0.0, g = 1.0;
+  // the coefficient, then its partials, which need it
+  #pragma unroll 1
+  for (int pass = 0; pass < (PJ ? 2 : 1); ++pass) {
+    const double* f = fb;
+    #pragma unroll 1
+    for (int k = 0; k < ninter; ++k) {
+      const int j = it[2 * k];
+      double li, dli;
+      const bool in = pdfite_inter<PJ>(it + 2 * k, f, a_w, ppm, &li, &dli);
+      f += 2 + it[2 * k + 1];
+      if (!in) continue;
+      if (pass == 0) {
+        if (j == x)
+          lng += li;
+        else if (omega > 0.0)
+          lng += li * cn(j) * an(j) * inv_omega;
+        continue;
+      }
+      if (j == x) {
+        P[pw] += g * dli;
+      } else if (omega > 0.0) {
+        const double cj = cn(j), aj = an(j);
+        P[pr[5 * j + 3]] += g * li * aj * F[2 * j] * inv_omega;
+        P[pr[5 * j + 4]] += g * li * cj * F[2 * j + 1] * inv_omega;
+        P[pw] += g * cj * aj * inv_omega * dli;
+        const double s = -g * li * cj * aj * inv_omega * inv_omega * 2.0;
+        #pragma unroll 1
+        for (int q = 0; q < npair; ++q) {
+          if (q == x) continue;
+          const double sq = s * pr[5 * q + 2];
+          P[pr[5 * q + 3]] += sq * an(q) * F[2 * q];
+          P[pr[5 * q + 4]] += sq * cn(q) * F[2 * q + 1];
+        }
+      }
+    }
+    if (pass == 0) g = exp(lng);
+  }
+  return g;
+}
+
+// Every computed species into cv; PJ: also the parameter Jacobian P (zeroed
+// first; element ids index it).  The parts over the lanes with scr their
+// scratch, or, where these would cost cells, a lane per computed species.
 template <bool PJ>
 __device__ __noinline__ void sub_model_eval(const double* y, const double* keff, double* cv,
                                             double* P, double* scr, int lane) {
@@ -479,6 +561,18 @@ __device__ __noinline__ void sub_model_eval(const double* y, const double* keff,
   const int* I0 = (const int*)(tb + o.sm_int);
   const double* F0 = (const double*)(tb + o.sm_flt);
   const double ppm = keff[o.sm_keff];
+  if (o.n_smi == 0) {
+    __syncwarp();
+    #pragma unroll 1
+    for (int c = lane; c < o.n_cv; c += 32) {
+      const int* I = I0 + rec[2 * c];
+      const double* F = F0 + rec[2 * c + 1];
+      cv[c] = I[0] == 1 ? zsr_water<PJ, false>(I, F, y, ppm, nullptr, P)
+                        : pdfite_serial<PJ>(I, F, y, ppm, P);
+    }
+    __syncwarp();
+    return;
+  }
   const uint4* item = (const uint4*)(tb + o.sm_item);
   #pragma unroll 1
   for (int e = lane; e < o.n_smi; e += 32) {
@@ -498,17 +592,7 @@ __device__ __noinline__ void sub_model_eval(const double* y, const double* keff,
       continue;
     }
     a_w = a_w < 0.0 ? 0.0 : (a_w > 1.0 ? 1.0 : a_w);
-    const double lo = F[0], hi = F[1];
-    const bool in = !((a_w <= lo || a_w > hi) && !(a_w <= 0.0 && lo <= 0.0));
-    double li = 0.0, dli = 0.0;
-    #pragma unroll 1
-    for (int z = I[1] - 1; z >= 0; --z) {
-      if (PJ) dli = dli * a_w + li;
-      li = li * a_w + F[2 + z];
-    }
-    s[0] = li;
-    if (PJ) s[1] = dli * ppm;
-    s[2] = in ? 1.0 : 0.0;
+    s[2] = pdfite_inter<PJ>(I, F, a_w, ppm, s, s + 1) ? 1.0 : 0.0;
   }
   __syncwarp();
   const uint4* sc = (const uint4*)(tb + o.sm_scr);
@@ -516,49 +600,53 @@ __device__ __noinline__ void sub_model_eval(const double* y, const double* keff,
   for (int c = lane; c < o.n_cv; c += 32) {
     const int* I = I0 + rec[2 * c];
     const uint4 q = sc[c];
-    cv[c] = I[0] == 1 ? zsr_water<PJ>(I, F0 + rec[2 * c + 1], y, ppm, scr + q.x, P)
+    cv[c] = I[0] == 1 ? zsr_water<PJ, true>(I, F0 + rec[2 * c + 1], y, ppm, scr + q.x, P)
                       : pdfite_gamma(I, scr + q.x, scr + q.z, scr + q.w);
   }
   __syncwarp();
   if constexpr (PJ) {
     const uint2* pel = (const uint2*)(tb + o.sm_pel);
-    const uint2* pst = (const uint2*)(tb + o.sm_pst);
     #pragma unroll 1
     for (int e = lane; e < o.n_smp; e += 32) {
       const uint2 w = pel[e];
-      const int c = w.x >> 16, end = pel[e + 1].y;
+      const int id = w.x & 0xFFFFu, c = w.x >> 16, npq = w.y >> 16;
+      const uint16_t* pq = (const uint16_t*)(tb + o.sm_pq) + (w.y & 0xFFFFu);
       const uint4 q = sc[c];
-      const int* pr = I0 + rec[2 * c] + 6;
+      const int* I = I0 + rec[2 * c];
       const double* F = F0 + rec[2 * c + 1];
+      const int x = I[3];
+      const bool water = id == I[5];
+      const int* pr = I + 6;
+      const int* it = pr + 5 * I[2];
       const double *si = scr + q.x, *sp = scr + q.z;
       const double g = scr[q.w], io = scr[q.w + 1];
       double v = 0.0;
       #pragma unroll 1
-      for (int n = w.y; n < end; ++n) {
-        const uint2 st = pst[n];
-        const int kind = st.x & 0xFu, k = st.x >> 4;
-        if (si[3 * k + 2] == 0.0) continue;
-        const double li = si[3 * k], dli = si[3 * k + 1];
-        if (kind == 0) {
-          v += g * dli;
+      for (int k = q.y; k > 0; --k, it += 2, si += 3) {
+        if (si[2] == 0.0) continue;
+        const int j = it[0];
+        const double li = si[0], dli = si[1];
+        if (j == x) {
+          if (water) v += g * dli;
           continue;
         }
         if (io < 0.0) continue;  // no omega
-        const int j = st.y & 0xFFFFu, r = st.y >> 16;
         const double cj = sp[2 * j], aj = sp[2 * j + 1];
-        if (kind == 1) {
+        if (water) {
           v += g * cj * aj * io * dli;
-        } else if (kind == 2) {
-          v += g * li * aj * F[2 * j] * io;
-        } else if (kind == 3) {
-          v += g * li * cj * F[2 * j + 1] * io;
-        } else {
-          const double s = -g * li * cj * aj * io * io * 2.0;
+          continue;
+        }
+        if (id == pr[5 * j + 3]) v += g * li * aj * F[2 * j] * io;
+        if (id == pr[5 * j + 4]) v += g * li * cj * F[2 * j + 1] * io;
+        const double s = -g * li * cj * aj * io * io * 2.0;
+        #pragma unroll 1
+        for (int m = 0; m < npq; ++m) {
+          const int r = pq[m] & 0x7FFF, an = pq[m] >> 15;
           const double sq = s * pr[5 * r + 2];
-          v += sq * sp[2 * r + (kind == 4 ? 1 : 0)] * F[2 * r + (kind == 4 ? 0 : 1)];
+          v += sq * sp[2 * r + 1 - an] * F[2 * r + an];
         }
       }
-      P[w.x & 0xFFFFu] += v;
+      P[id] += v;
     }
     __syncwarp();
   }

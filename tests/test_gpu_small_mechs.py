@@ -142,3 +142,74 @@ def test_guarded_terms_solve(tmp_path, precision):
     x, st, _, status, _ = _run(mech, y, np.zeros((6, 0)), 0.01, precision)
     assert (status == 0).all() and (st["status"] == 0).all()
     assert (x >= 0.0).all() and (x <= y + ATOL).all()
+
+
+# cations, anions, modes: the programs' parts over the lanes (the first two), a
+# lane per program
+INORGANIC = [(2, 2, 1), (3, 3, 2), (4, 5, 1), (3, 3, 6), (4, 5, 2)]
+
+
+def _inorganic(tmp_path, n_cation, n_anion, n_modes):
+    from camp_b200.cells import make_cells
+
+    mech = small_mechs.inorganic(tmp_path, n_cation, n_anion, n_modes)
+    cells = make_cells(mech, 6, 7)
+    cells.state[:, mech.species.index("H2O")] = [1e2, 2e3, 5e3, 1e4, 1.5e4, 2e4]  # ppm
+    return mech, cells
+
+
+@pytest.mark.parametrize("case", INORGANIC)
+def test_ion_pairs_f_and_jacobian(tmp_path, case):
+    """ZSR and PD-FiTE of a phase with many ion pairs: f to 1e-12 of production
+    plus loss; J to 1e-10, as the parameter partials are sums of up to twenty
+    signed terms that cancel before they enter the two parts."""
+    from camp_b200.solver import Solver
+    from oracle.oracle import OracleModel
+
+    mech, cells = _inorganic(tmp_path, *case)
+    s = Solver(mech, 6)
+    s.initialize(abs_tol=np.full(mech.n_state_var, 1e-14), rel_tol=1e-6)
+    s.set_photo_rates(cells.photo_rates)
+    om = OracleModel(mech)
+    f, p, l = s.eval_deriv(cells.state, cells.env, 1.0)
+    j, jp, jl = s.eval_jac(cells.state, cells.env, 1.0)
+    for c in range(6):
+        row = om.rxn_env_row(cells.env[c], cells.photo_rates[c])
+        of, _, _ = om.deriv(cells.state[c], row, 1.0)
+        oj = om.jac(cells.state[c], row, 1.0)
+        assert np.all(np.abs(f[c] - of) <= 1e-12 * (p[c] + l[c]))
+        assert np.all(np.abs(j[c] - oj) <= 1e-10 * (np.abs(jp[c]) + np.abs(jl[c])) + 1e-300)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("case", INORGANIC)
+def test_ion_pairs_solve(tmp_path, case, precision):
+    """The oracle's outcomes and, in FP64, an error against its tight solution
+    of at most ten times its own largest over the cells."""
+    from camp_b200.solver import Solver
+    from oracle.oracle import OracleModel
+
+    mech, cells = _inorganic(tmp_path, *case)
+    atol = np.full(mech.n_state_var, 1e-14)
+    s = Solver(mech, 6)
+    s.initialize(abs_tol=atol, rel_tol=1e-6)
+    s.set_precision(precision)
+    s.set_photo_rates(cells.photo_rates)
+    x = cells.state.copy()
+    s.solve(x, cells.env, 0.0, 10.0)
+    om = OracleModel(mech)
+
+    def oracle(rtol, atol):
+        _, st, _, y = om.solve(cells.state.copy(), cells.env, cells.photo_rates, 0.0, 10.0, rtol,
+                               np.full(mech.n_state_var, atol), max_steps=100000)
+        return st, y
+
+    status, o = oracle(1e-6, 1e-14)
+    tstatus, tight = oracle(1e-9, 1e-17)
+    assert (status == 0).all() and (tstatus == 0).all()
+    assert (s.cell_stats()["status"] == 0).all()
+    if precision == 0:
+        dep = mech.dep_index()
+        scale = 1e-6 * np.abs(tight) + 1e-14
+        eg, ec = (np.max((np.abs(v - tight) / scale)[:, dep]) for v in (x, o))
+        assert eg <= 10.0 * ec

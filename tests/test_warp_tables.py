@@ -40,7 +40,9 @@ class BlobOff(C.Structure):
             "jg_w0 jg_w1 jg_ptr jg_mid jg_lupos jg_row jg_lane jg_slots j_csc jg_slot lu_iperm "
             "lu_diag lu_src fl_hdr fs_rec fb_rec fb_ext n_fwd n_bwd sv_rec sv_ext lu_rowptr "
             "lu_col upd_ptr upd dep_state atol n_simpol n_keff n_rates n_part_all si_rec si_elem "
-            "si_ef n_aq aq_rec aq_sp aq_sm aq_cp aq_cpm aq_sim has_ug jg_umid").split()])
+            "si_ef n_aq aq_rec aq_sp aq_sm aq_cp aq_cpm aq_sim has_ug jg_umid n_cv n_pj sm_keff "
+            "sm_rec sm_int sm_flt sm_state n_smi sm_item sm_scr n_smp sm_pel sm_pq n_sms").split()]
+        + [("scr0", C.c_int * 2), ("scr_end", C.c_int * 2)])
 
 
 class Tables:
@@ -312,3 +314,29 @@ def test_guarded_terms_take_no_cells(tmp_path, n_species, n_rxn, any_sign):
     for at in (o.fg_ent, o.fg_unit, o.fg_lane, o.jg_slot, o.jg_w0, o.jg_w1, o.jg_ptr, o.jg_umid):
         assert (at < o.stage_bytes) == bool(any_sign)
     check_factor_and_solve(t, 13)
+
+
+@pytest.mark.parametrize("n_cation,n_anion,n_modes,parts", [
+    (2, 2, 1, True), (2, 2, 8, True), (3, 3, 2, True), (4, 5, 1, False), (3, 3, 6, False)])
+def test_ion_pairs(tmp_path, n_cation, n_anion, n_modes, parts):
+    """The parts of the sub-models' programs are left out where their tables
+    and scratch would cost cells, and their tables grow with the programs: an
+    item of 16 bytes per interaction and two list entries per ion pair."""
+    t = Tables(small_mechs.inorganic(tmp_path, n_cation, n_anion, n_modes))
+    o, n_pair = t.o, n_cation * n_anion
+    assert (o.n_smi > 0) == parts
+    if parts:
+        n_act = n_modes * n_pair
+        assert o.n_cv == n_act + n_modes
+        assert o.n_smi == n_act * n_pair + 2 * n_modes * n_pair
+        assert o.n_sms == n_act * (3 * n_pair + 2) + n_modes * (7 + 2) * n_pair
+        over = o.n_sms <= min(o.n_rates, o.n_part_all)
+        ends = [g.zero + 1 + g.n_neg for g in o.g]
+        assert list(o.scr0) == ([0, 0] if over else ends)
+        assert list(o.scr_end) == (ends if over else [e + o.n_sms for e in ends])
+        pel = t.arr(o.sm_pel, np.uint32, 2 * o.n_smp)
+        assert o.n_smp == n_act * (1 + n_cation + n_anion)
+        # every pair but the coefficient's own, against its cation and its anion
+        assert (pel[1::2] >> 16).sum() == n_act * 2 * (n_pair - 1)
+    check_factor_and_solve(t, 14)
+    check_gathers(t, 15)
