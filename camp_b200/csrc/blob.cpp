@@ -562,9 +562,11 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
   // Grouped phases as rounds of 32 targets, longest first within a level, so
   // that a round's targets have similar lengths and its padding stays small.
   // Targets of four pairs or more take two lanes, one for each of their
-  // alternating sums, 16 to a round.  Per round its pair count per lane | two
-  // lanes<<15, 32 records (first pair, target, pivot or finish mark) and its
-  // further pairs.
+  // alternating sums, 16 to a round.  Per round its pair count per lane (two
+  // lanes: | lanes in use<<9 | 1<<15), 32 records (first pair,
+  // target, pivot or finish mark) and its further pairs, with two lanes only
+  // those of the lanes in use: a hub species' target has hundreds, and 32 words
+  // for each pair of lanes filled 75 KB for 400 species around one.
   struct Rounds {
     std::vector<uint32_t> pair0, target, recip, ext;
     std::vector<int> cnt, level;
@@ -579,28 +581,36 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
         return g.unit_count[a] > g.unit_count[b];
       });
       for (size_t k0 = 0; k0 < us.size();) {
-        const bool two = g.unit_count[us[k0]] >= 4;
+        const int most = std::max(1, g.unit_count[us[k0]]);
+        const bool two = most >= 4;
+        // a round of very long targets leaves those of less than half their
+        // length to the next, which would be padding otherwise
+        size_t m = std::min(us.size() - k0, (size_t)(two ? kLanes / 2 : kLanes));
+        if (most >= 64)
+          while (2 * g.unit_count[us[k0 + m - 1]] < most) --m;
+        int row = two ? 2 : kLanes;  // lanes with a table word of their own
+        while (two && row < 2 * (int)m) row *= 2;
         auto pair = [&](size_t lane, int j) {
-          const size_t k = k0 + (two ? lane / 2 : lane);
+          const size_t k = two ? lane / 2 : lane;
           const int at = two ? 2 * j + (int)(lane & 1) : j;
-          if (k >= us.size() || at >= g.unit_count[us[k]]) return no_pair;
-          const int p = g.unit_begin[us[k]] + at;
+          if (k >= m || at >= g.unit_count[us[k0 + k]]) return no_pair;
+          const int p = g.unit_begin[us[k0 + k]] + at;
           return (uint32_t)g.pair_a[p] | ((uint32_t)g.pair_b[p] << 16);
         };
-        const int most = std::max(1, g.unit_count[us[k0]]);
         const int cnt = two ? (most + 1) / 2 : most;
-        o->cnt.push_back(cnt | (two ? 0x8000 : 0));
+        o->cnt.push_back(two ? 0x8000 | (row << 9) | cnt : cnt);
         o->level.push_back(l);
         for (size_t lane = 0; lane < kLanes; ++lane) {
-          const size_t k = k0 + (two ? lane / 2 : lane);
-          const bool real = k < us.size() && !(two && (lane & 1));
+          const size_t k = two ? lane / 2 : lane;
+          const bool real = k < m && !(two && (lane & 1));
           o->pair0.push_back(pair(lane, 0));
-          o->target.push_back(real ? (uint32_t)g.unit_target[us[k]] : (uint32_t)spare);
-          o->recip.push_back(real ? (uint32_t)g.unit_recip[us[k]] : 0u);
+          o->target.push_back(real ? (uint32_t)g.unit_target[us[k0 + k]] : (uint32_t)spare);
+          o->recip.push_back(real ? (uint32_t)g.unit_recip[us[k0 + k]] : 0u);
         }
         for (int j = 1; j < cnt; ++j)
-          for (size_t lane = 0; lane < kLanes; ++lane) o->ext.push_back(pair(lane, j));
-        k0 += two ? kLanes / 2 : kLanes;
+          for (size_t lane = 0; lane < (size_t)row; ++lane)
+            o->ext.push_back(pair(lane, j));
+        k0 += m;
       }
     }
   };

@@ -72,7 +72,8 @@ struct BlobOff {
   // round's largest, the same in every lane: shorter targets and idle lanes are
   // padded with the spare slot LU[n_lu] = 0.  Bit 15 of cnt: a round of targets
   // of four pairs or more on two neighbouring lanes each, one of the two
-  // alternating sums per lane.
+  // alternating sums per lane; bits 10 to 14 are then half of the lanes in use (a
+  // power of two), which are the words of a step in fb_ext.
   int fl_hdr, fs_rec, fb_rec, fb_ext;
   // triangular solves: n_fwd rounds forward, then n_bwd backward.  A round
   // gives every lane one target z[tgt] -= sum LU[a] z[x] (backward: then times

@@ -1476,16 +1476,17 @@ __device__ __forceinline__ LT more_pairs(LT s, uint32_t c, const LT* LU, const L
                                          const uint32_t** ext, int lane) {
   const uint32_t* e = *ext;
   if (c & 0x8000u) {
+    const int row = c >> 9 & 62;  // lanes in use; the others read on, their sums are dropped
     uint32_t q = *e;
     #pragma unroll 1
-    for (int k = c & 0x7FFFu; k > 1; --k) {
-      e += 32;
+    for (int k = c & 0x3FFu; k > 1; --k) {
+      e += row;
       const LT a = LU[q & 0xFFFFu], b = x[q >> 16];
       q = *e;
       s -= a * b;
     }
     s += __shfl_xor_sync(FULLMASK, s, 1);
-    if (lane & 1) s = (LT)0;
+    if (lane & (1 | -row)) s = (LT)0;
   } else {
     LT s1 = (LT)0;
     s1 -= LU[e[0] & 0xFFFFu] * x[e[0] >> 16];

@@ -77,7 +77,7 @@ def test_chain_conserves_its_total(tmp_path, n_species, reverse):
 
 
 @pytest.mark.parametrize("negative", [False, True])
-@pytest.mark.parametrize("n_species", [10, 41, 90])
+@pytest.mark.parametrize("n_species", [10, 41, 90, 400])
 def test_hub_f_and_jacobian(tmp_path, n_species, negative):
     """Long lists and guarded terms: f and J against the oracle's to 1e-12 of
     production plus loss, as on the packed mechanisms.  Half of the cells
@@ -213,3 +213,25 @@ def test_ion_pairs_solve(tmp_path, case, precision):
         scale = 1e-6 * np.abs(tight) + 1e-14
         eg, ec = (np.max((np.abs(v - tight) / scale)[:, dep]) for v in (x, o))
         assert eg <= 10.0 * ec
+
+
+@pytest.mark.parametrize("n_species", [41, 300])
+def test_hub_solve(tmp_path, n_species):
+    """Targets of hundreds of pairs (two lanes of each round in use) in the
+    factorization and solves: the oracle's outcomes and values to a hundred
+    times the tolerance (two runs at rtol 1e-6 each with its global error)."""
+    from camp_b200.solver import Solver
+    from oracle.oracle import OracleModel
+
+    mech = small_mechs.hub(tmp_path, n_species)
+    y = np.random.default_rng(6).uniform(0.1, 1.0, (6, n_species))
+    env = np.tile(np.array([298.0, 1.0e5]), (6, 1))
+    atol = np.full(n_species, 1e-12)
+    s = Solver(mech, 6)
+    s.initialize(abs_tol=atol, rel_tol=1e-6)
+    x = y.copy()
+    s.solve(x, env, 0.0, 10.0)
+    _, status, _, o = OracleModel(mech).solve(y.copy(), env, np.zeros((6, 0)), 0.0, 10.0, 1e-6,
+                                              atol)
+    assert (status == 0).all() and (s.cell_stats()["status"] == 0).all()
+    assert (np.abs(x - o) <= 1e-4 * np.abs(o) + 1e-10).all()

@@ -76,19 +76,21 @@ def pair_round(rec, ext, A, X, spare):
     a, x = w0 & 0xFFFF, w0 >> 16
     cnt = w1 >> 16
     assert (cnt == cnt[0]).all()
-    two, c = bool(cnt[0] & 0x8000), int(cnt[0] & 0x7FFF)
+    two = bool(cnt[0] & 0x8000)
+    c, row = (cnt[0] & 0x3FF, cnt[0] >> 9 & 62) if two else (cnt[0], LANES)
+    lanes = np.arange(LANES)
     tgt = w1 & 0x7FFF if spare < 0x8000 else w1 & 0xFFFF
     s = X[tgt] - A[a] * X[x]
     for k in range(c - 1):
-        q = ext[LANES * k:LANES * (k + 1)]
+        q = ext[row * k + lanes]  # idle lanes read on
         s = s - A[q & 0xFFFF] * X[q >> 16]
     if two:
-        s = np.where(np.arange(LANES) % 2 == 0, s + s[np.arange(LANES) ^ 1], 0.0)
-        assert (tgt[1::2] == spare).all()
+        s = np.where((lanes % 2 == 0) & (lanes < row), s + s[lanes ^ 1], 0.0)
+        assert (tgt[1::2] == spare).all() and (tgt[row:] == spare).all()
     assert (s[tgt == spare] == 0.0).all()
     real = tgt[tgt != spare]
     assert len(np.unique(real)) == len(real)
-    return tgt, s, LANES * (c - 1)
+    return tgt, s, int(row * (c - 1))
 
 
 def factor(t, LU):
@@ -276,7 +278,7 @@ def test_chain(tmp_path, n, reverse):
 
 
 @pytest.mark.parametrize("negative", [False, True])
-@pytest.mark.parametrize("n", [10, 41, 90])
+@pytest.mark.parametrize("n", [10, 41, 90, 300])
 def test_hub(tmp_path, n, negative):
     """Long lists (a lane per chain), long targets (two lanes each), guarded
     terms."""
@@ -285,7 +287,11 @@ def test_hub(tmp_path, n, negative):
     assert n < 41 or g[1].n_a > 0
     assert (g[0].n_neg > 0) == negative and (g[1].n_neg > 0) == negative
     cnt = t.words(t.o.sv_rec)[1:64 * (t.o.n_fwd + t.o.n_bwd):64] >> 16
-    assert (cnt & 0x8000).any()
+    two = cnt[cnt & 0x8000 != 0]
+    assert len(two)
+    # a row of further pairs has a word per lane in use: few for the hub's own
+    if n == 300:
+        assert (two & 0x3FF).max() > 64 and ((two[(two & 0x3FF) > 64] >> 9 & 62) <= 4).all()
     check_factor_and_solve(t, 9)
     check_gathers(t, 10)
 
