@@ -15,7 +15,6 @@ namespace {
 
 constexpr int kLanes = 32;
 constexpr uint16_t kNoSlot = 0xFFFF;
-constexpr int kEnoughCells = 8;  // cells per block beyond which more gain little
 
 struct Writer {
   std::vector<uint8_t> buf;
@@ -927,6 +926,8 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
     }
   };
   // cells per block (FP64, all in shared memory) with the given tables staged
+  const int most_cells =
+      t.n_simpol > 0 || t.n_aq > 0 || t.n_cv > 0 ? kMaxCellsAero : kMaxCellsPerBlock;
   auto cells = [&](bool any, bool parts) {
     BlobOff q = o;
     Sizer v{w.buf.size()};
@@ -934,7 +935,7 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
     any ? put_any(v, &q) : put_known(v, &q);
     place_scratch(&q);
     const int room = max_smem - (int)((v.at + 127) & ~size_t(127));
-    return std::max(0, room / make_layout(q, 8, true, false).bytes);
+    return std::min(std::max(0, room / make_layout(q, 8, true, false).bytes), most_cells);
   };
   // The parts of the sub-models' programs over the lanes, unless their tables and
   // scratch cost a quarter of the cells (4 000 cells of one phase in
@@ -944,19 +945,17 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
   // shipped mod37 configuration 5 / 5, 214 / 241).
   if (sm_pq.size() <= 65535 && !t.cv.empty()) {
     const int parts = cells(false, true);
-    if (parts >= kEnoughCells || 4 * parts > 3 * std::min(cells(false, false), kEnoughCells))
-      put_parts(w, &o);
+    if (parts == most_cells || 4 * parts > 3 * cells(false, false)) put_parts(w, &o);
   }
   // A guarded term takes eight bytes of every cell's slab beside its table
   // entry, so a mechanism with many of them holds fewer cells, or none at all,
   // with the known-sign gathers staged; it keeps the gathers for any signs
-  // where those hold a third more cells (1 500 cells of random mechanisms,
+  // where those hold a fifth more cells (1 500 cells of random mechanisms,
   // FP64, cells and ms of known / any signs: 20 species x 300 reactions, all
   // yields negative, 3 / 12 cells 111 / 37 ms; 15 x 600 1 / 7, 372 / 72;
-  // 40 x 100, half negative, 3 / 4, 131 / 110; 15 x 300 6 / 16, 51 / 47; with
-  // as many cells known signs are 0.99 to 1.8 times as fast (cb05 1.11, mod37
-  // gas 1.18), and beyond eight cells a block gains little: instruction fetch
-  // bounds it).
+  // 40 x 100, half negative, 3 / 4, 131 / 110; 15 x 300 6 / 12, 51 / 47; 20 x
+  // 100 10 / 12, 42 / 27; with as many cells known signs are 0.99 to 1.8 times as
+  // fast, cb05 1.11, mod37 gas 1.18).
   const bool fits = fgt.a_ent.size() <= 65535 && jgt.a_ent.size() <= 65535 &&
                     f_zero + fgt.neg.size() / 2 <= 65535 && j_zero + jgt.neg.size() / 2 <= 65535;
   const bool guards = !fgt.neg.empty() || !jgt.neg.empty();
@@ -964,8 +963,8 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
     o.any_sign = 1;
   } else if (guards) {
     const int known = cells(false, false);
-    const int any = known < kEnoughCells ? std::min(cells(true, false), kEnoughCells) : 0;
-    o.any_sign = any > 0 && 4 * known <= 3 * any;
+    const int any = known < most_cells ? cells(true, false) : 0;
+    o.any_sign = any > 0 && 6 * known <= 5 * any;
   }
   o.any_sign ? put_any(w, &o) : put_known(w, &o);
   place_scratch(&o);

@@ -136,6 +136,10 @@ struct BlobOff {
 };
 
 constexpr int kBlobHeader = 512;
+// Cells (warps) per block of the solve kernel: its launch bound leaves 168
+// registers per thread, enough to keep the BDF state without spilling.
+constexpr int kMaxCellsPerBlock = 12;
+constexpr int kMaxCellsAero = 8;  // cells per block of the aerosol form
 constexpr int kBlockSmem = 232448;  // the most shared memory of a block on sm_100a
 
 struct Tables;

@@ -44,11 +44,6 @@ constexpr int DO_ERROR_TEST = 100, PREDICT_AGAIN = 101, TRY_AGAIN = 102;
 // ---------------------------------------------------------------------------
 // Device tables
 // ---------------------------------------------------------------------------
-// Cells (warps) per block of the solve kernel: its launch bound leaves 168
-// registers per thread, enough to keep the BDF state without spilling.
-constexpr int kMaxCellsPerBlock = 12;
-constexpr int kMaxCellsAero = 8;  // cells per block of the aerosol form
-
 struct SolveArgs {
   DevMech m;
   const void* blob;  // table blob in global memory (copied to shared)
