@@ -1314,9 +1314,10 @@ __device__ __noinline__ int dev_jac_any(const double* y, double h, const double*
 // Returns 1 (recoverable) when some y < -SMALL.
 //
 // As in dev_f, nearly every call has no negative or non-finite partial,
-// concentration or step: then a product with a non-negative yield always
-// passes its guard; anything else takes dev_jac_any, with the sums in the same
-// order.
+// no negative concentration and a step above zero: then a product with a
+// non-negative yield always passes its guard (at a step of zero an infinite
+// concentration makes the guard NaN, which drops it); anything else takes
+// dev_jac_any, with the sums in the same order.
 template <typename JT, bool EV = false, int FORM = kEither>
 __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
                                     const double* keff, double* part, JT* Jout, int lane, int flags,
@@ -1330,7 +1331,7 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
   if (FORM == kAnySigns || (FORM == kEither && o.any_sign))
     return dev_jac_any<JT, true>(y, h, keff, part, Jout, lane, EV ? csc : nullptr,
                                  EV ? jp : nullptr, EV ? jl : nullptr);
-  bool odd = flags != 0 || !(h >= 0.0);
+  bool odd = flags != 0 || !(h > 0.0);
   const int n_rxn = o.n_rxn;
   // d rate / d y_k for every variable reactant occurrence k
   const uint32_t* rx_word = (const uint32_t*)(tb + o.rx_word);

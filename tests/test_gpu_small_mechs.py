@@ -235,3 +235,23 @@ def test_hub_solve(tmp_path, n_species):
                                               atol)
     assert (status == 0).all() and (s.cell_stats()["status"] == 0).all()
     assert (np.abs(x - o) <= 1e-4 * np.abs(o) + 1e-10).all()
+
+
+@pytest.mark.parametrize("h", [0.0, 1.0, -1.0])
+def test_jacobian_guard_with_infinite_concentration(tmp_path, h):
+    """The guard -rate * yield * h <= y is NaN for an infinite concentration at
+    a step of zero and then drops the product, as in the oracle: equal values
+    (small whole sums, no rounding)."""
+    from camp_b200.solver import Solver
+    from oracle.oracle import OracleModel
+
+    mech = small_mechs.chain(tmp_path, 33, k=0.5)
+    y = np.ones((4, 33))
+    y[1, 0], y[2, 7], y[3, :] = np.inf, np.inf, 0.0
+    env = np.tile(np.array([298.0, 1.0e5]), (4, 1))
+    s = Solver(mech, 4)
+    s.initialize(abs_tol=np.full(33, ATOL), rel_tol=RTOL)
+    j = s.eval_jac(y, env, h)[0]
+    om = OracleModel(mech)
+    row = om.rxn_env_row(env[0], np.zeros(0))
+    assert np.array_equal(j, np.stack([om.jac(y[c], row, h) for c in range(4)]))
