@@ -138,11 +138,10 @@ __device__ __forceinline__ void set_unit(double* y, int n, int lane) {
 // solve kernel is bound by instruction fetch (a warp per cell, each at its own
 // point of the BDF control flow), so compact code beats unrolled code here.
 
-// one out-of-line copy each of pow, division and square root for the BDF
-// control code (IEEE results, identical to the inline forms)
+// one out-of-line copy each of pow and division for the BDF control code (IEEE
+// results, identical to the inline forms)
 __device__ __noinline__ double dpow(double x, double y) { return pow(x, y); }
 __device__ __noinline__ double ddiv(double a, double b) { return a / b; }
-__device__ __noinline__ double dsqrt(double a) { return sqrt(a); }
 
 // step size ratio 1 / (x^(1/k) + ADDON)
 __device__ __noinline__ double step_ratio(double x, int k);
@@ -254,8 +253,9 @@ __device__ __forceinline__ Tab make_tab(const char* b) {
 }
 
 // Copies the table blob into the front of the block's shared memory with one
-// bulk (TMA) copy completed on an mbarrier.  The wait is bounded: a copy of
-// at most 64 KB from this GPU's memory completes in microseconds, and the
+// bulk (TMA) copy completed on an mbarrier (at most the block's 227 KB of shared
+// memory, well below an mbarrier's 2^20 - 1 bytes).  The wait is bounded: such a
+// copy from this GPU's memory completes in microseconds, and the
 // first limit (2^24 polls, each suspending in try_wait) is seconds.  On
 // timeout the block records the error flag that the host reads after the
 // launch, then waits again for its own copy, with a four times longer limit,
@@ -689,7 +689,7 @@ __device__ __forceinline__ SimpolState simpol_state(const Tab& t, int k, const d
 
 // the four pseudo-rates per instance; returns (warp-uniform) whether any is
 // negative
-__device__ __noinline__ bool simpol_rates(const char* tb, const double* y, const double* keff,
+__device__ __noinline__ bool simpol_rates(const double* y, const double* keff,
                                           const double* cv, double* rates, int lane) {
   y = sh(y);
   keff = sh(keff);
@@ -715,7 +715,7 @@ __device__ __noinline__ bool simpol_rates(const char* tb, const double* y, const
 // row's production and loss and the aerosol row's loss and production; an
 // HL instance whose water a sub-model computes adds the gas and aerosol
 // rows against that water (src/rxns/rxn_HL_phase_transfer.c:383-404)
-__device__ __noinline__ void simpol_partials(const char* tb, const double* y, const double* keff,
+__device__ __noinline__ void simpol_partials(const double* y, const double* keff,
                                              const double* cv, double* part, int lane) {
   y = sh(y);
   keff = sh(keff);
@@ -811,7 +811,7 @@ __device__ __forceinline__ void aq_fr(const Tab& t, const uint16_t* rec, const d
 // per dependent slot a loss and a gain pseudo-rate: a reactant loses
 // rf / m and gains rr / m, a product the reverse; returns (warp-uniform)
 // whether any is negative
-__device__ __noinline__ bool aq_rates(const char* tb, const double* y, const double* keff,
+__device__ __noinline__ bool aq_rates(const double* y, const double* keff,
                                       const double* cv, double* rates, int lane) {
   y = sh(y);
   keff = sh(keff);
@@ -843,7 +843,7 @@ __device__ __noinline__ bool aq_rates(const char* tb, const double* y, const dou
 // sub-model computes, each row slot against it, and for a computed
 // activity coefficient each row slot against that
 // (src/rxns/rxn_aqueous_equilibrium.c:486-537).
-__device__ __noinline__ void aq_partials(const char* tb, const double* y, const double* keff,
+__device__ __noinline__ void aq_partials(const double* y, const double* keff,
                                          const double* cv, double* part, int lane) {
   y = sh(y);
   keff = sh(keff);
@@ -903,21 +903,22 @@ __device__ __noinline__ void aq_partials(const char* tb, const double* y, const 
 // Both aerosol passes behind one call, so that the wrappers below keep a
 // single call site each (the solve kernel's register allocation follows
 // them).
-__device__ __noinline__ bool aero_rates(const char* tb, const double* y, const double* keff,
+__device__ __noinline__ bool aero_rates(const double* y, const double* keff,
                                         const double* cv, double* rates, int lane) {
-  const bool neg = simpol_rates(tb, y, keff, cv, rates, lane);
-  return aq_rates(tb, y, keff, cv, rates, lane) || neg;
+  const bool neg = simpol_rates(y, keff, cv, rates, lane);
+  return aq_rates(y, keff, cv, rates, lane) || neg;
 }
-__device__ __noinline__ void aero_partials(const char* tb, const double* y, const double* keff,
+__device__ __noinline__ void aero_partials(const double* y, const double* keff,
                                            const double* cv, double* part, int lane) {
-  simpol_partials(tb, y, keff, cv, part, lane);
-  aq_partials(tb, y, keff, cv, part, lane);
+  simpol_partials(y, keff, cv, part, lane);
+  aq_partials(y, keff, cv, part, lane);
 }
 
 // the species whose lists were split over several units
 template <bool EV>
-__device__ __forceinline__ void f_combine(const char* tb, const double* fscr, double* out,
+__device__ __forceinline__ void f_combine(const double* fscr, double* out,
                                           int lane, double* rp, double* rl) {
+  const char* const tb = g_smem;
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
   const uint16_t* split = (const uint16_t*)(tb + o.fg_split);
   #pragma unroll 1
@@ -1033,7 +1034,7 @@ __device__ __noinline__ int dev_f_any(const double* y, double h, const double* k
     }
   }
   __syncwarp();
-  f_combine<true>(g_smem, fscr, out, lane, rp, rl);
+  f_combine<true>(fscr, out, lane, rp, rl);
   return 0;
 }
 
@@ -1176,11 +1177,11 @@ __device__ __noinline__ void gather(int k, const double* src, double* out, doubl
 // dev_f_any, which classifies and guards term by term; the sums' order is the
 // same.
 template <typename LT, bool EV = false, int FORM = kEither>
-__device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
+__device__ __noinline__ int dev_f(const double* y, double h,
                                   const double* keff, double* rates, double* fscr,
                                   double* out, int lane, int flags, double* rp = nullptr,
                                   double* rl = nullptr) {
-  tb = g_smem;
+  const char* const tb = g_smem;
   y = sh(y);
   keff = sh(keff);
   rates = sh(rates);
@@ -1220,7 +1221,7 @@ __device__ __noinline__ int dev_f(const char* tb, const double* y, double h,
   __syncwarp();
   gather<LT, EV>(0, rates, out, fscr, nullptr, lane, nullptr, EV ? rp : nullptr,
                  EV ? rl : nullptr);
-  f_combine<EV>(tb, sh(fscr), sh(out), lane, rp, rl);
+  f_combine<EV>(sh(fscr), sh(out), lane, rp, rl);
   return 0;
 }
 
@@ -1319,11 +1320,11 @@ __device__ __noinline__ int dev_jac_any(const double* y, double h, const double*
 // concentration makes the guard NaN, which drops it); anything else takes
 // dev_jac_any, with the sums in the same order.
 template <typename JT, bool EV = false, int FORM = kEither>
-__device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
+__device__ __noinline__ int dev_jac(const double* y, double h,
                                     const double* keff, double* part, JT* Jout, int lane, int flags,
                                     const uint16_t* csc = nullptr, double* jp = nullptr,
                                     double* jl = nullptr) {
-  tb = g_smem;
+  const char* const tb = g_smem;
   y = sh(y);
   keff = sh(keff);
   part = sh(part);
@@ -1398,29 +1399,30 @@ __device__ __noinline__ int dev_jac(const char* tb, const double* y, double h,
 // the production / loss split jp / jl is asked for, each chained term adds to
 // the production part when positive and to the loss part when negative.
 template <typename LT, bool EV = false, int FORM = kEither>
-__device__ __noinline__ int dev_f_aero(const char* tb, const double* y, double h,
+__device__ __noinline__ int dev_f_aero(const double* y, double h,
                                        const double* keff, double* rates, double* fscr,
                                        double* out, int lane, int flags, double* rp = nullptr,
                                        double* rl = nullptr) {
-  const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
+  const BlobOff& o = *reinterpret_cast<const BlobOff*>(g_smem);
   double* cv = rates + o.n_rates;
   if (o.n_cv > 0) sub_model_eval<false>(y, keff, cv, nullptr, rates + o.scr0[0], lane);
-  const bool neg = aero_rates(tb, y, keff, cv, rates, lane);
-  return dev_f<LT, EV, FORM>(tb, y, h, keff, rates, fscr, out, lane, flags | (neg ? kNegRate : 0), rp,
+  const bool neg = aero_rates(y, keff, cv, rates, lane);
+  return dev_f<LT, EV, FORM>(y, h, keff, rates, fscr, out, lane, flags | (neg ? kNegRate : 0), rp,
                        rl);
 }
 template <typename JT, bool EV = false, int FORM = kEither>
-__device__ __noinline__ int dev_jac_aero(const char* tb, const double* y, double h,
+__device__ __noinline__ int dev_jac_aero(const double* y, double h,
                                          const double* keff, double* part, JT* Jout, int lane, int flags,
                                          const uint16_t* csc = nullptr, double* jp = nullptr,
                                          double* jl = nullptr) {
+  const char* const tb = g_smem;
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
   double* cv = part + o.n_part_all;
   double* P = cv + o.n_cv;
   double* V = P + o.n_pj;
   if (o.n_cv > 0) sub_model_eval<true>(y, keff, cv, P, part + o.scr0[1], lane);
-  aero_partials(tb, y, keff, cv, part, lane);
-  const int r = dev_jac<JT, EV, FORM>(tb, y, h, keff, part, Jout, lane, flags, csc, jp, jl);
+  aero_partials(y, keff, cv, part, lane);
+  const int r = dev_jac<JT, EV, FORM>(y, h, keff, part, Jout, lane, flags, csc, jp, jl);
   if (r != 0 || o.n_chain == 0) return r;
   const uint16_t* vptr = (const uint16_t*)(tb + o.jv_ptr);
   const uint16_t* vpart = (const uint16_t*)(tb + o.jv_part);
@@ -1504,16 +1506,16 @@ __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
 // factorization level by level: L columns scaled by the level's reciprocal
 // pivots (stored in dinv), then its Schur updates grouped by target.  Returns
 // false on a zero or non-finite pivot.
-// Bound by latency and instruction count (cb05cl_ae5: 22 levels, 60 rounds of
-// at most 32 targets, mostly of one pair).  So every lane that scales an entry
+// Bound by latency and instruction count (cb05cl_ae5: 23 levels, 22 of them with
+// updates, 63 rounds of at most 32 targets, mostly of one pair).  So every lane that scales an entry
 // takes the reciprocal of its pivot itself, which saves a barrier and a trip
 // through shared memory per level; a round of updates is one record per lane,
 // read two rounds ahead.  J is laid out in the order of the LU positions, so
 // that its loads (global memory, four in flight) are nearly contiguous.
 template <typename LT>
-__device__ __noinline__ bool dev_form_factor(const char* tb, const LT* J, double gamma,
+__device__ __noinline__ bool dev_form_factor(const LT* J, double gamma,
                                              LT* LU, LT* dinv, int lane) {
-  tb = g_smem;
+  const char* const tb = g_smem;
   LU = sh(LU);
   dinv = sh(dinv);
   const BlobOff& o = *reinterpret_cast<const BlobOff*>(tb);
@@ -1594,8 +1596,9 @@ __device__ __forceinline__ void clear_spare(const char* tb, LT* LU, int lane) {
 }
 
 // z (in pivot order) <- M^{-1} z.
-// Bound by latency: some thirty levels in a row (cb05cl_ae5: 14 forward, 16
-// backward), each a handful of dependent steps on at most 32 targets.  So a
+// Bound by latency: some thirty levels in a row (cb05cl_ae5: 14 forward and 16
+// backward, in 16 and 17 rounds), each a handful of dependent steps on at most
+// 32 targets.  So a
 // round is one record load per lane and as few instructions as will do: the
 // record holds its first pair (the only one in most rounds), it is read two
 // rounds ahead, its L / U value and reciprocal pivot one (1 where there is
@@ -1875,9 +1878,10 @@ struct Cell {
       blk::call<LT>(cmd, *bx, blk::OP_F, yy, out, h > 0.0 ? h : h0);
       return 0;
     } else if constexpr (AERO)
-      return dev_f_aero<LT, false, FORM>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
+      return dev_f_aero<LT, false, FORM>(yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane,
+                                         flags);
     else
-      return dev_f<LT, false, FORM>(tb, yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
+      return dev_f<LT, false, FORM>(yy, h > 0.0 ? h : h0, keff, rates, fscr, out, lane, flags);
   }
   __device__ bool set_ewt(const double* yy) {
     bool bad = false;
@@ -1928,7 +1932,8 @@ struct Cell {
   }
   // l and tq of the fixed-leading-coefficient BDF formula.  Its dozen
   // divisions are a serial chain only in part: they are taken in three turns,
-  // a quotient per lane, and handed round (3 500 -> 900 cycles at one warp).
+  // a quotient per lane, and handed round (900 cycles at one warp; 3 500 one after
+  // the other).
   __device__ void set() {
     // xi_j = h / (h + tau_1 + ... + tau_(j-1)) in lane j, the sum in this order
     double hsum = h;
@@ -2029,15 +2034,15 @@ struct Cell {
         blk::call<LT>(cmd, *bx, blk::OP_JAC, ypred, nullptr, h > 0.0 ? h : h0);
         jr = 0;
       } else if constexpr (AERO) {
-        jr = dev_jac_aero<LT, false, FORM>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
+        jr = dev_jac_aero<LT, false, FORM>(ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
       } else {
-        jr = dev_jac<LT, false, FORM>(tb, ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
+        jr = dev_jac<LT, false, FORM>(ypred, h > 0.0 ? h : h0, keff, rates, J, lane, flags);
       }
       if (jr) return 1;
     }
     if constexpr (BLK) return blk::call<LT>(cmd, *bx, blk::OP_FACTOR, nullptr, nullptr, gamma);
     const bool ok = lu_mode ? dev_form_factor_seq<LT>(tb, J, gamma, LU, dinv, lane)
-                            : dev_form_factor<LT>(tb, J, gamma, LU, dinv, lane);
+                            : dev_form_factor<LT>(J, gamma, LU, dinv, lane);
     return ok ? 0 : 1;
   }
   // viol: whether this lane's share of the converged y has a negative value
@@ -2748,11 +2753,11 @@ __global__ void eval_kernel(EvalArgs a) {
   if (!a.do_jac) {
     double* out = (double*)(base + a.lay.ftemp);
     if (has_simpol(smem))
-      dev_f_aero<double, true>(smem, y, a.h, keff, rates, fscr, out, lane, odd,
+      dev_f_aero<double, true>(y, a.h, keff, rates, fscr, out, lane, odd,
                        a.rp + (size_t)cell * t.n,
                  a.rl + (size_t)cell * t.n);
     else
-      dev_f<double, true>(smem, y, a.h, keff, rates, fscr, out, lane, odd,
+      dev_f<double, true>(y, a.h, keff, rates, fscr, out, lane, odd,
                        a.rp + (size_t)cell * t.n,
             a.rl + (size_t)cell * t.n);
     #pragma unroll 1
@@ -2760,11 +2765,11 @@ __global__ void eval_kernel(EvalArgs a) {
   } else {
     const uint16_t* csc = csc_of(smem);
     if (has_simpol(smem))
-      dev_jac_aero<double, true>(smem, y, a.h, keff, rates, a.jv + (size_t)cell * t.n_jac, lane,
+      dev_jac_aero<double, true>(y, a.h, keff, rates, a.jv + (size_t)cell * t.n_jac, lane,
                            odd, csc,
                            a.jp + (size_t)cell * t.n_jac, a.jl + (size_t)cell * t.n_jac);
     else
-      dev_jac<double, true>(smem, y, a.h, keff, rates, a.jv + (size_t)cell * t.n_jac, lane,
+      dev_jac<double, true>(y, a.h, keff, rates, a.jv + (size_t)cell * t.n_jac, lane,
                            odd, csc,
                       a.jp + (size_t)cell * t.n_jac, a.jl + (size_t)cell * t.n_jac);
   }
@@ -2823,9 +2828,9 @@ __global__ void jac_check_kernel(CheckArgs c) {
                a.photo ? a.photo + (size_t)cell * m.n_photo : nullptr, keff, lane);
   const bool aero = has_simpol(smem);
   const int odd = vec_odd(y, t.n, lane);
-  if (dev_f_aero<double, true>(smem, y, a.h, keff, rates, fscr, f0, lane, odd, rp0, rl0) ||
-      (aero ? dev_jac_aero<double, true>(smem, y, a.h, keff, rates, J, lane, odd, csc_of(smem))
-            : dev_jac<double, true>(smem, y, a.h, keff, rates, J, lane, odd, csc_of(smem)))) {
+  if (dev_f_aero<double, true>(y, a.h, keff, rates, fscr, f0, lane, odd, rp0, rl0) ||
+      (aero ? dev_jac_aero<double, true>(y, a.h, keff, rates, J, lane, odd, csc_of(smem))
+            : dev_jac<double, true>(y, a.h, keff, rates, J, lane, odd, csc_of(smem)))) {
     if (lane == 0) {
       c.nfail[cell] = -1;
       c.worst[cell] = -1.0;
@@ -2848,10 +2853,10 @@ __global__ void jac_check_kernel(CheckArgs c) {
       const double dx = x * scale;
       if (lane == 0) y[j] = x + dx;
       __syncwarp();
-      int r = dev_f_aero<double, true>(smem, y, a.h, keff, rates, fscr, f1, lane, vec_odd(y, t.n, lane));
+      int r = dev_f_aero<double, true>(y, a.h, keff, rates, fscr, f1, lane, vec_odd(y, t.n, lane));
       if (lane == 0) y[j] = x + 0.5 * dx;
       __syncwarp();
-      r |= dev_f_aero<double, true>(smem, y, a.h, keff, rates, fscr, f2, lane, vec_odd(y, t.n, lane));
+      r |= dev_f_aero<double, true>(y, a.h, keff, rates, fscr, f2, lane, vec_odd(y, t.n, lane));
       if (lane == 0) y[j] = x;
       __syncwarp();
       if (r) continue;
@@ -2949,9 +2954,9 @@ __global__ void precision_kernel(PrecArgs p) {
   compute_keff(m, st, a.env[2 * cell], a.env[2 * cell + 1],
                a.photo ? a.photo + (size_t)cell * m.n_photo : nullptr, keff, lane);
   const int odd = vec_odd(y, t.n, lane);
-  int r = has_simpol(smem) ? dev_jac_aero<LT>(smem, y, a.h, keff, rates, J, lane, odd)
-                           : dev_jac<LT>(smem, y, a.h, keff, rates, J, lane, odd);
-  bool ok = r == 0 && dev_form_factor<LT>(smem, J, a.h, LU, dinv, lane);
+  int r = has_simpol(smem) ? dev_jac_aero<LT>(y, a.h, keff, rates, J, lane, odd)
+                           : dev_jac<LT>(y, a.h, keff, rates, J, lane, odd);
+  bool ok = r == 0 && dev_form_factor<LT>(J, a.h, LU, dinv, lane);
   if (ok) {
     #pragma unroll 1
     for (int i = lane; i < t.n; i += 32) {
