@@ -106,10 +106,29 @@ void pack_gather(std::vector<GatherItem>& items, uint32_t zero, int bytes_per_in
   auto half = [](size_t n) { return (int)(n + 1) / 2; };
   auto up = [](int n, int m) { return (n + m - 1) / m * m; };
   for (GatherItem& x : items) x.measure();
-  std::stable_sort(items.begin(), items.end(), [](const GatherItem& a, const GatherItem& b) {
-    return !a.neg.empty() != !b.neg.empty() ? !a.neg.empty() : a.longest > b.longest;
-  });
   const int n = (int)items.size();
+  // sorts indices by decreasing value, equal ones in order (by counting: the
+  // values are list lengths)
+  auto sort_by = [&](std::vector<int>* order, auto value) {
+    int most = 0;
+    for (int k : *order) most = std::max(most, value(k));
+    std::vector<int> at(most + 2, 0), to(n);
+    for (int k : *order) at[most - value(k) + 1]++;
+    for (int v = 0; v <= most; ++v) at[v + 1] += at[v];
+    for (int k : *order) to[at[most - value(k)]++] = k;
+    order->swap(to);
+  };
+  std::vector<int> in_order(n);
+  std::iota(in_order.begin(), in_order.end(), 0);
+  {
+    std::vector<int> by = in_order;
+    sort_by(&by, [&](int k) { return items[k].longest; });
+    sort_by(&by, [&](int k) { return (int)!items[k].neg.empty(); });
+    std::vector<GatherItem> v;
+    v.reserve(n);
+    for (int k : by) v.push_back(items[k]);
+    items.swap(v);
+  }
   struct Steps {
     int u = 0, l = 0, p = 0;
   };
@@ -117,15 +136,12 @@ void pack_gather(std::vector<GatherItem>& items, uint32_t zero, int bytes_per_in
   for (int k = 0; k < n; ++k)
     sh[k] = {(int)items[k].lead.size(), half(items[k].loss.size()), (int)items[k].prod.size()};
   // orders that put similar lists together: by words, products, losses
-  std::vector<std::vector<int>> orders(3, std::vector<int>(n));
+  std::vector<int> orders[3];
   for (int w = 0; w < 3; ++w) {
-    std::iota(orders[w].begin(), orders[w].end(), 0);
-    std::stable_sort(orders[w].begin(), orders[w].end(), [&](int a, int b) {
-      const Steps &x = sh[a], &y = sh[b];
-      if (w == 1 && x.p != y.p) return x.p > y.p;
-      if (w == 2 && x.l != y.l) return x.l > y.l;
-      return x.u + x.l + x.p > y.u + y.l + y.p;
-    });
+    orders[w] = in_order;
+    sort_by(&orders[w], [&](int k) { return sh[k].u + sh[k].l + sh[k].p; });
+    if (w == 1) sort_by(&orders[w], [&](int k) { return sh[k].p; });
+    if (w == 2) sort_by(&orders[w], [&](int k) { return sh[k].l; });
   }
   // the items from `first` on, in order w, as rounds of 32
   auto rounds = [&](int first, int w) {
@@ -599,16 +615,20 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
         const int cnt = two ? (most + 1) / 2 : most;
         o->cnt.push_back(two ? 0x8000 | (row << 9) | cnt : cnt);
         o->level.push_back(l);
-        for (size_t lane = 0; lane < kLanes; ++lane) {
-          const size_t k = two ? lane / 2 : lane;
-          const bool real = k < m && !(two && (lane & 1));
-          o->pair0.push_back(pair(lane, 0));
-          o->target.push_back(real ? (uint32_t)g.unit_target[us[k0 + k]] : (uint32_t)spare);
-          o->recip.push_back(real ? (uint32_t)g.unit_recip[us[k0 + k]] : 0u);
+        const size_t at0 = o->pair0.size(), ext0 = o->ext.size();
+        o->pair0.resize(at0 + kLanes);
+        o->target.resize(at0 + kLanes, (uint32_t)spare);
+        o->recip.resize(at0 + kLanes, 0u);
+        for (size_t lane = 0; lane < kLanes; ++lane) o->pair0[at0 + lane] = pair(lane, 0);
+        for (size_t k = 0; k < m; ++k) {
+          const size_t lane = at0 + (two ? 2 * k : k);
+          o->target[lane] = (uint32_t)g.unit_target[us[k0 + k]];
+          o->recip[lane] = (uint32_t)g.unit_recip[us[k0 + k]];
         }
+        o->ext.resize(ext0 + (size_t)row * (cnt - 1));
         for (int j = 1; j < cnt; ++j)
-          for (size_t lane = 0; lane < (size_t)row; ++lane)
-            o->ext.push_back(pair(lane, j));
+          for (int lane = 0; lane < row; ++lane)
+            o->ext[ext0 + (size_t)row * (j - 1) + lane] = pair(lane, j);
         k0 += m;
       }
     }
@@ -619,6 +639,8 @@ bool build_blob(const Tables& t, const std::vector<double>& atol_dep, int max_sm
       return false;
     }
   Rounds fbr, svr;
+  for (Rounds* r : {&fbr, &svr})
+    for (auto* v : {&r->pair0, &r->target, &r->recip, &r->ext}) v->reserve(128 * kLanes);
   const uint32_t lu_none = (uint32_t)t.n_lu | ((uint32_t)t.n_lu << 16);
   const uint32_t sv_none = (uint32_t)t.n_lu | ((uint32_t)n << 16);
   // the factorization takes reciprocal pivots with the scaling, so its units
