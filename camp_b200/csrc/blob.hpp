@@ -26,13 +26,13 @@ struct BlobOff {
   // f gather for any signs: entries (rxn | coef<<16 | prod<<31), units
   // (species, begin, end of losses, end of non-negative-yield products, end,
   // slot) as 8 x uint16, lane pointers (33 x uint16); read from the blob in
-  // global memory (self) where they are the exception.  Split species (species, first slot, count) as 3 x
-  // uint16
+  // global memory (self) where they are the exception.  Split species (species,
+  // first slot, count) as 3 x uint16
   int fg_ent, fg_unit, fg_lane, fg_split;
   // f (g[0]) and J (g[1]) gathers where no rate (partial), concentration or
-  // step is negative (empty with any_sign); every item is a unit of the f gather or a slot of the
-  // solver Jacobian, its sums L0, L1, P0 and P1 four chains of entries (uint32
-  // index | coef<<16).  Long items come first, as n_a rounds of eight items
+  // step is negative (empty with any_sign); every item is a unit of the f gather
+  // or a slot of the solver Jacobian, its sums L0, L1, P0 and P1 four chains of
+  // entries (uint32 index | coef<<16).  Long items come first, as n_a rounds of eight items
   // with one lane per chain: per lane a_rec (uint32 first entry | entries<<16,
   // id | tag<<16) into a_ent (lists of a multiple of four).  The rest follows
   // as n_b rounds of 32 items, one lane each: per round b_hdr (uint32 x 2:
